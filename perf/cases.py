@@ -124,8 +124,9 @@ def transformer_weights(cfg, d):
     w = {"tok_embedding": d.normal(V, H, std=1.0), "norm_weight": ones(H), "lm_head_weight": d.normal(H, V)}
     for i in range(cfg.num_layers):
         # YaRN multiplies scores by its concentration twice: smaller projections keep them of size one
-        t = {"qkv_weight": d.normal(H, qkv, std=0.02 if cfg.rope_scaling_factor <= 1 else 0.012), "o_weight": d.normal(cfg.q_size, H), "input_layernorm_weight": ones(H),
-             "post_attention_layernorm_weight": ones(H)}
+        std = 0.02 if cfg.rope_scaling_factor <= 1 else 0.012
+        t = {"qkv_weight": d.normal(H, qkv, std=std), "o_weight": d.normal(cfg.q_size, H),
+             "input_layernorm_weight": ones(H), "post_attention_layernorm_weight": ones(H)}
         if cfg.qk_norm:
             t.update(q_norm_weight=ones(D), k_norm_weight=ones(D))
         if cfg.attn_bias:
