@@ -34,7 +34,11 @@ struct Gemm2Args {            // <= 128 bytes (see GemmArgs)
   int gate_off;               // row offset of the up half in B
   int act;                    // gated: 0 = SiLU, 1 = GELU (tanh form); plain: 2 = squared ReLU, 7 = xIELU of act_a, act_b
   float act_a, act_b;
+  int splits;                 // > 1: fp32 partial sums, split s at out + s * split_stride
+  int kb_per_split;
+  int static_b;               // B (weights) is not written by the kernel before this one: its tiles go ahead of the wait
   long long ldo;
+  long long split_stride;
   void* out;
   const __nv_bfloat16* bias;
   const __nv_bfloat16* residual;
@@ -44,6 +48,25 @@ static_assert(sizeof(Gemm2Args) <= 128, "Gemm2Args grew past the fast kernel-par
 
 constexpr int k2TileN = 256;
 constexpr int k2StageBytes = 2 * kATileBytes;     // A rows + B rows of this CTA, 16 KB each
+
+struct Work2 {
+  int tm, tn, sp, kb0, kb1;
+};
+// group_m row tiles share a sweep over the column tiles so that A and B tiles are re-read from L2; the splits of a tile
+// follow one another
+__device__ __forceinline__ Work2 decode_work2(const Gemm2Args& a, int w) {
+  Work2 o;
+  o.sp = w % a.splits;
+  const int t = w / a.splits;
+  const int per_group = a.group_m * a.tiles_n;
+  const int g = t / per_group, first = g * a.group_m;
+  const int gsz = min(a.tiles_m - first, a.group_m), in = t - g * per_group;
+  o.tm = first + in % gsz;
+  o.tn = in / gsz;
+  o.kb0 = o.sp * a.kb_per_split;
+  o.kb1 = min(a.kb_total, o.kb0 + a.kb_per_split);
+  return o;
+}
 
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const Gemm2Args args) {
@@ -85,27 +108,37 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
   volatile int* abort_flag = &ctrl->abort;
 
   const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
-  const int total_work = args.tiles_m * args.tiles_n;
+  const int total_work = args.tiles_m * args.tiles_n * args.splits;
   griddep_launch();
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (both CTAs)
+    auto b_row_of = [&](int tn) {
+      return args.gated ? (int(rank) * args.gate_off + tn * 128) : (tn * 256 + int(rank) * 128);
+    };
+    // Weight tiles do not depend on the preceding kernel: the first fill of the ring takes them before the wait.  (The second
+    // CTA's bytes may arrive before the first one has announced them: a barrier's phase ends only with the announcement.)
+    int pre = 0;
+    if (args.static_b && pair < total_work) {
+      const Work2 t = decode_work2(args, pair);
+      pre = min(stages, t.kb1 - t.kb0);
+      if (lane == 0)
+        for (int i = 0; i < pre; ++i) {
+          if (rank == 0) mbar_expect_tx(&ctrl->full[i], 2 * k2StageBytes);
+          tma_load_2d_pair(tiles + i * k2StageBytes + kATileBytes, &tmB, map_to_cta(&ctrl->full[i], 0), (t.kb0 + i) * kBlockK,
+                           b_row_of(t.tn));
+        }
+      __syncwarp();
+    }
     griddep_wait();
     int stage = 0;
     uint32_t phase = 0;
     bool alive = true;
     for (int w = pair; w < total_work && alive; w += npairs) {
-      // group_m row tiles share a sweep over the column tiles so that A and B tiles are re-read from L2
-      const int kGroup = args.group_m;
-      const int per_group = kGroup * args.tiles_n;
-      const int g = w / per_group;
-      const int first = g * kGroup;
-      const int gsz = min(args.tiles_m - first, kGroup);
-      const int in = w - g * per_group;
-      const int tm = first + in % gsz, tn = in / gsz;
-      const int a_row = tm * 256 + int(rank) * 128;
-      const int b_row = args.gated ? (int(rank) * args.gate_off + tn * 128) : (tn * 256 + int(rank) * 128);
-      for (int kb = 0; kb < args.kb_total; ++kb) {
+      const Work2 t = decode_work2(args, w);
+      const int a_row = t.tm * 256 + int(rank) * 128;
+      const int b_row = b_row_of(t.tn);
+      for (int kb = t.kb0; kb < t.kb1; ++kb) {
         bool ok = mbar_wait(&ctrl->empty[stage], phase ^ 1u, abort_flag, args.status, ERR_WAIT_SMEM_EMPTY);
         if (!__all_sync(0xffffffffu, ok)) { alive = false; break; }
         if (lane == 0) {
@@ -114,9 +147,10 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
           // the first CTA announces the bytes of both CTAs; the second only lets its loads complete there
           // (its loads of this phase cannot start before the barrier entered the phase: they wait for the
           // stage to be released, which follows the previous phase's completion)
-          if (rank == 0) mbar_expect_tx(&ctrl->full[stage], 2 * k2StageBytes);
+          const bool ahead = w == pair && kb - t.kb0 < pre;
+          if (rank == 0 && !ahead) mbar_expect_tx(&ctrl->full[stage], 2 * k2StageBytes);
           tma_load_2d_pair(a_ptr, &tmA, full0, kb * kBlockK, a_row);
-          tma_load_2d_pair(a_ptr + kATileBytes, &tmB, full0, kb * kBlockK, b_row);
+          if (!ahead) tma_load_2d_pair(a_ptr + kATileBytes, &tmB, full0, kb * kBlockK, b_row);
         }
         __syncwarp();
         if (++stage == stages) { stage = 0; phase ^= 1u; }
@@ -141,7 +175,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
         ok = mbar_wait(&ctrl->tempty[acc], acc_phase ^ 1u, abort_flag, args.status, ERR_WAIT_TMEM_EMPTY);
         if (!ok) break;
         const uint32_t d0 = tmem_base + uint32_t(acc * k2TileN);
-        for (int kb = 0; kb < args.kb_total; ++kb) {
+        const Work2 t = decode_work2(args, w);
+        for (int kb = t.kb0; kb < t.kb1; ++kb) {
           ok = mbar_wait(&ctrl->full[stage], phase, abort_flag, args.status, ERR_WAIT_SMEM_FULL);
           if (!ok) break;
           tc_fence_after();
@@ -149,7 +184,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
           const uint64_t da = d_hi | a_lo, db = d_hi | (a_lo + uint32_t(kATileBytes >> 4));
 #pragma unroll
           for (int k = 0; k < kBlockK / 16; ++k)
-            umma_f16_pair(d0, da + uint64_t(k * 2), db + uint64_t(k * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+            umma_f16_pair(d0, da + uint64_t(k * 2), db + uint64_t(k * 2), idesc, (kb > t.kb0 || k > 0) ? 1u : 0u);
           umma_commit_pair(empty0 + uint32_t(stage) * 8u);
           umma_commit_pair(empty1 + uint32_t(stage) * 8u);
           if (++stage == stages) { stage = 0; phase ^= 1u; }
@@ -170,13 +205,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
     uint32_t acc_phase = 0;
     __nv_bfloat16* out_h = reinterpret_cast<__nv_bfloat16*>(args.out);
     for (int w = pair; w < total_work; w += npairs) {
-      const int kGroup = args.group_m;
-      const int per_group = kGroup * args.tiles_n;
-      const int g = w / per_group;
-      const int first = g * kGroup;
-      const int gsz = min(args.tiles_m - first, kGroup);
-      const int in = w - g * per_group;
-      const int tm = first + in % gsz, tn = in / gsz;
+      const Work2 work = decode_work2(args, w);
+      const int tm = work.tm, tn = work.tn;
       bool ok = mbar_wait(&ctrl->tfull[acc], acc_phase, abort_flag, args.status, ERR_WAIT_TMEM_FULL);
       if (!__all_sync(0xffffffffu, ok)) break;
       tc_fence_after();
@@ -238,6 +268,19 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
         }
         const int cbase = col0 + c;
         if (row >= args.m || cbase >= args.n) continue;
+        if (args.splits > 1) {
+          float* o = reinterpret_cast<float*>(args.out) + work.sp * args.split_stride + (long long)row * args.ldo + cbase;
+          if (cbase + 32 <= args.n && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              reinterpret_cast<float4*>(o)[j] = make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
+                                                            __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
+          } else {
+            for (int j = 0; j < 32; ++j)
+              if (cbase + j < args.n) o[j] = __uint_as_float(v[j]);
+          }
+          continue;
+        }
         if (args.bias && args.bias_on_cols) {
 #pragma unroll
           for (int j = 0; j < 32; ++j)
@@ -320,12 +363,14 @@ extern "C" int nkb_gemm_2cta_pairs() { return g_pairs_last; }
 // the square of the positive part of (A B^T + bias); 7 (not gated): xIELU with the parameters act_a, act_b.
 extern "C" int nkb_gemm_bf16_2cta(const void* A, const void* B, void* out, int m, int n, int k, long long lda,
                                   long long ldb, long long ldo, const void* bias, const void* residual, int gated,
-                                  int gate_off, int act, float act_a, float act_b, void* stream) {
+                                  int gate_off, int act, float act_a, float act_b, int splits, long long split_stride,
+                                  int static_b, void* stream) {
+  if (splits < 1 || (splits > 1 && (gated || bias || residual || act))) return -2;
   if (act < 0 || (act > 2 && act != 7) || (act >= 2 && gated)) return -2;
   if (!status_word() && nkb_init() != 0) return -1;
   if (m <= 0 || n <= 0 || k <= 0) return -2;
   if ((k & 7) || (lda & 7) || (ldb & 7)) return -2;
-  if (m < 256 || n < 256) return -5;
+  if (n < 256) return -5;
   Gemm2Args a{};
   a.m = m; a.n = n; a.k = k;
   a.tiles_m = (m + 255) / 256;
@@ -337,6 +382,11 @@ extern "C" int nkb_gemm_bf16_2cta(const void* A, const void* B, void* out, int m
   a.act_b = act_b;
   if (gated && (bias || residual)) return -2;
   a.kb_total = (k + kBlockK - 1) / kBlockK;
+  a.splits = splits;
+  a.kb_per_split = (a.kb_total + splits - 1) / splits;
+  if ((splits - 1) * a.kb_per_split >= a.kb_total) return -2;       // an empty split would leave its partial unwritten
+  a.split_stride = split_stride;
+  a.static_b = static_b;
   a.bias_on_cols = 1;
   static int group_m = 0;
   if (group_m == 0) {
@@ -363,7 +413,7 @@ extern "C" int nkb_gemm_bf16_2cta(const void* A, const void* B, void* out, int m
     if (e != cudaSuccess) return int(e);
     attr_set = true;
   }
-  const int total = a.tiles_m * a.tiles_n;
+  const int total = a.tiles_m * a.tiles_n * splits;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * (num_sms() / 2));
   cfg.blockDim = dim3(kGemmThreads);

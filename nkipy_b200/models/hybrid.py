@@ -83,13 +83,13 @@ class GatedLayer:
         else:
             act = ops.linear(h, self.w_in2[:2 * ff], gated=True, act=self.spec.act, swap=False)
             gate = Proj(ops.linear(h, self.w_in2[2 * ff:], swap=False), 0, width)
-        return Proj(m.project(act, self.w_down), 0, width), gate
+        return Proj(m.project(act, self.w_down, True), 0, width), gate
 
     def _run(self, h, entry, cache, b) -> List[Branch]:
         m, width = self.model, self.width
         y = m.project(h[0], self.w_in1)
         mixed = self.mixer.run(m, y, h[0], entry, cache, b)
-        branches = [Branch(Proj(m.project(mixed, self.mixer.w_o), 0, width), Proj(y, sum(self.mixer.widths), width),
+        branches = [Branch(Proj(m.project(mixed, self.mixer.w_o, True), 0, width), Proj(y, sum(self.mixer.widths), width),
                            self.gate_bias[0])]
         if self.spec.ff:
             branches.append(Branch(*self._feed_forward(h[1]), self.gate_bias[1]))
@@ -113,7 +113,7 @@ class DenseMLP:
             a = ops.activation(Proj(model.project(h, self.up), 0, self.up.shape[0]), self.act, dtype=h.dtype)
         else:
             a = ops.linear(h, self.up, swap=False, out_act=self.act)
-        return [Branch(Proj(model.project(a, self.down), 0, h.shape[1]))]
+        return [Branch(Proj(model.project(a, self.down, True), 0, h.shape[1]))]
 
 
 class GatedMLP:
@@ -134,7 +134,7 @@ class GatedMLP:
             a = ops.gated_act(Proj(wide.t, wide.col, n), Proj(wide.t, wide.col + n, n), self.act, dtype=h.dtype)
         else:
             a = ops.linear(h, self.w_wide, gated=True, act=self.act, swap=False)
-        return [Branch(Proj(model.project(a, self.down), 0, h.shape[1]))]
+        return [Branch(Proj(model.project(a, self.down, True), 0, h.shape[1]))]
 
 
 class PreNormLayer:
@@ -162,7 +162,7 @@ class PreNormLayer:
     def _mix(self, h, entry, cache, b) -> List[Branch]:
         m = self.model
         y = m.project(h[0], self.mixer.w_in) if self.mixer.w_in is not None else None
-        return [Branch(Proj(m.project(self.mixer.run(m, y, h[0], entry, cache, b), self.mixer.w_o), 0, self.width))]
+        return [Branch(Proj(m.project(self.mixer.run(m, y, h[0], entry, cache, b), self.mixer.w_o, True), 0, self.width))]
 
 
 class SandwichLayer:
@@ -187,7 +187,7 @@ class SandwichLayer:
     def _mix(self, h, entry, cache, b) -> List[Branch]:
         m = self.model
         o = self.mixer.run(m, m.project(h[0], self.mixer.w_in), h[0], entry, cache, b)
-        return o if isinstance(o, list) else [Branch(Proj(m.project(o, self.mixer.w_o), 0, self.width))]
+        return o if isinstance(o, list) else [Branch(Proj(m.project(o, self.mixer.w_o, True), 0, self.width))]
 
 
 class ParallelLayer:
@@ -244,14 +244,14 @@ class ParallelLayer:
         else:
             mix = Proj(m.project(h, self.mixer.w_in), 0, self.spans[1][1])
         o = self.mixer.run(m, mix, h, entry, cache, b)
-        branches = [Branch(Proj(m.project(o, self.mixer.w_o), 0, self.width))]
+        branches = [Branch(Proj(m.project(o, self.mixer.w_o, True), 0, self.width))]
         return branches if self.mlp is None else branches + self.mlp.run(m, h, wide, narrow)
 
     def _token_input(self, h, entry, cache, b) -> List[Branch]:
         m, n = self.model, self.side_gate.shape[0]
         z = Proj(m.project(h[0], self.side_gate), 0, n)
         a = ops.gated_act(z, Proj(m.side_table, m.layers.index(self) * n, n), "gelu_tanh", dtype=m.dtype, up_rows=b.ids)
-        return [Branch(Proj(m.project(a, self.side_proj), 0, self.width), norm=self.side_norm)]
+        return [Branch(Proj(m.project(a, self.side_proj, True), 0, self.width), norm=self.side_norm)]
 
 
 LAYERS = {"gated": GatedLayer, "pre-norm": PreNormLayer, "sandwich": SandwichLayer, "parallel": ParallelLayer}
@@ -329,14 +329,16 @@ class HybridLM:
         """Whether projections of h come as fp32 (split-K) sums, see `project`."""
         return x_small(h)
 
-    def project(self, x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
-        """fp32 (split-K partials) for small batches, bf16 for large ones, fp32 for 32-bit models."""
+    def project(self, x: torch.Tensor, w: torch.Tensor, summed: bool = False) -> torch.Tensor:
+        """fp32 (split-K partials) for small batches, bf16 for large ones, fp32 for 32-bit models.  summed: the residual kernel
+        reads the result, so that middle-sized batches too may leave partials (`ops.prefill_plan`)."""
         if x.dtype == torch.float32:
             return ops.linear(x, w)
         if x.shape[0] <= SMALL_BATCH:
             splits = pick_splits(w.shape[0], w.shape[1])
             return ops.linear(x, w, splits=splits) if splits > 1 else ops.linear(x, w, fp32_out=True)
-        return ops.linear(x, w, swap=False)
+        splits = ops.prefill_plan(x.shape[0], w.shape[0], x.shape[1])[1] if summed and x.is_cuda and x.shape[1] % 8 == 0 else 1
+        return ops.linear(x, w, swap=False, splits=splits)
 
     def project_each(self, x: torch.Tensor, w: torch.Tensor) -> List[Proj]:
         """x[i] @ w[i].T for x [M, T, K], w [M, N, K]: one grouped product for small bf16 batches."""

@@ -362,7 +362,7 @@ class BlendMixer:
         left, right = columns(y, self.widths)
         outs = [(self.left, self.left.run(model, left, h, entry, cache, b)),
                 (self.right, self.right.run(model, right, h, entry + len(self.left.entries()), cache, b))]
-        return [Branch(Proj(model.project(o, m.w_o), 0, m.w_o.shape[0]), scale=0.5, norm=n, shift=getattr(m, "o_bias", None))
+        return [Branch(Proj(model.project(o, m.w_o, True), 0, m.w_o.shape[0]), scale=0.5, norm=n, shift=getattr(m, "o_bias", None))
                 for (m, o), n in zip(outs, self.norms)]
 
 

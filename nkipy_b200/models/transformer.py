@@ -429,7 +429,8 @@ class TransformerLM:
             resid, normed = inputs
         taps = [] if return_hidden else None
         for i, lw in enumerate(self.layers):
-            qkv = ops.linear(normed, lw.qkv, swap=False)
+            swap, splits = ops.prefill_plan(normed.shape[0], lw.qkv.shape[0], lw.qkv.shape[1])
+            qkv = ops.linear(normed, lw.qkv, swap=swap and splits > 1, splits=splits)
             q = ops.rope_kv_append(qkv, positions, slots, self.rope, cache.k[i], cache.v[i], self.nq, self.nkv,
                                    self.d, bias=lw.qkv_bias, q_norm_w=lw.q_norm, k_norm_w=lw.k_norm,
                                    norm_eps=cfg.rms_eps)
@@ -437,8 +438,7 @@ class TransformerLM:
                                           self.scale, max_q_len=max_q_len, causal=cfg.causal,
                                           window=cfg.window_for_layer(i), sinks=lw.sinks)
             if tp1:
-                resid = ops.linear(attn, lw.o, swap=False, residual=resid, bias=lw.o_bias)
-                normed = ops.rmsnorm(resid, lw.post_norm, cfg.rms_eps)
+                resid, normed = self._residual_linear(attn, lw.o, resid, lw.post_norm, lw.o_bias)
             else:
                 o = ops.linear(attn, lw.o, swap=False, bias=lw.o_bias)
                 self.tp.all_reduce(o)
@@ -449,13 +449,13 @@ class TransformerLM:
                 resid, normed = ops.add_rmsnorm(y, nxt, residual_in=resid, eps=cfg.rms_eps)
             else:
                 if cfg.swiglu_limit <= 0:
-                    act = ops.linear(normed, lw.gate_up, gated=True, swap=False)
+                    # tiles of 32 or 64 tokens on the narrow side up to 64 rows; with one of 128 the weights belong there
+                    act = ops.linear(normed, lw.gate_up, gated=True, swap=normed.shape[0] <= 64)
                 else:
                     act = ops.silu_mul(ops.linear(normed, lw.gate_up, swap=False), limit=cfg.swiglu_limit,
                                        alpha=cfg.swiglu_alpha)
                 if tp1:
-                    resid = ops.linear(act, lw.down, swap=False, residual=resid)
-                    normed = ops.rmsnorm(resid, nxt, cfg.rms_eps)
+                    resid, normed = self._residual_linear(act, lw.down, resid, nxt)
                 else:
                     dn = ops.linear(act, lw.down, swap=False)
                     self.tp.all_reduce(dn)
@@ -465,6 +465,16 @@ class TransformerLM:
         if return_hidden:
             return normed, taps
         return normed
+
+    def _residual_linear(self, x, w, resid, next_norm, bias=None):
+        """(resid + x w^T + bias, its norm) for a packed step on one rank: split-K partials summed by the norm kernel where a
+        step of that size splits (`ops.prefill_plan`), the residual in the epilogue otherwise."""
+        swap, splits = ops.prefill_plan(x.shape[0], w.shape[0], x.shape[1])
+        if splits > 1:
+            return ops.add_rmsnorm(None, next_norm, residual_in=resid, partials=ops.linear(x, w, swap=swap, splits=splits),
+                                   bias=bias, eps=self.cfg.rms_eps)
+        resid = ops.linear(x, w, swap=False, residual=resid, bias=bias)
+        return resid, ops.rmsnorm(resid, next_norm, self.cfg.rms_eps)
 
     SP_MIN_CAPACITY = 16384       # tokens; the engine's default prefill chunk
     # Local token count from which the MoE block of the sequence-parallel prefill exchanges tokens with the

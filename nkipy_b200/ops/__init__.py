@@ -87,6 +87,47 @@ def _check_bf16(*tensors):
 _USE_2CTA = os.environ.get("NKIPY_B200_GEMM_2CTA", "1") == "1"
 
 
+def _pair_tiles(rows: int, cols: int, gated: bool) -> int:
+    """256 x 256 tiles of the CTA-pair kernel (gated: 128 columns of gate and up each)."""
+    return -(-rows // 256) * -(-cols // (128 if gated else 256))
+
+
+def _use_pairs(rows: int, cols: int, gated: bool) -> bool:
+    """Whether CTA pairs on 256 x 256 tiles beat single CTAs on 128 x 256 ones.  A round of pairs (74 tiles) takes about 24 us per
+    4096 of k, one of single CTAs (148 half-size tiles, three quarters of the loads per multiply-add more) about 31, so only
+    rounding decides: 300 rows of a 2 x 14336 gate / up product take 108 us on single CTAs and 120 on pairs, 414 rows 140 and
+    122, 200 rows 79 and 68."""
+    if rows <= 128 or cols < 256 or not _USE_2CTA:
+        return False
+    single = -(-rows // 128) * -(-cols // (128 if gated else 256))
+    return rows >= 2048 or -(-_pair_tiles(rows, cols, gated) // 74) * 24 <= -(-single // 148) * 31
+
+
+def prefill_plan(rows: int, cols: int, k: int) -> Tuple[bool, int]:
+    """(swap, splits) of a product whose consumer can sum split-K partials, for a packed step of `rows` tokens.
+
+    Up to 128 rows a decode step's form (weights on the 128-row side, `models.transformer.pick_splits`); above, pairs of CTAs
+    split over k while their tiles leave SMs idle: a round takes 0.4 us per 64 of k, and partials are written and read once
+    at some 4 TB/s; a gain of less than 3 us is left alone.  414 rows of 14336 -> 4096: 74 us whole, 48 us in two; 130 rows: 71 and 32 us in four; 414 rows of
+    4096 -> 6144 stay whole (30 us, 33 in three)."""
+    if rows <= 128:
+        from ..models.transformer import pick_splits
+
+        return True, pick_splits(cols, k)
+    if cols < 256 or not _USE_2CTA or k % 8:
+        return False, 1
+    slabs, tiles = -(-k // 64), _pair_tiles(rows, cols, False)
+    best, best_cost = 1, -(-tiles // 74) * slabs * 0.4 - 3.0
+    for s in range(2, 9):
+        per = -(-slabs // s)
+        if per < 8 or -(-slabs // per) != s:
+            continue
+        cost = -(-tiles * s // 74) * per * 0.4 + s * rows * cols * 8 / 4e6
+        if cost < best_cost:
+            best, best_cost = s, cost
+    return False, best
+
+
 def _pick_block_n(cols: int, gated: bool) -> int:
     cap = 128 if gated else 256
     for bn in (32, 64, 128, 256):
@@ -190,12 +231,12 @@ def linear(
         out_fp32, split_stride = 1 if fp32_out else 0, 0
     ldo = out_view.stride(-2) if out_view.dim() >= 2 else N
     act_code = mixers.ACTIVATIONS[act][0] if gated else (epi.code if out_act is not None else 0)
-    if (not swap and splits <= 1 and not fp32_out and M >= 512 and N >= 256 and _USE_2CTA and (ldo & 7) == 0
-            and not (gated and (bias is not None or residual is not None))):
+    if (not swap and not fp32_out and (ldo & 7) == 0 and not (gated and (bias is not None or residual is not None))
+            and (_use_pairs(M, N, gated) if splits <= 1 else M > 128 and N >= 256 and _USE_2CTA and bias is None and residual is None)):
         # prefill-sized: CTA pairs on 256 x 256 tiles (csrc/kernels/gemm_2cta.cu)
         rc = L.nkb_gemm_bf16_2cta(x.data_ptr(), w.data_ptr(), out_view.data_ptr(), M, N, K, x.stride(0), w.stride(0),
                                   ldo, _ptr(bias), _ptr(residual), 1 if gated else 0, N if gated else 0, act_code, epi.a, epi.b,
-                                  _stream())
+                                  eff, split_stride, 1 if weights_static else 0, _stream())
         if rc != -5:
             _lib.check(rc, "nkb_gemm_bf16_2cta")
             _launches += 1

@@ -1,0 +1,52 @@
+"""CTA-pair products split over k, and the plan of a packed step's projections."""
+import pytest
+import torch
+
+from nkipy_b200 import ops
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m", [129, 255, 256, 257, 414])
+@pytest.mark.parametrize("n,k,splits", [(256, 512, 2), (300, 4096, 3), (2880, 1032, 5), (4096, 14336, 8)])
+def test_split_sums(m, n, k, splits):
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    x = torch.randn((m, k + 8), generator=g, device="cuda").to(torch.bfloat16)[:, :k]
+    w = torch.randn((n, k), generator=g, device="cuda").to(torch.bfloat16)
+    parts = ops.linear(x, w, swap=False, splits=splits)
+    assert parts.dtype == torch.float32 and parts.shape[1:] == (m, n) and 1 < parts.shape[0] <= splits
+    want = x.double() @ w.double().T
+    # exact products summed in 32 bits, at most k roundings of values below the sum of the absolute products
+    bound = k * 2.0 ** -23 * (x.double().abs() @ w.double().abs().T)
+    assert ((parts.double().sum(0) - want).abs() <= bound).all()
+    ops.raise_on_device_error()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("gated", [False, True])
+@pytest.mark.parametrize("m", [129, 200, 300, 500])
+def test_whole_products_of_middle_sizes(m, gated):
+    """Either kernel of the rule, with the epilogues a packed step uses."""
+    g = torch.Generator(device="cuda").manual_seed(m)
+    n, k = 520, 384
+    x = torch.randn((m, k), generator=g, device="cuda").to(torch.bfloat16)
+    w = (0.05 * torch.randn((2 * n if gated else n, k), generator=g, device="cuda")).to(torch.bfloat16)
+    bias, res = None, None
+    want = x.double() @ w.double().T
+    if gated:
+        want = torch.nn.functional.silu(want[:, :n]) * want[:, n:]
+    else:
+        bias = torch.randn((n,), generator=g, device="cuda").to(torch.bfloat16)
+        res = torch.randn((m, n), generator=g, device="cuda").to(torch.bfloat16)
+        want = want + bias.double() + res.double()
+    y = ops.linear(x, w, swap=False, gated=gated, bias=bias, residual=res)
+    # one rounding to bf16, and the approximate exponential of the gate
+    assert ((y.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-3).all()
+
+
+def test_plan_leaves_no_split_empty():
+    for rows in (1, 64, 128, 129, 257, 512, 1500, 5000):
+        for cols, k in ((256, 64), (300, 128), (4096, 1032), (4096, 14336), (22016, 4096)):
+            swap, splits = ops.prefill_plan(rows, cols, k)
+            slabs = -(-k // 64)
+            assert swap == (rows <= 128) and 1 <= splits <= 8
+            assert splits == 1 or swap or -(-slabs // -(-slabs // splits)) == splits
