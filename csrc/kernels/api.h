@@ -78,6 +78,10 @@ int nkb_gemm_effective_splits(int k, int splits);
 int nkb_gemm_bf16_2cta(const void* A, const void* B, void* out, int m, int n, int k, long long lda, long long ldb,
                        long long ldo, const void* bias, const void* residual, int gated, int gate_off, int act,
                        float act_a, float act_b, int splits, long long split_stride, int static_b, void* stream);
+int nkb_gemm_bf16_2cta_grouped(const void* weights, const void* x_sorted, void* out, const int* group_offsets, int num_groups,
+                               int features, int k, int total_rows, long long ldx, long long ldo, int gated, int gate_off,
+                               const void* bias, long long bias_group_stride, float act_limit, float act_alpha,
+                               const int* tile_list, const int* tile_count, int max_tiles, void* stream);
 int nkb_gemm_bf16_push(const void* weights, const void* x, int features, int tokens, int k, long long ldw,
                        long long ldx, long long ldo, int splits, const void* bias, int block_n, void* const* peer_out,
                        void* const* peer_flag, int n_peers, int rank, void* done_counter, void* mc_out, void* mc_flag,

@@ -28,7 +28,6 @@ struct Gemm2Args {            // <= 128 bytes (see GemmArgs)
   int m, n, k;
   int tiles_m, tiles_n;       // 256 x 256 tiles
   int kb_total, stages;
-  int bias_on_cols;
   int group_m;                // row tiles that share one sweep over the column tiles (L2 reuse)
   int gated;                  // B holds [gate; up] rows: the pair's first CTA loads gate rows, the second up rows
   int gate_off;               // row offset of the up half in B
@@ -49,27 +48,58 @@ static_assert(sizeof(Gemm2Args) <= 128, "Gemm2Args grew past the fast kernel-par
 constexpr int k2TileN = 256;
 constexpr int k2StageBytes = 2 * kATileBytes;     // A rows + B rows of this CTA, 16 KB each
 
+// Rows of A sorted by group, one weight matrix per group (stacked in B): tile t of the list is rows [256 ct, 256 ct + 256) of a
+// group.  A struct of its own: the plain kernel's arguments stay small.
+struct Group2Args {
+  const int* tile_list;       // (group, ct) pairs
+  const int* tile_count;
+  const int* offsets;         // first row of each group
+  int w_rows;                 // rows of B per group
+  long long bias_stride;
+  float limit, alpha;         // limit > 0: clamped gate (up + 1) * gate * sigmoid(alpha * gate)
+};
+
 struct Work2 {
   int tm, tn, sp, kb0, kb1;
+  int a_row0, row_end, b_row0, group;    // first row of A and end of its rows, first row of B
 };
 // group_m row tiles share a sweep over the column tiles so that A and B tiles are re-read from L2; the splits of a tile
-// follow one another
-__device__ __forceinline__ Work2 decode_work2(const Gemm2Args& a, int w) {
+// follow one another.  Groups: the column tiles of a row tile follow one another (its weights are read once either way).
+template <bool GROUPED>
+__device__ __forceinline__ Work2 decode_work2(const Gemm2Args& a, const Group2Args& g, int w) {
   Work2 o;
+  if constexpr (GROUPED) {
+    const int t = w / a.tiles_n;
+    o.tm = 0;
+    o.tn = w - t * a.tiles_n;
+    o.sp = 0;
+    o.kb0 = 0;
+    o.kb1 = a.kb_total;
+    o.group = g.tile_list[2 * t];
+    o.a_row0 = g.offsets[o.group] + g.tile_list[2 * t + 1] * 256;
+    o.row_end = g.offsets[o.group + 1];
+    o.b_row0 = o.group * g.w_rows;
+    return o;
+  }
   o.sp = w % a.splits;
   const int t = w / a.splits;
   const int per_group = a.group_m * a.tiles_n;
-  const int g = t / per_group, first = g * a.group_m;
-  const int gsz = min(a.tiles_m - first, a.group_m), in = t - g * per_group;
+  const int gr = t / per_group, first = gr * a.group_m;
+  const int gsz = min(a.tiles_m - first, a.group_m), in = t - gr * per_group;
   o.tm = first + in % gsz;
   o.tn = in / gsz;
   o.kb0 = o.sp * a.kb_per_split;
   o.kb1 = min(a.kb_total, o.kb0 + a.kb_per_split);
+  o.a_row0 = o.tm * 256;
+  o.row_end = a.m;
+  o.b_row0 = 0;
+  o.group = 0;
   return o;
 }
 
-__global__ void __launch_bounds__(kGemmThreads, 1)
-gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const Gemm2Args args) {
+template <bool GROUPED>
+__device__ __forceinline__ void gemm2_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const Gemm2Args& args,
+                                           const Group2Args& grp) {
   extern __shared__ uint8_t smem_raw[];
   // identical layout in both CTAs: [control 1 KB][ring]
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -108,25 +138,27 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
   volatile int* abort_flag = &ctrl->abort;
 
   const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
-  const int total_work = args.tiles_m * args.tiles_n * args.splits;
+  // the tile list comes from the kernels before this one: every role waits before it reads the count
+  if constexpr (GROUPED) griddep_wait();
+  const int total_work = GROUPED ? *grp.tile_count * args.tiles_n : args.tiles_m * args.tiles_n * args.splits;
   griddep_launch();
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (both CTAs)
-    auto b_row_of = [&](int tn) {
-      return args.gated ? (int(rank) * args.gate_off + tn * 128) : (tn * 256 + int(rank) * 128);
+    auto b_row_of = [&](const Work2& t) {
+      return t.b_row0 + (args.gated ? (int(rank) * args.gate_off + t.tn * 128) : (t.tn * 256 + int(rank) * 128));
     };
     // Weight tiles do not depend on the preceding kernel: the first fill of the ring takes them before the wait.  (The second
     // CTA's bytes may arrive before the first one has announced them: a barrier's phase ends only with the announcement.)
     int pre = 0;
-    if (args.static_b && pair < total_work) {
-      const Work2 t = decode_work2(args, pair);
+    if (!GROUPED && args.static_b && pair < total_work) {
+      const Work2 t = decode_work2<GROUPED>(args, grp, pair);
       pre = min(stages, t.kb1 - t.kb0);
       if (lane == 0)
         for (int i = 0; i < pre; ++i) {
           if (rank == 0) mbar_expect_tx(&ctrl->full[i], 2 * k2StageBytes);
           tma_load_2d_pair(tiles + i * k2StageBytes + kATileBytes, &tmB, map_to_cta(&ctrl->full[i], 0), (t.kb0 + i) * kBlockK,
-                           b_row_of(t.tn));
+                           b_row_of(t));
         }
       __syncwarp();
     }
@@ -135,9 +167,9 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
     uint32_t phase = 0;
     bool alive = true;
     for (int w = pair; w < total_work && alive; w += npairs) {
-      const Work2 t = decode_work2(args, w);
-      const int a_row = t.tm * 256 + int(rank) * 128;
-      const int b_row = b_row_of(t.tn);
+      const Work2 t = decode_work2<GROUPED>(args, grp, w);
+      const int a_row = t.a_row0 + int(rank) * 128;
+      const int b_row = b_row_of(t);
       for (int kb = t.kb0; kb < t.kb1; ++kb) {
         bool ok = mbar_wait(&ctrl->empty[stage], phase ^ 1u, abort_flag, args.status, ERR_WAIT_SMEM_EMPTY);
         if (!__all_sync(0xffffffffu, ok)) { alive = false; break; }
@@ -175,7 +207,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
         ok = mbar_wait(&ctrl->tempty[acc], acc_phase ^ 1u, abort_flag, args.status, ERR_WAIT_TMEM_EMPTY);
         if (!ok) break;
         const uint32_t d0 = tmem_base + uint32_t(acc * k2TileN);
-        const Work2 t = decode_work2(args, w);
+        const Work2 t = decode_work2<GROUPED>(args, grp, w);
         for (int kb = t.kb0; kb < t.kb1; ++kb) {
           ok = mbar_wait(&ctrl->full[stage], phase, abort_flag, args.status, ERR_WAIT_SMEM_FULL);
           if (!ok) break;
@@ -205,13 +237,17 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
     uint32_t acc_phase = 0;
     __nv_bfloat16* out_h = reinterpret_cast<__nv_bfloat16*>(args.out);
     for (int w = pair; w < total_work; w += npairs) {
-      const Work2 work = decode_work2(args, w);
-      const int tm = work.tm, tn = work.tn;
+      const Work2 work = decode_work2<GROUPED>(args, grp, w);
+      const int tn = work.tn;
+      const __nv_bfloat16* bias = args.bias;
+      if constexpr (GROUPED) {
+        if (bias) bias += work.group * grp.bias_stride;
+      }
       bool ok = mbar_wait(&ctrl->tfull[acc], acc_phase, abort_flag, args.status, ERR_WAIT_TMEM_FULL);
       if (!__all_sync(0xffffffffu, ok)) break;
       tc_fence_after();
       const uint32_t t0 = tmem_base + (uint32_t(quad * 32) << 16) + uint32_t(acc * k2TileN);
-      const int row = tm * 256 + int(rank) * 128 + quad * 32 + lane;
+      const int row = work.a_row0 + int(rank) * 128 + quad * 32 + lane;
       if (args.gated) {
         // accumulator columns [0, 128) = gate, [128, 256) = up: out[:, tn * 128 + j] = silu(gate_j) * up_j
         const int gcol0 = tn * 128;
@@ -227,8 +263,25 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
             if (lane == 0) mbar_arrive_cluster(map_to_cta(&ctrl->tempty[acc], 0));
           }
           const int cbase = gcol0 + c;
-          if (row >= args.m || cbase >= args.n) continue;
-          if (args.act) {
+          if (row >= work.row_end || cbase >= args.n) continue;
+          if constexpr (GROUPED) {
+            if (bias) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) {
+                const int c1 = min(cbase + j, args.n - 1);
+                v[j] = __float_as_uint(__uint_as_float(v[j]) + __bfloat162float(bias[c1]));
+                u[j] = __float_as_uint(__uint_as_float(u[j]) + __bfloat162float(bias[args.gate_off + c1]));
+              }
+            }
+          }
+          if (GROUPED && grp.limit > 0.f) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              const float gg = fminf(__uint_as_float(v[j]), grp.limit);
+              const float uu = fminf(fmaxf(__uint_as_float(u[j]), -grp.limit), grp.limit);
+              v[j] = __float_as_uint((uu + 1.f) * gg / (1.f + __expf(-grp.alpha * gg)));
+            }
+          } else if (args.act) {
 #pragma unroll
             for (int j = 0; j < 32; ++j)
               v[j] = __float_as_uint(gelu_tanh_f(__uint_as_float(v[j])) * __uint_as_float(u[j]));
@@ -267,7 +320,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
           if (lane == 0) mbar_arrive_cluster(map_to_cta(&ctrl->tempty[acc], 0));
         }
         const int cbase = col0 + c;
-        if (row >= args.m || cbase >= args.n) continue;
+        if (row >= work.row_end || cbase >= args.n) continue;
         if (args.splits > 1) {
           float* o = reinterpret_cast<float*>(args.out) + work.sp * args.split_stride + (long long)row * args.ldo + cbase;
           if (cbase + 32 <= args.n && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {
@@ -281,11 +334,11 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
           }
           continue;
         }
-        if (args.bias && args.bias_on_cols) {
+        if (bias) {
 #pragma unroll
           for (int j = 0; j < 32; ++j)
             if (cbase + j < args.n)
-              v[j] = __float_as_uint(__uint_as_float(v[j]) + __bfloat162float(args.bias[cbase + j]));
+              v[j] = __float_as_uint(__uint_as_float(v[j]) + __bfloat162float(bias[cbase + j]));
         }
         if (args.act == 7) {       // xIELU
 #pragma unroll
@@ -347,6 +400,55 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
   }
 }
 
+__global__ void __launch_bounds__(kGemmThreads, 1)
+gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const Gemm2Args args) {
+  gemm2_body<false>(tmA, tmB, args, Group2Args{});
+}
+__global__ void __launch_bounds__(kGemmThreads, 1)
+gemm2_grouped_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const Gemm2Args args,
+                     const Group2Args grp) {
+  gemm2_body<true>(tmA, tmB, args, grp);
+}
+
+// Launches `pairs` CTA pairs, at most as many as can be resident at once (the persistent loop strides by their number, and
+// pairs need two SMs of one GPC: not every SM can be paired) and as there are tiles.
+template <typename K, typename... Args>
+static int launch_pairs(K kernel, int* resident, int total, int smem, cudaStream_t stream, int* used, const Args&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2 * (num_sms() / 2));
+  cfg.blockDim = dim3(kGemmThreads);
+  cfg.dynamicSmemBytes = size_t(smem);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (*resident == 0) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
+    if (e != cudaSuccess) return int(e);
+    int n = 0;
+    e = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
+    *resident = (e == cudaSuccess && n > 0) ? n : num_sms() / 4;
+  }
+  const int pairs = *resident < total ? *resident : total;
+  if (used) *used = pairs;
+  cfg.gridDim = dim3(2 * pairs);
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  return int(cudaLaunchKernelEx(&cfg, kernel, args...));
+}
+
+static int ring2(Gemm2Args& a) {
+  int stages = (232448 - 1024 - 1024) / k2StageBytes;
+  if (stages > kMaxStages) stages = kMaxStages;
+  a.stages = stages;
+  return stages * k2StageBytes + 2048;
+}
+
 }  // namespace nkb
 
 using namespace nkb;
@@ -387,7 +489,6 @@ extern "C" int nkb_gemm_bf16_2cta(const void* A, const void* B, void* out, int m
   if ((splits - 1) * a.kb_per_split >= a.kb_total) return -2;       // an empty split would leave its partial unwritten
   a.split_stride = split_stride;
   a.static_b = static_b;
-  a.bias_on_cols = 1;
   static int group_m = 0;
   if (group_m == 0) {
     const char* e = getenv("NKIPY_B200_2CTA_GROUP");
@@ -400,45 +501,53 @@ extern "C" int nkb_gemm_bf16_2cta(const void* A, const void* B, void* out, int m
   a.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
   a.residual = reinterpret_cast<const __nv_bfloat16*>(residual);
   a.status = status_word();
-  int stages = (232448 - 1024 - 1024) / k2StageBytes;
-  if (stages > kMaxStages) stages = kMaxStages;
-  a.stages = stages;
-  const int smem = stages * k2StageBytes + 2048;
+  const int smem = ring2(a);
   CUtensorMap ta, tb;
   if (encode_tmap_bf16_2d(&ta, A, k, m, lda, kBlockK, kTileRows)) return -4;
   if (encode_tmap_bf16_2d(&tb, B, k, gated ? uint64_t(gate_off) + n : uint64_t(n), ldb, kBlockK, kTileRows)) return -4;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(gemm2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
-    if (e != cudaSuccess) return int(e);
-    attr_set = true;
-  }
-  const int total = a.tiles_m * a.tiles_n * splits;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(2 * (num_sms() / 2));
-  cfg.blockDim = dim3(kGemmThreads);
-  cfg.dynamicSmemBytes = size_t(smem);
-  cfg.stream = reinterpret_cast<cudaStream_t>(stream);
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  // The persistent loop strides by the number of pairs, so every pair must be resident at once: pairs need
-  // two SMs of one GPC, and not every SM can be paired.
-  static int max_pairs = 0;
-  if (max_pairs == 0) {
-    int n = 0;
-    cudaError_t e = cudaOccupancyMaxActiveClusters(&n, gemm2_kernel, &cfg);
-    max_pairs = (e == cudaSuccess && n > 0) ? n : num_sms() / 4;
-  }
-  int pairs = max_pairs < total ? max_pairs : total;
-  g_pairs_last = pairs;
-  cfg.gridDim = dim3(2 * pairs);
-  cfg.numAttrs = pdl_enabled() ? 2 : 1;
-  return int(cudaLaunchKernelEx(&cfg, gemm2_kernel, ta, tb, a));
+  static int resident = 0;
+  return launch_pairs(gemm2_kernel, &resident, a.tiles_m * a.tiles_n * splits, smem, reinterpret_cast<cudaStream_t>(stream),
+                      &g_pairs_last, ta, tb, a);
+}
+
+// Per-group products of rows sorted by group: out[r, :] = x[r] * w[g(r)]^T for the row tiles of 256 in tile_list (see
+// nkb_moe_dispatch).  w [groups, features (gated: gate_off + features), k], contiguous; bias as in nkb_gemm_bf16_grouped.
+extern "C" int nkb_gemm_bf16_2cta_grouped(const void* weights, const void* x_sorted, void* out, const int* group_offsets,
+                                          int num_groups, int features, int k, int total_rows, long long ldx, long long ldo,
+                                          int gated, int gate_off, const void* bias, long long bias_group_stride,
+                                          float act_limit, float act_alpha, const int* tile_list, const int* tile_count,
+                                          int max_tiles, void* stream) {
+  if (!status_word() && nkb_init() != 0) return -1;
+  if (num_groups <= 0 || features <= 0 || k <= 0 || total_rows <= 0) return 0;
+  if ((k & 7) || (ldx & 7) || !tile_list || !tile_count || max_tiles <= 0) return -2;
+  Gemm2Args a{};
+  a.m = total_rows; a.n = features; a.k = k;
+  a.tiles_n = gated ? (features + 127) / 128 : (features + 255) / 256;
+  a.gated = gated ? 1 : 0;
+  a.gate_off = gate_off;
+  a.kb_total = (k + kBlockK - 1) / kBlockK;
+  a.splits = 1;
+  a.kb_per_split = a.kb_total;
+  a.group_m = 1;
+  a.ldo = ldo;
+  a.out = out;
+  a.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
+  a.status = status_word();
+  Group2Args g{};
+  g.tile_list = tile_list;
+  g.tile_count = tile_count;
+  g.offsets = group_offsets;
+  const long long w_rows = gated ? (long long)gate_off + features : features;
+  if (w_rows * num_groups > 0x7fffffffll) return -2;
+  g.w_rows = int(w_rows);
+  g.bias_stride = bias_group_stride;
+  g.limit = act_limit;
+  g.alpha = act_alpha;
+  const int smem = ring2(a);
+  CUtensorMap ta, tb;
+  if (encode_tmap_bf16_2d(&ta, x_sorted, k, total_rows, ldx, kBlockK, kTileRows)) return -4;
+  if (encode_tmap_bf16_2d(&tb, weights, k, uint64_t(w_rows) * num_groups, k, kBlockK, kTileRows)) return -4;
+  static int resident = 0;
+  return launch_pairs(gemm2_grouped_kernel, &resident, max_tiles * a.tiles_n, smem, reinterpret_cast<cudaStream_t>(stream),
+                      nullptr, ta, tb, a, g);
 }

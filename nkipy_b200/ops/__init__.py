@@ -1108,8 +1108,14 @@ class MoEPlan:
         return iter((self.x_sorted, self.offsets, self.pair_pos))
 
 
-def moe_tile_widths(tokens: int):
-    """(gated GEMM tile width, down GEMM tile width) in tokens for a batch of `tokens`."""
+MOE_PAIR_ROWS = 64
+
+
+def moe_tile_widths(tokens: int, per_group: float = 0.0):
+    """(gated GEMM tile width, down GEMM tile width) in tokens for a batch of `tokens`, on average `per_group` of them in a
+    group.  256: row tiles of the CTA-pair kernel (gemm_2cta.cu)."""
+    if per_group >= MOE_PAIR_ROWS:
+        return 256, 256
     if tokens <= 512:
         return 32, 32
     return 64, 128
@@ -1147,7 +1153,7 @@ def moe_dispatch(x: torch.Tensor, experts: torch.Tensor, expert_lo: int, num_loc
         x_sorted[:n_local] = rows if weights is None else (rows.float() * weights.reshape(-1)[order[:n_local], None]).to(x.dtype)
         return MoEPlan(x_sorted, offsets, pair_pos, None, T, row_token)
     global _launches
-    bn_a, bn_b = moe_tile_widths(T)
+    bn_a, bn_b = moe_tile_widths(T, pairs / num_local)
     cap_a, cap_b = num_local + pairs // bn_a + 1, num_local + pairs // bn_b + 1
     if weights is not None and (not gather or weights.dtype != torch.float32 or not weights.is_contiguous()):
         raise ValueError("weights are contiguous fp32 and scale gathered rows")
@@ -1219,6 +1225,15 @@ def grouped_linear(x_sorted: torch.Tensor, w: torch.Tensor, offsets: torch.Tenso
         out = torch.empty((R, N), dtype=torch.bfloat16, device=x_sorted.device)
     tl = tc = None
     max_tiles = 0
+    if tiles is not None and 256 in tiles:
+        tl_t, tc_t, max_tiles = tiles[256]
+        rc = _lib.lib().nkb_gemm_bf16_2cta_grouped(
+            w.data_ptr(), x_sorted.data_ptr(), out.data_ptr(), offsets.data_ptr(), G, N, K, R, x_sorted.stride(0), out.stride(0),
+            1 if gated else 0, N if gated else 0, _ptr(bias), bias.stride(0) if bias is not None else 0, float(act_limit),
+            float(act_alpha), tl_t.data_ptr(), tc_t.data_ptr(), int(max_tiles), _stream())
+        _lib.check(rc, "nkb_gemm_bf16_2cta_grouped")
+        _launches += 1
+        return out
     if tiles is not None:
         bn_a, bn_b = moe_tile_widths(max_rows_per_group)
         block_n = bn_a if gated else bn_b

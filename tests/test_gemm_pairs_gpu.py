@@ -50,3 +50,37 @@ def test_plan_leaves_no_split_empty():
             slabs = -(-k // 64)
             assert swap == (rows <= 128) and 1 <= splits <= 8
             assert splits == 1 or swap or -(-slabs // -(-slabs // splits)) == splits
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tokens,experts,top,width,inner", [(300, 4, 2, 256, 136), (1500, 5, 2, 264, 384), (257, 3, 3, 512, 104)])
+@pytest.mark.parametrize("limit", [0.0, 7.0])
+def test_grouped_products_on_pairs(tokens, experts, top, width, inner, limit):
+    """Experts with at least 64 rows on average: unequal groups, one of them empty, sizes off the tiles, biases and clamped gates."""
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    rnd = lambda *shape, s=1.0: (s * torch.randn(shape, generator=g, device="cuda")).to(torch.bfloat16)
+    x, w1, w2 = rnd(tokens, width), rnd(experts, 2 * inner, width, s=0.1), rnd(experts, width, inner, s=0.1)
+    b1, b2 = rnd(experts, 2 * inner), rnd(experts, width)
+    pick = torch.rand((tokens, experts), generator=g, device="cuda").argsort(1)[:, :top].to(torch.int32)
+    if experts > top:
+        pick[pick == experts - 1] = 0                 # an empty group, and a token that names one expert twice
+    plan = ops.moe_dispatch(x, pick, 0, experts)
+    assert 256 in plan.tiles
+    off = plan.offsets.tolist()
+    h = ops.grouped_linear(plan.x_sorted, w1, plan.offsets, max_rows_per_group=tokens, gated=True, bias=b1, act_limit=limit,
+                           tiles=plan.tiles)
+    y = ops.grouped_linear(h, w2, plan.offsets, max_rows_per_group=tokens, bias=b2, tiles=plan.tiles)
+    for e in range(experts):
+        rows = slice(off[e], off[e + 1])
+        z = plan.x_sorted[rows].double() @ w1[e].double().T + b1[e].double()
+        a, u = z[:, :inner], z[:, inner:]
+        if limit:
+            a, u = a.clamp(max=limit), u.clamp(-limit, limit) + 1
+            want = u * a * torch.sigmoid(1.702 * a)
+        else:
+            want = torch.nn.functional.silu(a) * u
+        # one rounding to bf16; sums and the approximate exponential are far below it
+        assert ((h[rows].double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-3).all()
+        want = h[rows].double() @ w2[e].double().T + b2[e].double()
+        assert ((y[rows].double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-3).all()
+    ops.raise_on_device_error()
