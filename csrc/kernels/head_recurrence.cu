@@ -571,14 +571,15 @@ static int launch_rec(const NkbHeadRec& p, bool async, cudaStream_t s) {
 }
 
 // ------------------------------------------------------------------------------------------------ step
-constexpr int kRecStepThreads = 256;
-constexpr int kRecStepBlocks = 4;   // column blocks of 32 in flight
-
-template <int CH, bool DELTA, typename OutT>
-__global__ void __launch_bounds__(kRecStepThreads) head_rec_step_kernel(const __grid_constant__ NkbHeadRec p) {
-  constexpr int D8 = 8 * CH;
+// TH threads hold 128 columns of the state at a time, in blocks of TH / 8.  Bound by streaming the state twice; what keeps it from
+// that is the time in which a CTA's loads are back and the convolution, norms and gates of its head are not.  512 threads with
+// half the columns each do that part in one pass and hold two heads per SM in 64 registers a thread: 64 sequences of 32 heads of
+// 128 x 128, 84 -> 79 us with the delta rule and 78 -> 65 us without (256 threads held one head per SM).
+template <int TH, int CH, bool DELTA, typename OutT>
+__global__ void __launch_bounds__(TH, TH == 512 ? 2 : 1) head_rec_step_kernel(const __grid_constant__ NkbHeadRec p) {
+  constexpr int D8 = 8 * CH, kCols = TH / 8, kBlocks = 128 / kCols;
   __shared__ __align__(16) float qs[D8], ks[D8];
-  __shared__ float red[kRecStepThreads / 32], gates[3];      // decay, step size, write strength
+  __shared__ float red[TH / 32], gates[3];      // decay, step size, write strength
   extern __shared__ float dyn[];                    // v, o, norm weight times gate [vdim] each
   float* vs = dyn;
   float* os = dyn + p.vdim;
@@ -597,7 +598,7 @@ __global__ void __launch_bounds__(kRecStepThreads) head_rec_step_kernel(const __
   };
   const int ctx = p.context_lens[b];
   if (ctx <= 0) {
-    for (int c = threadIdx.x; c < p.vdim; c += kRecStepThreads) put(c, 0.f);
+    for (int c = threadIdx.x; c < p.vdim; c += TH) put(c, 0.f);
     return;
   }
   const int slot = p.slot_ids ? p.slot_ids[b] : b, pos = ctx - 1;
@@ -613,13 +614,13 @@ __global__ void __launch_bounds__(kRecStepThreads) head_rec_step_kernel(const __
     if (owner) ring[(long long)(pos % p.taps) * p.channels + c] = x;
     return y / (1.f + expf(-y));
   };
-  const int nblk = (p.vdim + 31) / 32;
+  const int nblk = (p.vdim + kCols - 1) / kCols;
   float g_t = 0.f, ev = 0.f, es = 0.f, oq = 0.f, ou = 0.f;
-  for (int b0 = 0; b0 < nblk; b0 += kRecStepBlocks) {
-    float4 S[kRecStepBlocks][CH / 4];
+  for (int b0 = 0; b0 < nblk; b0 += kBlocks) {
+    float4 S[kBlocks][CH / 4];
 #pragma unroll
-    for (int k = 0; k < kRecStepBlocks; ++k) {
-      const int col = (b0 + k) * 32 + cl;
+    for (int k = 0; k < kBlocks; ++k) {
+      const int col = (b0 + k) * kCols + cl;
 #pragma unroll
       for (int j = 0; j < CH / 4; ++j) {
         const int c = (j * 8 + g) * 4;
@@ -629,7 +630,7 @@ __global__ void __launch_bounds__(kRecStepThreads) head_rec_step_kernel(const __
       }
     }
     if (b0 == 0) {
-      for (int i = threadIdx.x; i < 2 * D8 + p.vdim; i += kRecStepThreads) {
+      for (int i = threadIdx.x; i < 2 * D8 + p.vdim; i += TH) {
         if (i < 2 * D8) {
           const int c = i < D8 ? i : i - D8;
           const float y = c < p.dim ? channel((i < D8 ? p.q_col : p.k_col) + kvh * p.dim + c, head % per == 0) : 0.f;
@@ -640,7 +641,7 @@ __global__ void __launch_bounds__(kRecStepThreads) head_rec_step_kernel(const __
           if (finish) gs[c] = p.norm_w[c] * apply_act(proj_load(p.g, b, hv + c), p.gate_act);
         }
       }
-      if (threadIdx.x == kRecStepThreads - 1) {
+      if (threadIdx.x == TH - 1) {
         const float dt = softplus_f(proj_load(p.a, b, head) + p.dt_bias[head]);
         gates[0] = expf(-p.rate[head] * dt);
         gates[1] = dt;
@@ -670,8 +671,8 @@ __global__ void __launch_bounds__(kRecStepThreads) head_rec_step_kernel(const __
       }
     }
 #pragma unroll
-    for (int k = 0; k < kRecStepBlocks; ++k) {
-      const int col = (b0 + k) * 32 + cl;
+    for (int k = 0; k < kBlocks; ++k) {
+      const int col = (b0 + k) * kCols + cl;
       const bool ok = col < p.vdim;
       const float v = ok ? vs[col] : 0.f;
       float sk = 0.f, sq = 0.f;
@@ -713,31 +714,31 @@ __global__ void __launch_bounds__(kRecStepThreads) head_rec_step_kernel(const __
   }
   __syncthreads();
   if (!finish) {
-    for (int c = threadIdx.x; c < p.vdim; c += kRecStepThreads) put(c, os[c]);
+    for (int c = threadIdx.x; c < p.vdim; c += TH) put(c, os[c]);
     return;
   }
   float ss = 0.f;
-  for (int c = threadIdx.x; c < p.vdim; c += kRecStepThreads) ss += os[c] * os[c];
+  for (int c = threadIdx.x; c < p.vdim; c += TH) ss += os[c] * os[c];
   ss = warp_sum(ss);
   if (lane == 0) red[warp] = ss;
   __syncthreads();
   float tot = 0.f;
 #pragma unroll
-  for (int w = 0; w < kRecStepThreads / 32; ++w) tot += red[w];
+  for (int w = 0; w < TH / 32; ++w) tot += red[w];
   const float inv = 1.f / sqrtf(tot / float(p.vdim) + p.eps);
-  for (int c = threadIdx.x; c < p.vdim; c += kRecStepThreads) put(c, os[c] * inv * gs[c]);
+  for (int c = threadIdx.x; c < p.vdim; c += TH) put(c, os[c] * inv * gs[c]);
 }
 
-template <int CH>
+template <int TH, int CH>
 static int launch_rec_step(const NkbHeadRec& p, cudaStream_t s) {
-  const dim3 grid(p.heads, p.batch), block(kRecStepThreads);
+  const dim3 grid(p.heads, p.batch), block(TH);
   const size_t smem = size_t(3 * p.vdim) * sizeof(float);
   using bf = __nv_bfloat16;
   if (p.b.ptr)
-    return p.bf16 ? launch_pdl(head_rec_step_kernel<CH, true, bf>, grid, block, smem, s, p)
-                  : launch_pdl(head_rec_step_kernel<CH, true, float>, grid, block, smem, s, p);
-  return p.bf16 ? launch_pdl(head_rec_step_kernel<CH, false, bf>, grid, block, smem, s, p)
-                : launch_pdl(head_rec_step_kernel<CH, false, float>, grid, block, smem, s, p);
+    return p.bf16 ? launch_pdl(head_rec_step_kernel<TH, CH, true, bf>, grid, block, smem, s, p)
+                  : launch_pdl(head_rec_step_kernel<TH, CH, true, float>, grid, block, smem, s, p);
+  return p.bf16 ? launch_pdl(head_rec_step_kernel<TH, CH, false, bf>, grid, block, smem, s, p)
+                : launch_pdl(head_rec_step_kernel<TH, CH, false, float>, grid, block, smem, s, p);
 }
 
 // ------------------------------------------------------------------------------------------------ group norm
@@ -911,10 +912,10 @@ extern "C" int nkb_head_rec_step(const NkbHeadRec* a, void* stream) {
       a->gate_act < 0 || a->gate_act >= ACT_CLAMPED)
     return -2;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  if (a->dim <= 32) return launch_rec_step<4>(*a, s);
-  if (a->dim <= 64) return launch_rec_step<8>(*a, s);
-  if (a->dim <= 128) return launch_rec_step<16>(*a, s);
-  return launch_rec_step<32>(*a, s);
+  if (a->dim <= 32) return launch_rec_step<256, 4>(*a, s);
+  if (a->dim <= 64) return launch_rec_step<512, 8>(*a, s);
+  if (a->dim <= 128) return launch_rec_step<512, 16>(*a, s);
+  return launch_rec_step<256, 32>(*a, s);
 }
 
 extern "C" int nkb_gated_group_norm(const void* y, int y_bf16, const NkbProj* gate, int gate_act, const float* w, float eps,
