@@ -30,35 +30,43 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 
 // h = sum_s partials[s] (+ x) (+ bias) (+ residual_in);  residual_out = h;
 // normed_out = h * rsqrt(mean(h^2) + eps) * w        (skipped when w == nullptr)
-__global__ void add_rmsnorm_kernel(const float* __restrict__ partials, int splits, long long split_stride,
-                                   const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ residual_in,
-                                   const __nv_bfloat16* __restrict__ bias, const __nv_bfloat16* __restrict__ w,
-                                   __nv_bfloat16* __restrict__ residual_out, __nv_bfloat16* __restrict__ normed_out,
-                                   int hidden, float eps) {
+// Bound by latency in a decode step: everything a thread reads is on its way before the first sum (the norm weight behind the
+// barriers, and the residual behind the partials, each cost one more round trip).  IT: pieces of eight elements per thread.
+template <int IT>
+__global__ void __launch_bounds__(1024) add_rmsnorm_kernel(
+    const float* __restrict__ partials, int splits, long long split_stride, const __nv_bfloat16* __restrict__ x,
+    const __nv_bfloat16* __restrict__ residual_in, const __nv_bfloat16* __restrict__ bias, const __nv_bfloat16* __restrict__ w,
+    __nv_bfloat16* __restrict__ residual_out, __nv_bfloat16* __restrict__ normed_out, int hidden, float eps) {
   __shared__ float red[32];
   const long long row = blockIdx.x;
   const int nvec = hidden >> 3;
   griddep_wait();
   griddep_launch();
-  float h[kNormMaxIters][8];
+  float h[IT][8];
+  uint4 wr[IT];
   float ss = 0.f;
 #pragma unroll
-  for (int it = 0; it < kNormMaxIters; ++it) {
+  for (int it = 0; it < IT; ++it) {
     const int v = threadIdx.x + it * blockDim.x;
     if (v < nvec) {
       const long long off = row * hidden + (long long)v * 8;
+      const uint4 none = make_uint4(0u, 0u, 0u, 0u);
+      const uint4 rr = residual_in ? *reinterpret_cast<const uint4*>(residual_in + off) : none;
+      const uint4 xr = x ? *reinterpret_cast<const uint4*>(x + off) : none;
+      const uint4 br = bias ? *reinterpret_cast<const uint4*>(bias + (long long)v * 8) : none;
+      wr[it] = w ? *reinterpret_cast<const uint4*>(w + (long long)v * 8) : none;
       float a[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) a[j] = 0.f;
+#pragma unroll 4
       for (int s = 0; s < splits; ++s) {
         const float4* p = reinterpret_cast<const float4*>(partials + s * split_stride + off);
         float4 p0 = p[0], p1 = p[1];
         a[0] += p0.x; a[1] += p0.y; a[2] += p0.z; a[3] += p0.w;
         a[4] += p1.x; a[5] += p1.y; a[6] += p1.z; a[7] += p1.w;
       }
-      auto add_bf16 = [&](const __nv_bfloat16* src, long long o) {
-        uint4 r = *reinterpret_cast<const uint4*>(src + o);
-        uint32_t rw[4] = {r.x, r.y, r.z, r.w};
+      auto add_bf16 = [&](const uint4& r) {
+        const uint32_t rw[4] = {r.x, r.y, r.z, r.w};
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           float2 f = unpack_bf16x2(rw[e]);
@@ -66,9 +74,9 @@ __global__ void add_rmsnorm_kernel(const float* __restrict__ partials, int split
           a[2 * e + 1] += f.y;
         }
       };
-      if (x) add_bf16(x, off);
-      if (bias) add_bf16(bias, (long long)v * 8);
-      if (residual_in) add_bf16(residual_in, off);
+      if (x) add_bf16(xr);
+      if (bias) add_bf16(br);
+      if (residual_in) add_bf16(rr);
       if (residual_out) {
         uint4 o;
         o.x = pack_bf16x2(a[0], a[1]); o.y = pack_bf16x2(a[2], a[3]);
@@ -95,20 +103,84 @@ __global__ void add_rmsnorm_kernel(const float* __restrict__ partials, int split
   const float tot = block_sum(ss, red);
   const float inv = rsqrtf(tot / float(hidden) + eps);
 #pragma unroll
-  for (int it = 0; it < kNormMaxIters; ++it) {
+  for (int it = 0; it < IT; ++it) {
     const int v = threadIdx.x + it * blockDim.x;
     if (v < nvec) {
-      const long long off = row * hidden + (long long)v * 8;
-      uint4 wr = *reinterpret_cast<const uint4*>(w + (long long)v * 8);
-      uint32_t ww[4] = {wr.x, wr.y, wr.z, wr.w};
+      const uint32_t ww[4] = {wr[it].x, wr[it].y, wr[it].z, wr[it].w};
       uint32_t o[4];
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         float2 f = unpack_bf16x2(ww[e]);
         o[e] = pack_bf16x2(h[it][2 * e] * inv * f.x, h[it][2 * e + 1] * inv * f.y);
       }
-      *reinterpret_cast<uint4*>(normed_out + off) = make_uint4(o[0], o[1], o[2], o[3]);
+      *reinterpret_cast<uint4*>(normed_out + row * hidden + (long long)v * 8) = make_uint4(o[0], o[1], o[2], o[3]);
     }
+  }
+}
+
+// The same without partial sums and bias for many rows: one warp owns a row and has all of it in flight, V pieces of sixteen bytes
+// per lane, and no barrier.  Bound by memory; a block per row (the kernel above) spends most of its time between its loads, its
+// two barriers and the launch of the next block.  16384 x 4096: 141 us as blocks, 76 us as rows (0.54 of the copy bandwidth).
+// residual_in needs residual_out: what is kept in registers is the rounded stream.
+template <int V>
+__global__ void __launch_bounds__(128, V > 12 ? 3 : 4) rmsnorm_rows_kernel(const __nv_bfloat16* __restrict__ x,
+                                                           const __nv_bfloat16* __restrict__ residual_in,
+                                                           const __nv_bfloat16* __restrict__ w,
+                                                           __nv_bfloat16* __restrict__ residual_out,
+                                                           __nv_bfloat16* __restrict__ normed_out, int rows, int hidden,
+                                                           float eps) {
+  const int lane = threadIdx.x & 31, nvec = hidden >> 3;
+  griddep_wait();
+  griddep_launch();
+  const long long row = blockIdx.x * 4ll + (threadIdx.x >> 5);
+  if (row >= rows) return;
+  const uint4* src = reinterpret_cast<const uint4*>(x + row * hidden);
+  uint4 h[V];
+#pragma unroll
+  for (int i = 0; i < V; ++i) h[i] = lane + 32 * i < nvec ? src[lane + 32 * i] : make_uint4(0u, 0u, 0u, 0u);
+  if (residual_in) {
+    const uint4* res = reinterpret_cast<const uint4*>(residual_in + row * hidden);
+    uint4* dst = reinterpret_cast<uint4*>(residual_out + row * hidden);
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      if (lane + 32 * i >= nvec) break;
+      const uint4 r = res[lane + 32 * i];
+      const uint32_t rw[4] = {r.x, r.y, r.z, r.w}, hw[4] = {h[i].x, h[i].y, h[i].z, h[i].w};
+      uint32_t o[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 a = unpack_bf16x2(hw[e]), b = unpack_bf16x2(rw[e]);
+        o[e] = pack_bf16x2(a.x + b.x, a.y + b.y);
+      }
+      h[i] = make_uint4(o[0], o[1], o[2], o[3]);
+      dst[lane + 32 * i] = h[i];
+    }
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    const uint32_t hw[4] = {h[i].x, h[i].y, h[i].z, h[i].w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 a = unpack_bf16x2(hw[e]);
+      ss = fmaf(a.x, a.x, ss);
+      ss = fmaf(a.y, a.y, ss);
+    }
+  }
+  const float inv = rsqrtf(warp_sum(ss) / float(hidden) + eps);
+  uint4* dst = reinterpret_cast<uint4*>(normed_out + row * hidden);
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    if (lane + 32 * i >= nvec) break;
+    const uint4 wr = __ldg(reinterpret_cast<const uint4*>(w) + lane + 32 * i);
+    const uint32_t ww[4] = {wr.x, wr.y, wr.z, wr.w}, hw[4] = {h[i].x, h[i].y, h[i].z, h[i].w};
+    uint32_t o[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 a = unpack_bf16x2(hw[e]), f = unpack_bf16x2(ww[e]);
+      o[e] = pack_bf16x2(a.x * inv * f.x, a.y * inv * f.y);
+    }
+    dst[lane + 32 * i] = make_uint4(o[0], o[1], o[2], o[3]);
   }
 }
 
@@ -297,6 +369,120 @@ __global__ void rope_kv_append_kernel(const __nv_bfloat16* __restrict__ qkv, con
   }
 }
 
+// The same in pieces of sixteen bytes: D / 16 lanes share a head, each with eight elements of its first half and the eight that
+// turn with them, so a warp takes four heads of 128.  Bound by memory; with two elements per access (the kernel above) it is
+// bound by instructions.  16384 tokens of 32 + 16 heads of 128: 214 -> 94 us.  Every pointer on 16 bytes, split_stride a multiple of four.
+template <int D>
+__global__ void __launch_bounds__(256) rope_kv_append8_kernel(
+    const __nv_bfloat16* __restrict__ qkv, const float* __restrict__ partials, int splits, long long split_stride,
+    const __nv_bfloat16* __restrict__ bias, const int* __restrict__ positions, const int* __restrict__ slots,
+    const float* __restrict__ cos_sin, const __nv_bfloat16* __restrict__ q_norm_w, const __nv_bfloat16* __restrict__ k_norm_w,
+    float norm_eps, __nv_bfloat16* __restrict__ q_out, __nv_bfloat16* __restrict__ k_cache, __nv_bfloat16* __restrict__ v_cache,
+    int tokens, int nq, int nkv, int max_pos, int block_size) {
+  constexpr int L = D / 16;
+  const int heads = nq + 2 * nkv;
+  const long long unit = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / L;
+  const int i0 = (threadIdx.x % L) * 8;
+  griddep_wait();
+  griddep_launch();
+  // a warp's lanes leave together or stay for the sums: units past the end repeat the last one and store nothing
+  const bool on = unit < (long long)tokens * heads;
+  const long long u = on ? unit : (long long)tokens * heads - 1;
+  const int t = int(u / heads), h = int(u % heads);
+  const long long base = (long long)t * heads * D + (long long)h * D + i0;
+  float lo[8], hi[8];
+  auto get8 = [](const __nv_bfloat16* src, float (&o)[8]) {
+    const uint4 r = *reinterpret_cast<const uint4*>(src);
+    const uint32_t rw[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 f = unpack_bf16x2(rw[e]);
+      o[2 * e] = f.x;
+      o[2 * e + 1] = f.y;
+    }
+  };
+  if (partials) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) lo[j] = hi[j] = 0.f;
+#pragma unroll 2
+    for (int s = 0; s < splits; ++s) {
+      const float4* a = reinterpret_cast<const float4*>(partials + s * split_stride + base);
+      const float4* b = reinterpret_cast<const float4*>(partials + s * split_stride + base + D / 2);
+      const float4 a0 = a[0], a1 = a[1], b0 = b[0], b1 = b[1];
+      lo[0] += a0.x; lo[1] += a0.y; lo[2] += a0.z; lo[3] += a0.w;
+      lo[4] += a1.x; lo[5] += a1.y; lo[6] += a1.z; lo[7] += a1.w;
+      hi[0] += b0.x; hi[1] += b0.y; hi[2] += b0.z; hi[3] += b0.w;
+      hi[4] += b1.x; hi[5] += b1.y; hi[6] += b1.z; hi[7] += b1.w;
+    }
+  } else {
+    get8(qkv + base, lo);
+    get8(qkv + base + D / 2, hi);
+  }
+  if (bias) {
+    float a[8], b[8];
+    get8(bias + h * D + i0, a);
+    get8(bias + h * D + D / 2 + i0, b);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      lo[j] += a[j];
+      hi[j] += b[j];
+    }
+  }
+  const bool is_q = h < nq, is_k = !is_q && h < nq + nkv;
+  if (q_norm_w || k_norm_w) {
+    const __nv_bfloat16* nw = is_q ? q_norm_w : (is_k ? k_norm_w : nullptr);
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) ss += lo[j] * lo[j] + hi[j] * hi[j];
+#pragma unroll
+    for (int m = L / 2; m > 0; m >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, m);
+    if (nw) {
+      const float inv = rsqrtf(ss / float(D) + norm_eps);
+      float a[8], b[8];
+      get8(nw + i0, a);
+      get8(nw + D / 2 + i0, b);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        // round to bf16 after the norm like an unfused implementation would
+        lo[j] = __bfloat162float(__float2bfloat16(lo[j] * inv * a[j]));
+        hi[j] = __bfloat162float(__float2bfloat16(hi[j] * inv * b[j]));
+      }
+    }
+  }
+  if ((is_q || is_k) && cos_sin) {
+    int pos = positions[t];
+    pos = pos < 0 ? 0 : (pos >= max_pos ? max_pos - 1 : pos);
+    const float* cs = cos_sin + (long long)pos * D + i0;  // [cos(d/2) | sin(d/2)]
+    float c[8], sn[8];
+#pragma unroll
+    for (int j = 0; j < 8; j += 4) {
+      *reinterpret_cast<float4*>(c + j) = *reinterpret_cast<const float4*>(cs + j);
+      *reinterpret_cast<float4*>(sn + j) = *reinterpret_cast<const float4*>(cs + D / 2 + j);
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float a = lo[j], b = hi[j];
+      lo[j] = a * c[j] - b * sn[j];
+      hi[j] = b * c[j] + a * sn[j];
+    }
+  }
+  if (!on) return;
+  __nv_bfloat16* dst;
+  if (is_q) {
+    dst = q_out + (long long)t * nq * D + (long long)h * D;
+  } else {
+    const int slot = slots ? slots[t] : -1;
+    if (slot < 0) return;
+    const int kh = is_k ? h - nq : h - nq - nkv;
+    const long long blk = slot / block_size, off = slot % block_size;
+    dst = (is_k ? k_cache : v_cache) + ((blk * nkv + kh) * block_size + off) * D;
+  }
+  *reinterpret_cast<uint4*>(dst + i0) =
+      make_uint4(pack_bf16x2(lo[0], lo[1]), pack_bf16x2(lo[2], lo[3]), pack_bf16x2(lo[4], lo[5]), pack_bf16x2(lo[6], lo[7]));
+  *reinterpret_cast<uint4*>(dst + D / 2 + i0) =
+      make_uint4(pack_bf16x2(hi[0], hi[1]), pack_bf16x2(hi[2], hi[3]), pack_bf16x2(hi[4], hi[5]), pack_bf16x2(hi[6], hi[7]));
+}
+
 }  // namespace nkb
 
 using namespace nkb;
@@ -314,7 +500,20 @@ extern "C" int nkb_add_rmsnorm(const float* partials, int splits, long long spli
   if (nvec <= 1024) threads = (nvec + 31) / 32 * 32;
   if (threads > 1024) threads = 1024;
   if (!partials) splits = 0;
-  return launch_pdl(add_rmsnorm_kernel, dim3(rows), dim3(threads), 0, S(stream), partials, splits, split_stride,
+  // From about seven warps per SM on a row per warp; fewer rows need the loads of a whole block per row in flight.
+  const int lane_vecs = (nvec + 31) / 32;
+  if (!partials && x && !bias && w && normed_out && rows >= 1024 && lane_vecs <= 16 && !residual_in == !residual_out) {
+    const dim3 grid((rows + 3) / 4), block(128);
+    auto go = [&](auto kernel) {
+      return launch_pdl(kernel, grid, block, 0, S(stream), (const __nv_bfloat16*)x, (const __nv_bfloat16*)residual_in,
+                        (const __nv_bfloat16*)w, (__nv_bfloat16*)residual_out, (__nv_bfloat16*)normed_out, rows, hidden, eps);
+    };
+    if (lane_vecs <= 4) return go(rmsnorm_rows_kernel<4>);
+    if (lane_vecs <= 8) return go(rmsnorm_rows_kernel<8>);
+    if (lane_vecs <= 12) return go(rmsnorm_rows_kernel<12>);
+    return go(rmsnorm_rows_kernel<16>);
+  }
+  return launch_pdl(nvec <= 1024 ? add_rmsnorm_kernel<1> : add_rmsnorm_kernel<kNormMaxIters>, dim3(rows), dim3(threads), 0, S(stream), partials, splits, split_stride,
                     (const __nv_bfloat16*)x, (const __nv_bfloat16*)residual_in, (const __nv_bfloat16*)bias,
                     (const __nv_bfloat16*)w, (__nv_bfloat16*)residual_out, (__nv_bfloat16*)normed_out, hidden, eps);
 }
@@ -361,9 +560,16 @@ extern "C" int nkb_rope_kv_append(const void* qkv_bf16, const float* qkv_partial
   if (tokens <= 0) return 0;
   const long long warps = (long long)tokens * (nq + 2 * nkv);
   const int threads = 256;
-  const long long blocks = (warps * 32 + threads - 1) / threads;
+  // Sixteen-byte pieces once there are enough units to fill the SMs; a decode-sized batch is bound by latency and keeps a warp per
+  // head.
+  uintptr_t at = 0;
+  for (const void* p : {qkv_bf16, (const void*)qkv_partials, bias, (const void*)cos_sin, q_norm_w, k_norm_w, (const void*)q_out,
+                        (const void*)k_cache, (const void*)v_cache})
+    at |= reinterpret_cast<uintptr_t>(p);
+  const bool pieces = tokens >= 256 && (at & 15) == 0 && (!qkv_partials || (split_stride & 3) == 0);
+  const long long blocks = pieces ? (warps * (head_dim / 16) + threads - 1) / threads : (warps * 32 + threads - 1) / threads;
 #define NKB_ROPE(D)                                                                                               \
-  return launch_pdl(rope_kv_append_kernel<D>, dim3((unsigned)blocks), dim3(threads), 0, S(stream),                \
+  return launch_pdl(pieces ? rope_kv_append8_kernel<D> : rope_kv_append_kernel<D>, dim3((unsigned)blocks), dim3(threads), 0, S(stream), \
                     (const __nv_bfloat16*)qkv_bf16, qkv_partials, splits, split_stride,                           \
                     (const __nv_bfloat16*)bias, positions, slots, cos_sin, (const __nv_bfloat16*)q_norm_w,        \
                     (const __nv_bfloat16*)k_norm_w, norm_eps, (__nv_bfloat16*)q_out, (__nv_bfloat16*)k_cache,     \

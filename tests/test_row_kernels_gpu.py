@@ -1,0 +1,85 @@
+"""Row-per-warp norms, RoPE in sixteen-byte pieces and argmax with several accesses ahead, against the CPU statement of the same
+operators, around the sizes where the kernels change."""
+import pytest
+import torch
+
+from nkipy_b200 import ops
+
+pytestmark = pytest.mark.gpu
+
+
+def rnd(*shape, seed=0, s=1.0):
+    return (s * torch.randn(shape, generator=torch.Generator().manual_seed(seed + sum(shape)))).to(torch.bfloat16)
+
+
+def close(got, want):
+    # both round once to bf16; the fp32 value before that may differ by the order of a sum and an approximate square root
+    got, want = got.float().cpu(), want.float()
+    assert ((got - want).abs() <= 2.0 ** -7 * want.abs() + 1e-6).all()
+
+
+@pytest.mark.parametrize("rows", [1023, 1024, 1027, 2500])
+@pytest.mark.parametrize("hidden", [8, 264, 1024, 2048, 2056, 2880, 4096, 4104])
+@pytest.mark.parametrize("residual", [False, True])
+def test_norms(rows, hidden, residual):
+    x, r, w = rnd(rows, hidden), rnd(rows, hidden, seed=1), rnd(hidden, seed=2)
+    want = ops.add_rmsnorm(x, w, residual_in=r if residual else None)
+    got = ops.add_rmsnorm(x.cuda(), w.cuda(), residual_in=r.cuda() if residual else None)
+    if residual:
+        assert torch.equal(got[0].cpu(), want[0])
+    close(got[1], want[1])
+
+
+@pytest.mark.parametrize("hidden,splits", [(4096, 8), (4096, 3), (2880, 5), (8200, 2)])
+def test_norm_of_partials(hidden, splits):
+    p = torch.randn((splits, 9, hidden), generator=torch.Generator().manual_seed(4))
+    r, w, b = rnd(9, hidden), rnd(hidden, seed=2), rnd(hidden, seed=3)
+    want = ops.add_rmsnorm(None, w, residual_in=r, partials=p, bias=b)
+    got = ops.add_rmsnorm(None, w.cuda(), residual_in=r.cuda(), partials=p.cuda(), bias=b.cuda())
+    # sums in another order may round the stream differently
+    assert ((got[0].float().cpu() - want[0].float()).abs() <= 2.0 ** -7 * want[0].float().abs() + 1e-5).all()
+    assert (got[1].float().cpu() - want[1].float()).norm() <= 2.0 ** -8 * want[1].float().norm()
+
+
+@pytest.mark.parametrize("tokens", [255, 256, 301])
+@pytest.mark.parametrize("dim,nq,nkv", [(64, 6, 2), (128, 4, 1), (128, 5, 2), (256, 2, 1)])
+@pytest.mark.parametrize("splits", [0, 3])
+@pytest.mark.parametrize("norm,bias,shift", [(True, True, 0), (False, False, 0), (False, True, 1)])
+def test_rope_append(tokens, dim, nq, nkv, splits, norm, bias, shift):
+    """shift 1: a bias that does not start on sixteen bytes (the general kernel)."""
+    width, bs, blocks = (nq + 2 * nkv) * dim, 32, 12
+    qkv = (torch.randn((splits, tokens, width), generator=torch.Generator().manual_seed(dim)) if splits
+           else rnd(tokens, width, seed=dim))
+    pos = torch.randint(0, 700, (tokens,), generator=torch.Generator().manual_seed(1)).to(torch.int32)
+    slots = torch.randperm(blocks * bs, generator=torch.Generator().manual_seed(2))[:tokens].to(torch.int32)
+    slots[5] = -1
+    table = ops.rope_table(dim, 700)
+    qw, kw = (rnd(dim, seed=5), rnd(dim, seed=6)) if norm else (None, None)
+    b = rnd(width + 1, seed=7)[shift:shift + width] if bias else None
+    outs = []
+    for dev in ("cpu", "cuda"):
+        k = torch.zeros((blocks, nkv, bs, dim), dtype=torch.bfloat16, device=dev)
+        v = torch.zeros_like(k)
+        to = lambda t: None if t is None else t.to(dev)
+        bd = None if b is None else rnd(width + 1, seed=7).to(dev)[shift:shift + width]
+        q = ops.rope_kv_append(qkv.to(dev), pos.to(dev), slots.to(dev), table.to(dev), k, v, nq, nkv, dim, bias=bd, q_norm_w=to(qw),
+                               k_norm_w=to(kw), norm_eps=1e-6)
+        outs.append((q, k, v))
+    for got, want in zip(outs[1], outs[0]):
+        got, want = got.float().cpu(), want.float()
+        # the norm is rounded to bf16 before the rotation: a rounding that falls the other way is a unit of either operand
+        assert ((got - want).abs() <= 2.0 ** -6 * want.abs() + 2.0 ** -6).all()
+        assert (got - want).norm() <= 2.0 ** -8 * want.norm()
+
+
+@pytest.mark.parametrize("rows,vocab", [(1, 128256), (3, 4099), (2, 8), (5, 1003), (1, 201088)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_argmax(rows, vocab, dtype):
+    z = torch.randn((rows, vocab), generator=torch.Generator().manual_seed(vocab)).to(dtype)
+    z[0, vocab - 1] = z[0, vocab // 2] = 50.0         # a tie: the first wins
+    assert torch.equal(ops.argmax(z.cuda()).cpu().long(), z.float().argmax(-1))
+    z[0, vocab // 2 - 1] = float("nan")               # loses against any number
+    z[rows - 1, :] = -0.0
+    z[rows - 1, vocab // 3:] = 0.0                    # zeros of either sign are a tie
+    got = ops.argmax(z.cuda()).cpu().tolist()
+    assert got[rows - 1] == 0 and (rows == 1 or got[0] == vocab // 2)
