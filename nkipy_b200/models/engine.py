@@ -20,6 +20,7 @@ import time
 from dataclasses import dataclass, field
 from typing import Dict, List, Optional, Sequence
 
+import numpy as np
 import torch
 
 from .. import ops
@@ -79,6 +80,19 @@ class Sampling:
     seed: int = 0
 
 
+def _token_array(tokens: Sequence[int]) -> np.ndarray:
+    """Token ids as int32."""
+    try:
+        a = np.asarray(tokens)
+    except (TypeError, ValueError, RuntimeError):
+        a = None
+    if a is None or a.dtype.kind not in "iu" or a.ndim != 1:
+        a = np.array([int(t) for t in tokens], dtype=np.int64)
+    if a.size and not -2 ** 31 <= int(a.min()) <= int(a.max()) < 2 ** 31:
+        raise ValueError("token ids are 32-bit numbers")
+    return a.astype(np.int32)
+
+
 class GenerationEngine:
     """Owns the KV cache and the static decode buffers of one model replica."""
 
@@ -97,10 +111,14 @@ class GenerationEngine:
         self.use_cuda_graph = (self.device.type == "cuda") if use_cuda_graph is None else use_cuda_graph
         dev = self.device
         B = max_batch
-        self.ids = torch.zeros((B,), dtype=torch.int32, device=dev)
+        # ids, context lengths (-1: inactive row) and wanted rows of a step lie behind one another, so that a scheduler's decode
+        # step brings them over with one copy
+        self._pitch = pitch = (B + 63) // 64 * 64
+        self._inputs = torch.zeros((3 * pitch,), dtype=torch.int32, device=dev)
+        self.ids, self.context_lens = self._inputs[:B], self._inputs[pitch:pitch + B]
+        self.context_lens.fill_(-1)
         self.positions = torch.zeros((B,), dtype=torch.int32, device=dev)
         self.slots = torch.full((B,), -1, dtype=torch.int32, device=dev)
-        self.context_lens = torch.full((B,), -1, dtype=torch.int32, device=dev)   # -1 = inactive row
         pin = dev.type == "cuda"
         self.ids_host = torch.zeros((B,), dtype=torch.int32, pin_memory=pin)
         self.out_host = torch.zeros((B,), dtype=torch.int32, pin_memory=pin)
@@ -123,29 +141,40 @@ class GenerationEngine:
             self.active[s.slot] = s
         return seqs
 
-    def _packed(self, parts: Sequence[tuple]) -> tuple:
+    def _to_device(self, *arrays: np.ndarray) -> List[torch.Tensor]:
+        """int32 arrays on the device, brought over by one copy from pinned memory (the allocator keeps that until the copy
+        is done); each starts on 256 bytes."""
+        starts, n = [], 0
+        for a in arrays:
+            starts.append(n)
+            n += (a.size + 63) // 64 * 64
+        host = torch.empty((n,), dtype=torch.int32, pin_memory=self.device.type == "cuda")
+        flat = host.numpy()
+        for a, o in zip(arrays, starts):
+            flat[o:o + a.size] = a.reshape(-1)
+        there = host.to(self.device, non_blocking=True)
+        return [there[o:o + a.size].view(a.shape) for a, o in zip(arrays, starts)]
+
+    def _packed(self, parts: Sequence[tuple], ids: Optional[List[np.ndarray]] = None, want: Optional[List[int]] = None) -> tuple:
         """Run tokens [start, end) of each (sequence, start, end) as one packed batch; returns (final-normed hidden
-        states of all tokens, packed row of each part's last token)."""
-        m, cache, dev = self.model, self.cache, self.device
-        ids, pos, slots, q_start, q_lens, ctx, rows = [], [], [], [], [], [], []
-        off = 0
-        for s, c, n in parts:
-            ids.append(torch.tensor(s.tokens[c:n], dtype=torch.int32))
-            pos.append(torch.arange(c, n, dtype=torch.int32))
-            slots.append(cache.slots_for(s, c, n))
-            q_start.append(off)
-            q_lens.append(n - c)
-            ctx.append(n)
-            rows.append(s.slot)
-            off += n - c
-        to = lambda xs, cat=True: (torch.cat(xs) if cat else torch.tensor(xs, dtype=torch.int32)).to(
-            dev, non_blocking=True)
-        ids_d, pos_d, slots_d = to(ids), to(pos), to(slots)
-        qs_d, ql_d, ctx_d, rows_d = to(q_start, False), to(q_lens, False), to(ctx, False), to(rows, False)
-        table = cache.block_table[rows_d.long()]
-        hidden = m.prefill(ids_d, pos_d, slots_d, cache, table, qs_d, ql_d, ctx_d, max(q_lens), rows=rows_d,
+        states of all tokens, packed rows `want`, by default that of each part's last token).  ids: the parts' tokens, where
+        the caller has them as arrays."""
+        m, cache = self.model, self.cache
+        if ids is None:
+            ids = [np.array(s.tokens[c:n], dtype=np.int32) for s, c, n in parts]
+        lens = np.array([n - c for _, c, n in parts], dtype=np.int32)
+        ends = np.cumsum(lens, dtype=np.int32)
+        pos = np.concatenate([np.arange(c, n, dtype=np.int32) for _, c, n in parts])
+        rows = np.array([s.slot for s, _, _ in parts], dtype=np.int32)
+        table = cache.table_rows(rows)
+        page = np.repeat(np.arange(len(parts)), lens), pos // BLOCK_SIZE
+        ids_d, pos_d, slots_d, qs_d, ql_d, ctx_d, rows_d, want_d, table_d = self._to_device(
+            np.concatenate(ids), pos, table[page] * BLOCK_SIZE + pos % BLOCK_SIZE, ends - lens, lens,
+            np.array([n for _, _, n in parts], dtype=np.int32), rows, ends - 1 if want is None else np.array(want, dtype=np.int32),
+            table)
+        hidden = m.prefill(ids_d, pos_d, slots_d, cache, table_d, qs_d, ql_d, ctx_d, int(lens.max()), rows=rows_d,
                            spans=[(c, n) for _, c, n in parts])
-        return hidden, (qs_d + ql_d - 1).long()
+        return hidden, want_d
 
     def _portions(self, seqs: Sequence[SequenceState]):
         """Uncached prompt tokens as packed batches of at most prefill_chunk_tokens, [(index, sequence, start, end)];
@@ -176,7 +205,7 @@ class GenerationEngine:
             if not done:
                 cache.mark_computed(batch[0][1], batch[0][3])
                 continue
-            h = hidden[last].contiguous()
+            h = hidden.index_select(0, last)
             tok_ids = m.greedy(h) if sampling is None else self._sample(m.logits(h), sampling, len(batch[0][1].tokens))
             for j, (gi, _, _, _) in enumerate(batch):
                 first[gi:gi + 1].copy_(tok_ids[j:j + 1])
@@ -314,52 +343,73 @@ class GenerationEngine:
                 raise ValueError("an entry needs at least one token")
             if e.seq.num_computed + len(e.tokens) > self.max_seq_len:
                 raise RuntimeError(f"sequence would exceed max_seq_len={self.max_seq_len}")
-        for e in entries:
-            e.seq.tokens = e.seq.tokens[:e.seq.num_computed] + [int(t) for t in e.tokens]
-            self.cache.ensure_capacity(e.seq, len(e.seq.tokens))
+        news = [_token_array(e.tokens) for e in entries]
+        try:
+            for e, new in zip(entries, news):
+                tokens = e.seq.tokens
+                del tokens[e.seq.num_computed:]
+                tokens.extend(new.tolist())
+                self.cache.ensure_capacity(e.seq, len(tokens), flush=False)
+        finally:
+            self.cache.flush()
         if not entries:
             return None
         decode = self.model.tp.world_size == 1 and all(len(e.tokens) == 1 and e.seq.num_computed > 0 for e in entries)
-        rows: List[int] = []
+        logits = None
         if decode:
-            hidden = None
-            self._decode_rows(entries)
-            rows = [e.seq.slot for e in entries if len(e.want)]
+            logits = self._decode_rows(entries)
         else:
-            hidden, _ = self._packed([(e.seq, e.seq.num_computed, len(e.seq.tokens)) for e in entries])
-            off = 0
+            rows, off, total = [], 0, sum(len(e.tokens) for e in entries)
             for e in entries:
                 rows += [off + int(w) for w in e.want]
                 off += len(e.tokens)
-        logits = None
-        if rows:
-            idx = torch.tensor(rows, dtype=torch.long, device=self.device)
-            logits = self.step_logits[idx] if decode else self.model.logits(hidden[idx].contiguous())
+            if any(not -total <= r < total for r in rows):
+                raise IndexError("a wanted place lies outside the step's tokens")
+            rows = [r % total for r in rows]
+            hidden, want = self._packed([(e.seq, e.seq.num_computed, len(e.seq.tokens)) for e in entries], news, rows)
+            if rows:
+                logits = self.model.logits(hidden.index_select(0, want))
         for e in entries:
             if decode:
                 e.seq.num_computed += 1
             else:
                 self.cache.mark_computed(e.seq, len(e.seq.tokens))
         if self.device.type == "cuda":
-            # the block-table rows are copied from pinned memory that the next step or release may rewrite
+            # the block table and the step's inputs are copied from pinned memory that the next step or release may rewrite
             torch.cuda.current_stream().synchronize()
         return logits
 
-    def _decode_rows(self, entries: Sequence[StepEntry]) -> None:
-        """A decode step of the rows in `entries` only; the other rows are inactive in it."""
-        self.prepare_decode(0, reserve=False)
-        ctx = torch.full((self.max_batch,), -1, dtype=torch.int32)
+    def _decode_rows(self, entries: Sequence[StepEntry]) -> Optional[torch.Tensor]:
+        """A decode step of the rows in `entries` only; the other rows are inactive in it.  Returns the wanted rows' logits."""
+        self._ensure_graph()
+        B, pitch = self.max_batch, self._pitch
+        inputs = torch.empty((3 * pitch,), dtype=torch.int32, pin_memory=self.device.type == "cuda")
+        host = inputs.numpy()
+        ids, ctx, rows = self.ids_host.numpy(), host[pitch:pitch + B], host[2 * pitch:]
+        ctx.fill(-1)
+        wanted = 0
         for e in entries:
-            ctx[e.seq.slot] = e.seq.num_computed
-            self.ids_host[e.seq.slot] = e.seq.tokens[-1]
-        self.context_lens.copy_(ctx)
-        self.ids.copy_(self.ids_host)
+            slot = e.seq.slot
+            ctx[slot] = e.seq.num_computed
+            ids[slot] = e.seq.tokens[-1]
+            for _ in range(min(len(e.want), 1)):
+                rows[wanted] = slot
+                wanted += 1
+        host[:B] = ids
+        host[pitch + B:2 * pitch] = host[B:pitch] = 0
+        rows[wanted:] = 0
+        self._inputs.copy_(inputs, non_blocking=True)
         self.decode_step_device()
-        for s in self.active.values():
-            ctx[s.slot] = s.num_computed
-        for e in entries:
-            ctx[e.seq.slot] = e.seq.num_computed + 1
-        self.context_lens.copy_(ctx)
+        logits = self.step_logits.index_select(0, self._inputs[2 * pitch:2 * pitch + wanted]) if wanted else None
+        if len(entries) < len(self.active):
+            # the rows that were left out become active again; the others have been counted on by the step
+            full = np.full((B,), -1, dtype=np.int32)
+            for s in self.active.values():
+                full[s.slot] = s.num_computed
+            for e in entries:
+                full[e.seq.slot] = e.seq.num_computed + 1
+            self.context_lens.copy_(self._to_device(full)[0])
+        return logits
 
     # ------------------------------------------------------------------ top-level API
     def generate(self, prompts: Sequence[Sequence[int]], max_new_tokens: int, eos_token_id: Optional[int] = None,
@@ -400,9 +450,13 @@ class GenerationEngine:
         return outs
 
     def release(self, seqs: Sequence[SequenceState]) -> None:
-        ctx_host = self.context_lens.cpu()
+        if not len(seqs):
+            return
+        slots = np.array([s.slot for s in seqs], dtype=np.int32)
+        self.context_lens.index_fill_(0, self._to_device(slots)[0].long(), -1)
+        if self.device.type == "cuda":
+            # steps in flight still read the blocks and table rows that are given back here
+            torch.cuda.current_stream().synchronize()
         for s in seqs:
-            ctx_host[s.slot] = -1
             self.active.pop(s.slot, None)
             self.cache.free_sequence(s)
-        self.context_lens.copy_(ctx_host)

@@ -22,6 +22,7 @@ from collections import OrderedDict
 from dataclasses import dataclass, field
 from typing import Dict, List, Optional, Sequence, Tuple, Union
 
+import numpy as np
 import torch
 
 BLOCK_SIZE = 32
@@ -203,6 +204,7 @@ class PagedKVCache:
         self.block_table = torch.zeros((max_batch, max_blocks_per_seq), dtype=torch.int32, device=device)
         pin = self.device.type == "cuda"
         self._table_host = torch.zeros((max_batch, max_blocks_per_seq), dtype=torch.int32, pin_memory=pin)
+        self._dirty = set()                  # rows of the host's table that the device has not got yet
         self.sequences: Dict[int, SequenceState] = {}
         self._free_slots = list(range(max_batch - 1, -1, -1))
         self._next_id = 0
@@ -228,14 +230,34 @@ class PagedKVCache:
         self._write_row(seq)
         return seq
 
-    def ensure_capacity(self, seq: SequenceState, new_len: int) -> bool:
-        """Make sure the sequence has blocks for new_len tokens; True when the table changed."""
+    def ensure_capacity(self, seq: SequenceState, new_len: int, flush: bool = True) -> bool:
+        """Make sure the sequence has blocks for new_len tokens; True when the table changed.  flush False: the device's table
+        follows with `flush`, one copy for all sequences of a step."""
         if (new_len + BLOCK_SIZE - 1) // BLOCK_SIZE > self.max_blocks_per_seq:
             raise OutOfBlocks("sequence longer than max_blocks_per_seq")
-        added = self.allocator.extend(seq.blocks, new_len)
-        if added:
-            self._write_row(seq)
+        had = len(seq.blocks)
+        try:
+            self.allocator.extend(seq.blocks, new_len)
+        finally:
+            added = len(seq.blocks) - had
+            if added:
+                self._table_host.numpy()[seq.slot, had:had + added] = seq.blocks[had:]
+                self._dirty.add(seq.slot)
+        if added and flush:
+            self.flush()
         return added > 0
+
+    def flush(self) -> None:
+        """Bring the rows that have grown to the device's table."""
+        if not self._dirty:
+            return
+        lo, hi = min(self._dirty), max(self._dirty) + 1
+        self._dirty.clear()
+        self.block_table[lo:hi].copy_(self._table_host[lo:hi], non_blocking=True)
+
+    def table_rows(self, rows: np.ndarray) -> np.ndarray:
+        """Block table of the given batch rows, from the host's copy."""
+        return self._table_host.numpy()[rows]
 
     def mark_computed(self, seq: SequenceState, upto: int) -> None:
         seq.num_computed = upto
