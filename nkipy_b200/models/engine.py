@@ -359,14 +359,22 @@ class GenerationEngine:
         if decode:
             logits = self._decode_rows(entries)
         else:
-            rows, off, total = [], 0, sum(len(e.tokens) for e in entries)
+            # places count through the entries as they were given; single tokens lie ahead of portions in the batch, where
+            # attention takes them together
+            order = sorted(range(len(entries)), key=lambda i: len(entries[i].tokens) > 1)
+            starts, total = np.zeros((len(entries),), dtype=np.int64), 0
+            for i in order:
+                starts[i] = total
+                total += len(entries[i].tokens)
+            place = np.concatenate([starts[i] + np.arange(len(e.tokens)) for i, e in enumerate(entries)])
+            rows, off = [], 0
             for e in entries:
                 rows += [off + int(w) for w in e.want]
                 off += len(e.tokens)
             if any(not -total <= r < total for r in rows):
                 raise IndexError("a wanted place lies outside the step's tokens")
-            rows = [r % total for r in rows]
-            hidden, want = self._packed([(e.seq, e.seq.num_computed, len(e.seq.tokens)) for e in entries], news, rows)
+            parts = [(e.seq, e.seq.num_computed, len(e.seq.tokens)) for e in entries]
+            hidden, want = self._packed([parts[i] for i in order], [news[i] for i in order], place[rows] if rows else [])
             if rows:
                 logits = self.model.logits(hidden.index_select(0, want))
         for e in entries:

@@ -422,13 +422,14 @@ class Batch:
     """The tokens of a step, where they sit (cache slots, block tables) and how they are grouped into sequences (q_lens
     None: one per batch row)."""
     __slots__ = ("positions", "slots", "block_table", "context_lens", "q_start", "q_lens", "max_q_len", "rows", "ids",
-                 "_spans", "_pages")
+                 "singles", "_spans", "_pages")
 
     def __init__(self, positions, slots, block_table, context_lens, q_start=None, q_lens=None, max_q_len=1, rows=None,
                  ids=None, spans=None):
         self.positions, self.slots, self.block_table, self.context_lens = positions, slots, block_table, context_lens
         self.q_start, self.q_lens, self.max_q_len, self.rows = q_start, q_lens, max_q_len, rows
         self.ids, self._spans, self._pages = ids, spans, {}
+        self.singles = ops.leading_singles(spans)
 
     def visible_pages(self, window: int):
         """Cache pages that the new tokens see through a sliding window (0: all before them), sequence by sequence (int32 block

@@ -139,7 +139,7 @@ class WindowAttentionMixer:
         kc, vc = cache.k[entry], cache.v[entry]
         q = ops.row_norm_append(self.maps, q, k, v, self.q_norm, self.k_norm, b.slots, kc, vc)
         o = ops.heads_attention(self.maps, q, kc, vc, b.block_table, b.context_lens, q_start=b.q_start, q_lens=b.q_lens,
-                                max_q_len=b.max_q_len)
+                                singles=b.singles, max_q_len=b.max_q_len)
         return ops.gate_heads(o, g, "sigmoid", scale=self.scale, out=out)
 
 
@@ -166,7 +166,7 @@ class ChunkAttentionMixer:
         q = ops.rope_norm_append(self.maps, q, *(kv or (None, None)), self.bias, model.rope_table(self.spec.rope), b.positions,
                                  b.slots, kc, vc)
         o = ops.heads_attention(self.maps, q, kc, vc, b.block_table, b.context_lens, q_start=b.q_start, q_lens=b.q_lens,
-                                max_q_len=b.max_q_len)
+                                singles=b.singles, max_q_len=b.max_q_len)
         return ops.gate_heads(o, g, "sigmoid")
 
 
@@ -291,7 +291,7 @@ class GroupedAttentionMixer:
         q = ops.rope_norm_append(self.maps, q, *(kv or (None, None)), self.bias, model.rope_table(rope) if rope else None,
                                  b.positions, b.slots, kc, vc, norm=False, interleaved=True)
         o = ops.heads_attention(self.maps, q, kc, vc, b.block_table, b.context_lens, q_start=b.q_start, q_lens=b.q_lens,
-                                max_q_len=b.max_q_len, sinks=self.sink)
+                                singles=b.singles, max_q_len=b.max_q_len, sinks=self.sink)
         return o.flatten(1) if g is None else ops.gate_heads(o, g, "sigmoid")
 
 

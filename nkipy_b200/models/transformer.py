@@ -413,7 +413,8 @@ class TransformerLM:
         """Packed prefill of several sequences.  ids / positions / slots [T]; returns the
         final-normed hidden states [T, H] (and the per-layer residual streams when
         return_hidden is set, for speculative-decoding taps).  inputs: see `decode_step`.
-        rows (the sequences' batch rows) and spans (their new positions on the host) are for layer-by-layer models; unused here."""
+        spans: the sequences' new positions on the host; single tokens ahead of the others run decode attention.  rows (batch
+        rows) are for layer-by-layer models; unused here."""
         cfg = self.cfg
         tp1 = self.tp.world_size == 1
         if (not tp1 and not return_hidden and inputs is None and getattr(self.tp, "fused", None) is not None
@@ -428,15 +429,16 @@ class TransformerLM:
         else:
             resid, normed = inputs
         taps = [] if return_hidden else None
+        singles = ops.leading_singles(spans)
         for i, lw in enumerate(self.layers):
             swap, splits = ops.prefill_plan(normed.shape[0], lw.qkv.shape[0], lw.qkv.shape[1])
             qkv = ops.linear(normed, lw.qkv, swap=swap and splits > 1, splits=splits)
             q = ops.rope_kv_append(qkv, positions, slots, self.rope, cache.k[i], cache.v[i], self.nq, self.nkv,
                                    self.d, bias=lw.qkv_bias, q_norm_w=lw.q_norm, k_norm_w=lw.k_norm,
                                    norm_eps=cfg.rms_eps)
-            attn = ops.flash_attn_prefill(q, cache.k[i], cache.v[i], block_table, q_start, q_lens, context_lens,
-                                          self.scale, max_q_len=max_q_len, causal=cfg.causal,
-                                          window=cfg.window_for_layer(i), sinks=lw.sinks)
+            attn = ops.packed_attention(q, cache.k[i], cache.v[i], block_table, q_start, q_lens, context_lens, self.scale,
+                                        max_q_len=max_q_len, singles=singles, causal=cfg.causal,
+                                        window=cfg.window_for_layer(i), sinks=lw.sinks)
             if tp1:
                 resid, normed = self._residual_linear(attn, lw.o, resid, lw.post_norm, lw.o_bias)
             else:

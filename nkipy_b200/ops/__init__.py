@@ -30,7 +30,7 @@ from ._lib import KernelLibraryError, device_status, raise_on_device_error
 
 __all__ = [
     "linear", "decode_linear", "qkv_rope_append", "reduce_partials", "rmsnorm", "add_rmsnorm", "silu_mul", "embedding", "rope_kv_append",
-    "argmax", "sample", "decode_advance", "router_topk", "moe_dispatch", "grouped_linear", "moe_combine", "paged_attn_decode", "flash_attn_prefill", "rope_table",
+    "argmax", "sample", "decode_advance", "router_topk", "moe_dispatch", "grouped_linear", "moe_combine", "paged_attn_decode", "flash_attn_prefill", "packed_attention", "leading_singles", "rope_table",
     "Branch", "MapsSpec", "Norm", "Proj", "activation", "gate_heads", "gated_act", "gated_residual", "hgrn2", "maps_append",
     "heads_attention", "maps_attention", "row_norm_append", "rope_norm_append", "head_linear", "softcap",
     "LatentSpec", "latent_append", "latent_attention", "latent_gather", "latent_prefill", "latent_queries",
@@ -1093,6 +1093,33 @@ def flash_attn_prefill(
     _lib.check(rc, "nkb_flash_attn_prefill")
     _launches += 1
     return out
+
+
+def packed_attention(q, k_cache, v_cache, block_table, q_start, q_lens, context_lens, scale, *, max_q_len: int, singles: int = 0,
+                     causal: bool = True, **kw) -> torch.Tensor:
+    """`flash_attn_prefill` of a packed step whose first `singles` sequences have one new token each, in the first rows: those
+    run the decode kernel, which reads a kv head's pages once for its whole group and has no 128-row tile to fill.  24 sequences
+    of 300 to 600 tokens beside a prompt of 390: 74 us in the blockwise kernel alone."""
+    B, nkv, D = block_table.shape[0], k_cache.shape[1], k_cache.shape[3]
+    if singles <= 0 or not causal or not _native(q) or q.shape[-1] // D // nkv > 16:
+        return flash_attn_prefill(q, k_cache, v_cache, block_table, q_start, q_lens, context_lens, scale, max_q_len=max_q_len,
+                                  causal=causal, **kw)
+    out = torch.empty_like(q)
+    paged_attn_decode(q[:singles], k_cache, v_cache, block_table[:singles], context_lens[:singles], scale, out=out[:singles], **kw)
+    if singles < B:
+        flash_attn_prefill(q, k_cache, v_cache, block_table[singles:], q_start[singles:], q_lens[singles:], context_lens[singles:],
+                           scale, max_q_len=max_q_len, out=out, **kw)
+    return out
+
+
+def leading_singles(spans) -> int:
+    """How many of the first (start, end) spans of a packed step are single tokens."""
+    n = 0
+    for start, end in spans or ():
+        if end - start != 1:
+            break
+        n += 1
+    return n
 
 
 # --------------------------------------------------------------------------- mixture of experts

@@ -31,7 +31,7 @@ import torch
 import torch.nn.functional as F
 
 from . import _lib
-from . import (ScoreMods, _count_launch, _decode_scratch, _gather_kv, _native, _ptr, _stream, flash_attn_prefill,
+from . import (ScoreMods, _count_launch, _decode_scratch, _gather_kv, _native, _ptr, _stream, packed_attention,
                paged_attn_decode, pick_kv_splits)
 
 # name -> (kernel code, PyTorch function)
@@ -643,11 +643,12 @@ def maps_attention(*args, **kw) -> torch.Tensor:
 def heads_attention(spec: MapsSpec, q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
                    block_table: torch.Tensor, context_lens: torch.Tensor, *, q_start: Optional[torch.Tensor] = None,
                    q_lens: Optional[torch.Tensor] = None, max_q_len: int = 1, num_splits: int = 0,
-                   sinks: Optional[torch.Tensor] = None) -> torch.Tensor:
+                   sinks: Optional[torch.Tensor] = None, singles: int = 0) -> torch.Tensor:
     """Causal attention of the new tokens over the paged cache (which already holds them); returns the combined heads
     [T, heads, vdim] (strided when the cache's values are padded).  sinks [heads] fp32: logarithms of an addend of every
     softmax's denominator.  q_lens None: one new token per sequence (decode); otherwise sequence b owns rows
-    q_start[b] .. q_start[b] + q_lens[b], the last of which sits at position context_lens[b] - 1."""
+    q_start[b] .. q_start[b] + q_lens[b], the last of which sits at position context_lens[b] - 1; singles: see
+    `packed_attention`."""
     T, H = q.shape[0], spec.heads
     bs = k_cache.shape[2]
     B = block_table.shape[0]
@@ -659,8 +660,8 @@ def heads_attention(spec: MapsSpec, q: torch.Tensor, k_cache: torch.Tensor, v_ca
             o = paged_attn_decode(qf, k_cache, v_cache, block_table, context_lens, spec.scale, window=spec.window,
                                   chunk=spec.chunk, sinks=sinks, mods=spec.mods, num_splits=num_splits)
         else:
-            o = flash_attn_prefill(qf, k_cache, v_cache, block_table, q_start, q_lens, context_lens, spec.scale,
-                                   max_q_len=max_q_len, window=spec.window, chunk=spec.chunk, sinks=sinks, mods=spec.mods)
+            o = packed_attention(qf, k_cache, v_cache, block_table, q_start, q_lens, context_lens, spec.scale, singles=singles,
+                                 max_q_len=max_q_len, window=spec.window, chunk=spec.chunk, sinks=sinks, mods=spec.mods)
         return o.view(T, H, spec.vdim_p)[..., :spec.vdim]
     out = torch.empty((T, H, spec.vdim), dtype=k_cache.dtype, device=k_cache.device)
     if not _native(k_cache):

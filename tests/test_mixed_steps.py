@@ -1,0 +1,81 @@
+"""Steps of an external scheduler: single tokens and portions in any order give what they give alone."""
+import pytest
+import torch
+
+from nkipy_b200.models import config as C
+from nkipy_b200.models.engine import GenerationEngine, StepEntry
+from nkipy_b200.models.kv_cache import BLOCK_SIZE, OutOfBlocks
+from nkipy_b200.models.transformer import TransformerLM
+from nkipy_b200.models.weights import random_weights
+
+DEVICES = ["cpu", pytest.param("cuda", marks=pytest.mark.gpu)]
+
+
+def engine(device, **kw):
+    cfg = C.tiny(hidden_size=256, head_dim=64, num_heads=8, num_kv_heads=2, intermediate_size=512, vocab_size=512, num_layers=2)
+    model = TransformerLM(cfg, random_weights(cfg, device=device, seed=1, std=0.05), device=device)
+    return GenerationEngine(model, max_batch=6, max_seq_len=256, enable_prefix_sharing=False, **kw)
+
+
+def ids(n, seed):
+    return torch.randint(0, 512, (n,), generator=torch.Generator().manual_seed(seed)).tolist()
+
+
+@pytest.mark.parametrize("device", DEVICES)
+def test_any_order_of_singles_and_portions(device):
+    prompts, news = [ids(n, n) for n in (70, 1, 33, 64, 5)], [ids(1, 90), ids(40, 91), ids(1, 92), ids(2, 93), ids(1, 94)]
+    want = [[0], [39, 0], [0], [-1], [0]]
+    alone = []
+    for p, n, w in zip(prompts, news, want):
+        e = engine(device)
+        s = e.open_request()
+        e.run_step([StepEntry(s, p)])
+        # -1 counts from the end of the step's tokens
+        alone.append(e.run_step([StepEntry(s, n + [7], [x % len(n) for x in w])]).float().cpu())
+    e = engine(device)
+    seqs = [e.open_request() for _ in prompts]
+    for s, p in zip(seqs, prompts):
+        e.run_step([StepEntry(s, p)])
+    entries = [StepEntry(s, n, [x for x in w]) for s, n, w in zip(seqs, news, want)]
+    entries[3].want = [1]
+    got = e.run_step(entries).float().cpu()
+    ref = torch.cat(alone)
+    assert got.shape == ref.shape
+    # bf16 activations in batches of other sizes
+    assert (got - ref).norm() <= (2e-2 if device == "cuda" else 1e-2) * ref.norm()
+    assert ((got - ref).norm(dim=1) <= 4e-2 * ref.norm(dim=1)).all()
+
+
+@pytest.mark.parametrize("device", DEVICES)
+def test_places_outside_a_step_are_refused(device):
+    e = engine(device)
+    s = e.open_request()
+    with pytest.raises(IndexError):
+        e.run_step([StepEntry(s, ids(4, 1), [4])])
+    with pytest.raises(IndexError):
+        e.run_step([StepEntry(s, ids(4, 1), [-5])])
+    with pytest.raises(ValueError):
+        e.run_step([StepEntry(s, [2 ** 40], [0])])
+    assert s.num_computed == 0 and e.run_step([StepEntry(s, ids(4, 1), [-1])]).shape[0] == 1
+
+
+@pytest.mark.parametrize("device", DEVICES)
+def test_tables_and_lengths_follow_growth_and_release(device):
+    """The device's block table and context lengths after steps that cross blocks, leave sequences out and give rows back."""
+    e = engine(device)
+    seqs = [e.open_request() for _ in range(4)]
+    e.run_step([StepEntry(s, ids(BLOCK_SIZE - 2 + i, i)) for i, s in enumerate(seqs)])
+    for step in range(5):
+        out = [s for i, s in enumerate(seqs) if (i + step) % 3]
+        before = {s.seq_id: s.num_computed for s in seqs}
+        assert e.run_step([StepEntry(s, ids(1, step), [0]) for s in out]).shape[0] == len(out)
+        for s in seqs:
+            assert s.num_computed == before[s.seq_id] + (s in out) == len(s.tokens)
+            assert int(e.context_lens[s.slot]) == s.num_computed
+            assert e.cache.block_table[s.slot, :len(s.blocks)].tolist() == s.blocks
+    e.release([seqs[0], seqs[2], seqs[3]])
+    assert [int(e.context_lens[s.slot]) for s in seqs] == [-1, seqs[1].num_computed, -1, -1]
+    free = e.cache.allocator.num_free()
+    with pytest.raises((OutOfBlocks, RuntimeError)):
+        e.run_step([StepEntry(seqs[1], ids(300, 1))])
+    assert e.cache.allocator.num_free() == free
