@@ -80,17 +80,28 @@ class Sampling:
     seed: int = 0
 
 
-def _token_array(tokens: Sequence[int]) -> np.ndarray:
-    """Token ids as int32."""
-    try:
-        a = np.asarray(tokens)
-    except (TypeError, ValueError, RuntimeError):
-        a = None
-    if a is None or a.dtype.kind not in "iu" or a.ndim != 1:
-        a = np.array([int(t) for t in tokens], dtype=np.int64)
-    if a.size and not -2 ** 31 <= int(a.min()) <= int(a.max()) < 2 ** 31:
+def _token_arrays(entries: Sequence[StepEntry]) -> List[np.ndarray]:
+    """Token ids of every entry as int32."""
+    def one(tokens) -> np.ndarray:
+        try:
+            a = np.asarray(tokens)
+        except (TypeError, ValueError, RuntimeError):
+            a = None
+        if a is None or a.dtype.kind not in "iu" or a.ndim != 1:
+            a = np.array([int(t) for t in tokens], dtype=np.int64)
+        return a
+
+    if all(len(e.tokens) == 1 for e in entries):
+        flat = one([e.tokens[0] for e in entries])
+    else:
+        flat = np.concatenate([one(e.tokens) for e in entries])
+    if flat.size and not -2 ** 31 <= int(flat.min()) <= int(flat.max()) < 2 ** 31:
         raise ValueError("token ids are 32-bit numbers")
-    return a.astype(np.int32)
+    flat, out, n = flat.astype(np.int32), [], 0
+    for e in entries:
+        out.append(flat[n:n + len(e.tokens)])
+        n += len(e.tokens)
+    return out
 
 
 class GenerationEngine:
@@ -343,17 +354,18 @@ class GenerationEngine:
                 raise ValueError("an entry needs at least one token")
             if e.seq.num_computed + len(e.tokens) > self.max_seq_len:
                 raise RuntimeError(f"sequence would exceed max_seq_len={self.max_seq_len}")
-        news = [_token_array(e.tokens) for e in entries]
+        if not entries:
+            return None
+        news = _token_arrays(entries)
         try:
             for e, new in zip(entries, news):
                 tokens = e.seq.tokens
                 del tokens[e.seq.num_computed:]
                 tokens.extend(new.tolist())
-                self.cache.ensure_capacity(e.seq, len(tokens), flush=False)
+                if len(tokens) > len(e.seq.blocks) * BLOCK_SIZE:
+                    self.cache.ensure_capacity(e.seq, len(tokens), flush=False)
         finally:
             self.cache.flush()
-        if not entries:
-            return None
         decode = self.model.tp.world_size == 1 and all(len(e.tokens) == 1 and e.seq.num_computed > 0 for e in entries)
         logits = None
         if decode:
@@ -393,19 +405,15 @@ class GenerationEngine:
         B, pitch = self.max_batch, self._pitch
         inputs = torch.empty((3 * pitch,), dtype=torch.int32, pin_memory=self.device.type == "cuda")
         host = inputs.numpy()
-        ids, ctx, rows = self.ids_host.numpy(), host[pitch:pitch + B], host[2 * pitch:]
+        ids, ctx = self.ids_host.numpy(), host[pitch:pitch + B]
+        slots = np.array([e.seq.slot for e in entries])
         ctx.fill(-1)
-        wanted = 0
-        for e in entries:
-            slot = e.seq.slot
-            ctx[slot] = e.seq.num_computed
-            ids[slot] = e.seq.tokens[-1]
-            for _ in range(min(len(e.want), 1)):
-                rows[wanted] = slot
-                wanted += 1
+        ctx[slots] = [e.seq.num_computed for e in entries]
+        ids[slots] = [e.seq.tokens[-1] for e in entries]
+        rows = [e.seq.slot for e in entries if len(e.want)]
+        wanted = len(rows)
         host[:B] = ids
-        host[pitch + B:2 * pitch] = host[B:pitch] = 0
-        rows[wanted:] = 0
+        host[2 * pitch:2 * pitch + wanted] = rows
         self._inputs.copy_(inputs, non_blocking=True)
         self.decode_step_device()
         logits = self.step_logits.index_select(0, self._inputs[2 * pitch:2 * pitch + wanted]) if wanted else None
@@ -460,8 +468,13 @@ class GenerationEngine:
     def release(self, seqs: Sequence[SequenceState]) -> None:
         if not len(seqs):
             return
-        slots = np.array([s.slot for s in seqs], dtype=np.int32)
-        self.context_lens.index_fill_(0, self._to_device(slots)[0].long(), -1)
+        # runs of neighbouring rows
+        slots = sorted(s.slot for s in seqs)
+        first = 0
+        for i in range(1, len(slots) + 1):
+            if i == len(slots) or slots[i] != slots[i - 1] + 1:
+                self.context_lens[slots[first]:slots[i - 1] + 1].fill_(-1)
+                first = i
         if self.device.type == "cuda":
             # steps in flight still read the blocks and table rows that are given back here
             torch.cuda.current_stream().synchronize()

@@ -227,7 +227,8 @@ class PagedKVCache:
         seq = SequenceState(self._next_id, list(tokens), blocks, cached, cached, self._free_slots.pop())
         self._next_id += 1
         self.sequences[seq.seq_id] = seq
-        self._write_row(seq)
+        if blocks:
+            self._write_row(seq)
         return seq
 
     def ensure_capacity(self, seq: SequenceState, new_len: int, flush: bool = True) -> bool:

@@ -16,10 +16,10 @@ is transposed once at load time.
 
 from __future__ import annotations
 
-import os
-
 import ctypes
+import functools
 import math
+import os
 from dataclasses import dataclass
 from typing import Optional, Tuple, Union
 
@@ -67,7 +67,8 @@ def _ptr(t: Optional[torch.Tensor]):
 
 
 def _stream():
-    return torch.cuda.current_stream().cuda_stream
+    # the current device's current stream, without the stream object (a launch of a packed step has a few microseconds in all)
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _native(t: torch.Tensor) -> bool:
@@ -79,7 +80,7 @@ def _native(t: torch.Tensor) -> bool:
 
 def _check_bf16(*tensors):
     for t in tensors:
-        if t is not None and t.dtype != torch.bfloat16:
+        if t is not None and t.dtype is not torch.bfloat16:
             raise TypeError(f"expected bfloat16 tensor, got {t.dtype}")
 
 
@@ -114,8 +115,11 @@ def prefill_plan(rows: int, cols: int, k: int) -> Tuple[bool, int]:
         from ..models.transformer import pick_splits
 
         return True, pick_splits(cols, k)
-    if cols < 256 or not _USE_2CTA or k % 8:
-        return False, 1
+    return False, _pair_splits(rows, cols, k) if cols >= 256 and _USE_2CTA and k % 8 == 0 else 1
+
+
+@functools.lru_cache(maxsize=1024)
+def _pair_splits(rows: int, cols: int, k: int) -> int:
     slabs, tiles = -(-k // 64), _pair_tiles(rows, cols, False)
     best, best_cost = 1, -(-tiles // 74) * slabs * 0.4 - 3.0
     for s in range(2, 9):
@@ -125,7 +129,7 @@ def prefill_plan(rows: int, cols: int, k: int) -> Tuple[bool, int]:
         cost = -(-tiles * s // 74) * per * 0.4 + s * rows * cols * 8 / 4e6
         if cost < best_cost:
             best, best_cost = s, cost
-    return False, best
+    return best
 
 
 def _pick_block_n(cols: int, gated: bool) -> int:
@@ -134,6 +138,12 @@ def _pick_block_n(cols: int, gated: bool) -> int:
         if cols <= bn and bn <= cap:
             return bn
     return cap
+
+
+def effective_splits(k: int, splits: int) -> int:
+    """Partials that a product split `splits` ways really has: whole slabs of 64 k, none of them empty (the launchers' rule)."""
+    slabs = -(-k // 64)
+    return -(-slabs // -(-slabs // max(1, min(splits, slabs))))
 
 
 def linear(
@@ -197,12 +207,14 @@ def linear(
             return out
         return y
     global _launches
-    if x.stride(1) != 1 or w.stride(1) != 1:
+    (ldx, sx), (ldw, sw) = x.stride(), w.stride()
+    if sx != 1 or sw != 1:
         raise ValueError("linear needs K-contiguous operands")
-    epi = mixers.Act.of(out_act) if out_act is not None else mixers.Act("silu")
+    epi = _PLAIN if out_act is None else mixers.Act.of(out_act)
     if out_act is not None and (epi.name not in ("relu2", "xielu") or gated or residual is not None or fp32_out):
         raise ValueError("out_act is relu2 or xielu, for finished plain products")
-    if x.dtype == torch.float32 or (K | x.stride(0) | w.stride(0)) & 7 or (x.data_ptr() | w.data_ptr()) & 15:
+    xp, wp = x.data_ptr(), w.data_ptr()
+    if x.dtype == torch.float32 or (K | ldx | ldw) & 7 or (xp | wp) & 15:
         if bias is not None or residual is not None or out is not None:
             raise ValueError("the CUDA-core GEMM has no bias, residual or out argument")
         y = mixers.linear_simt(x, w, gated=gated, act=act, fp32_out=fp32_out or splits > 1 or out_act is not None)
@@ -216,25 +228,26 @@ def linear(
         raise ValueError("out_act wants finished values in the prefill orientation (swap=False)")
     L = _lib.lib()
     if splits > 1:
-        eff = L.nkb_gemm_effective_splits(K, splits)
+        eff = effective_splits(K, splits)
         if out is None:
-            out = torch.empty((eff, M, N), dtype=torch.float32, device=x.device)
-        elif out.dtype != torch.float32 or out.numel() < eff * M * N:
-            raise ValueError("split-K output must be fp32 with room for [S, M, N]")
-        out_view = out.view(-1)[: eff * M * N].view(eff, M, N)
-        out_fp32, split_stride = 1, M * N
+            out_view = torch.empty((eff, M, N), dtype=torch.float32, device=x.device)
+        else:
+            if out.dtype != torch.float32 or out.numel() < eff * M * N:
+                raise ValueError("split-K output must be fp32 with room for [S, M, N]")
+            out_view = out.view(-1)[: eff * M * N].view(eff, M, N)
+        out_fp32, split_stride, ldo = 1, M * N, N
     else:
         eff = 1
         if out is None:
             out = torch.empty((M, N), dtype=torch.float32 if fp32_out else torch.bfloat16, device=x.device)
         out_view = out
         out_fp32, split_stride = 1 if fp32_out else 0, 0
-    ldo = out_view.stride(-2) if out_view.dim() >= 2 else N
+        ldo = out.stride(-2) if out.dim() >= 2 else N
     act_code = mixers.ACTIVATIONS[act][0] if gated else (epi.code if out_act is not None else 0)
     if (not swap and not fp32_out and (ldo & 7) == 0 and not (gated and (bias is not None or residual is not None))
             and (_use_pairs(M, N, gated) if splits <= 1 else M > 128 and N >= 256 and _USE_2CTA and bias is None and residual is None)):
         # prefill-sized: CTA pairs on 256 x 256 tiles (csrc/kernels/gemm_2cta.cu)
-        rc = L.nkb_gemm_bf16_2cta(x.data_ptr(), w.data_ptr(), out_view.data_ptr(), M, N, K, x.stride(0), w.stride(0),
+        rc = L.nkb_gemm_bf16_2cta(xp, wp, out_view.data_ptr(), M, N, K, ldx, ldw,
                                   ldo, _ptr(bias), _ptr(residual), 1 if gated else 0, N if gated else 0, act_code, epi.a, epi.b,
                                   eff, split_stride, 1 if weights_static else 0, _stream())
         if rc != -5:
@@ -242,20 +255,14 @@ def linear(
             _launches += 1
             return out_view
     if swap:
-        a, b, rows, cols = w, x, N, M
-        lda, ldb = w.stride(0), x.stride(0)
-        gate_mode = 1 if gated else 0
-        block_n = _pick_block_n(cols, gated)
-        transpose_out, bias_on_rows = 1, 1
+        block_n, gate_mode, on_rows = _pick_block_n(M, gated), 1 if gated else 0, 1
+        ap, bp, rows, cols, lda, ldb = wp, xp, N, M, ldw, ldx
     else:
-        a, b, rows, cols = x, w, M, N
-        lda, ldb = x.stride(0), w.stride(0)
-        gate_mode = 2 if gated else 0
-        block_n = 128 if gated else (256 if N >= 256 else _pick_block_n(N, False))
-        transpose_out, bias_on_rows = 0, 0
+        block_n, gate_mode, on_rows = 128 if gated else (256 if N >= 256 else _pick_block_n(N, False)), 2 if gated else 0, 0
+        ap, bp, rows, cols, lda, ldb = xp, wp, M, N, ldx, ldw
     rc = L.nkb_gemm_bf16(
-        a.data_ptr(), b.data_ptr(), out_view.data_ptr(), rows, cols, K, lda, ldb, ldo, transpose_out, out_fp32,
-        eff if splits > 1 else 1, split_stride, gate_mode, N if gated else 0, _ptr(bias), bias_on_rows,
+        ap, bp, out_view.data_ptr(), rows, cols, K, lda, ldb, ldo, on_rows, out_fp32,
+        eff, split_stride, gate_mode, N if gated else 0, _ptr(bias), on_rows,
         _ptr(residual), block_n, max_ctas, (0 if swap else 1) if weights_static else -1,
         (2 if (swap and not gated) else 1) if ctas_per_sm is None else ctas_per_sm, act_code, epi.a, epi.b, _stream(),
     )
@@ -1360,3 +1367,5 @@ from .latent_attention import (LatentSpec, latent_append, latent_attention, late
 from .linear_attention import Decay, linear_attention, low_rank, token_mix  # noqa: E402,F401
 from .head_recurrence import (HeadRecurrence, ShortConv, gated_group_norm, head_recurrence,  # noqa: E402,F401
                               short_conv)
+
+_PLAIN = Act("silu")
