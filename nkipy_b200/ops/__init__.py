@@ -245,7 +245,8 @@ def linear(
         ldo = out.stride(-2) if out.dim() >= 2 else N
     act_code = mixers.ACTIVATIONS[act][0] if gated else (epi.code if out_act is not None else 0)
     if (not swap and not fp32_out and (ldo & 7) == 0 and not (gated and (bias is not None or residual is not None))
-            and (_use_pairs(M, N, gated) if splits <= 1 else M > 128 and N >= 256 and _USE_2CTA and bias is None and residual is None)):
+            and (_use_pairs(M, N, gated) if splits <= 1 else
+                 eff > 1 and M > 128 and N >= 256 and _USE_2CTA and bias is None and residual is None)):
         # prefill-sized: CTA pairs on 256 x 256 tiles (csrc/kernels/gemm_2cta.cu)
         rc = L.nkb_gemm_bf16_2cta(xp, wp, out_view.data_ptr(), M, N, K, ldx, ldw,
                                   ldo, _ptr(bias), _ptr(residual), 1 if gated else 0, N if gated else 0, act_code, epi.a, epi.b,

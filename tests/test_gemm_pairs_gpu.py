@@ -84,3 +84,13 @@ def test_grouped_products_on_pairs(tokens, experts, top, width, inner, limit):
         want = h[rows].double() @ w2[e].double().T + b2[e].double()
         assert ((y[rows].double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-3).all()
     ops.raise_on_device_error()
+
+
+@pytest.mark.gpu
+def test_one_partial_of_a_requested_split():
+    """Splits of a contraction of one slab are one partial, in fp32."""
+    x, w = torch.randn((130, 64), device="cuda").to(torch.bfloat16), torch.randn((256, 64), device="cuda").to(torch.bfloat16)
+    y = ops.linear(x, w, swap=False, splits=4)
+    assert y.shape == (1, 130, 256) and y.dtype == torch.float32
+    assert ((y[0] - x.double() @ w.double().T).abs() <= 64 * 2.0 ** -23 * (x.double().abs() @ w.double().abs().T)).all()
+    ops.raise_on_device_error()
