@@ -189,6 +189,8 @@ int nkb_gated_act(const NkbProj* gate, const NkbProj* up, void* out, int out_bf1
 // CUDA-core GEMM for 32-bit models and untileable sizes (gemm_simt.cu)
 int nkb_gemm_simt(const void* x, int x_bf16, const void* w, int w_bf16, void* out, int out_bf16, int m, int n, int k,
                   long long ldx, long long ldw, long long ldo, void* stream);
+int nkb_gemm_f32_split(const float* x, const float* w, float* out, void* planes, float* parts, int m, int n, int k, long long ldx,
+                       long long ldw, int block_n, int splits, void* stream);
 int nkb_gemm_simt_grouped(const void* x, int x_bf16, const void* w, int w_bf16, void* out, int out_bf16,
                           const int* offsets, const int* row_token, int groups, int max_rows, int n, int k,
                           long long ldx, long long ldo, void* stream);

@@ -108,6 +108,7 @@ _SIGNATURES = {
                                            c_longlong, c_float, c_float, _P, _P, c_int, _P]),
     "nkb_gemm_simt": (c_int, [_P, c_int, _P, c_int, _P, c_int, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong,
                               _P]),
+    "nkb_gemm_f32_split": (c_int, [_P, _P, _P, _P, _P, c_int, c_int, c_int, c_longlong, c_longlong, c_int, c_int, _P]),
     "nkb_gemm_simt_grouped": (c_int, [_P, c_int, _P, c_int, _P, c_int, _P, _P, c_int, c_int, c_int, c_int, c_longlong,
                                       c_longlong, _P]),
     "nkb_linattn_scan": (c_int, [ctypes.POINTER(LinAttnArg), _P]),

@@ -24,6 +24,7 @@ statement of the same op.
 from __future__ import annotations
 
 import ctypes
+import functools
 from dataclasses import dataclass
 from typing import List, NamedTuple, Optional, Sequence, Tuple, Union
 
@@ -179,19 +180,55 @@ def _ptr_array(ts: Sequence[Optional[torch.Tensor]]):
     return (ctypes.c_void_p * max(len(ts), 1))(*[_ptr(t) for t in ts])
 
 
+@functools.lru_cache(maxsize=1024)
+def f32_split_plan(rows: int, cols: int, k: int) -> Tuple[int, int]:
+    """(rows of x per tile, splits of k) of a 32-bit product on the tensor cores (gemm_f32_split.cu).  An SM runs one tile at a time; a
+    slab of 64 k takes 1 us with few rows of x and 1.5 with 160, a tile some three slabs' time around its own, and planes of partial
+    sums go through the cache once more."""
+    tiles = -(-rows // 160)
+    block = next(b for b in (32, 64, 96, 128, 160) if b >= -(-rows // tiles))
+    slabs, slab_us = -(-k // 64), 0.9 + 0.004 * block
+    best, best_cost = 1, None
+    for s in range(1, 17):
+        per = -(-slabs // s)
+        if s > 1 and (per < 4 or -(-slabs // per) != s):
+            continue
+        cost = -(-(-(-cols // 128)) * tiles * s // 148) * (per + 3) * slab_us + (3.0 + (s + 1) * rows * cols * 4 / 5e6 if s > 1 else 0.0)
+        if best_cost is None or cost < best_cost:
+            best, best_cost = s, cost
+    return block, best
+
+
 def linear_simt(x: torch.Tensor, w: torch.Tensor, *, gated: bool = False, act: str = "silu",
                 fp32_out: bool = False) -> torch.Tensor:
-    """``x @ w.T`` with fp32 accumulation on the CUDA cores; x and w both fp32 or both bf16."""
+    """``x @ w.T`` with fp32 accumulation; x and w both fp32 or both bf16.  Products of 256 k or more of fp32 operands whose rows lie on
+    16 bytes run on the tensor cores as sums of exact bf16 parts, the others on the CUDA cores.  (The error of the parts does not grow
+    with k, 1.9e-7 of the result; that of a running sum is 1.1e-6 at 4096 k and would be the smaller one for very short sums.)"""
     M, K = x.shape
     N = w.shape[0]
     f32 = x.dtype == torch.float32
     if x.dtype != w.dtype:
         raise TypeError(f"operands of different types: {x.dtype} and {w.dtype}")
     out = torch.empty((M, N), dtype=torch.float32 if f32 or fp32_out or gated else torch.bfloat16, device=x.device)
-    rc = _lib.lib().nkb_gemm_simt(x.data_ptr(), 0 if f32 else 1, w.data_ptr(), 0 if f32 else 1, out.data_ptr(),
-                                  0 if out.dtype == torch.float32 else 1, M, N, K, x.stride(0), w.stride(0), N, _stream())
-    _lib.check(rc, "nkb_gemm_simt")
-    _count_launch()
+    if (f32 and K >= 256 and M > 0 and w.stride(0) >= K and not (K | x.stride(0) | w.stride(0)) & 3
+            and not (x.data_ptr() | w.data_ptr()) & 15):
+        kp = -(-K // 64) * 64
+        step = max((1 << 28) // (6 * kp) // 160 * 160, 160)          # rows at a time: at most 256 MB of parts of x
+        for r in range(0, M, step):
+            rows = min(step, M - r)
+            block, splits = f32_split_plan(rows, N, K)
+            planes = torch.empty((3, rows, kp), dtype=torch.bfloat16, device=x.device)
+            parts = torch.empty((splits, -(-rows * N // 4) * 4), dtype=torch.float32, device=x.device) if splits > 1 else None
+            rc = _lib.lib().nkb_gemm_f32_split(x.data_ptr() + 4 * r * x.stride(0), w.data_ptr(), out.data_ptr() + 4 * r * N,
+                                               planes.data_ptr(), _ptr(parts), rows, N, K, x.stride(0), w.stride(0), block, splits,
+                                               _stream())
+            _lib.check(rc, "nkb_gemm_f32_split")
+            _count_launch(3 if splits > 1 else 2)
+    else:
+        rc = _lib.lib().nkb_gemm_simt(x.data_ptr(), 0 if f32 else 1, w.data_ptr(), 0 if f32 else 1, out.data_ptr(),
+                                      0 if out.dtype == torch.float32 else 1, M, N, K, x.stride(0), w.stride(0), N, _stream())
+        _lib.check(rc, "nkb_gemm_simt")
+        _count_launch()
     if gated:
         return gated_act(Proj(out, 0, N // 2), Proj(out, N // 2, N // 2), act, dtype=x.dtype)
     return out

@@ -1,4 +1,4 @@
-"""32-bit products on the CUDA cores against float64, at the edges of tiles, slabs and splits."""
+"""32-bit products against float64 (CUDA cores, and tensor cores over exact bf16 parts), at the edges of tiles, slabs and splits."""
 import pytest
 import torch
 
@@ -9,7 +9,9 @@ pytestmark = pytest.mark.gpu
 # rows around the tiles of 16, 32 and 64; columns around 256 and without whole vectors; k of one slab, a ragged one, and long
 # enough to be split over a cluster
 CASES = [(1, 256, 4), (15, 255, 8), (16, 257, 12), (17, 1000, 260), (33, 4096, 4096), (64, 512, 20), (65, 770, 1028),
-         (130, 2048, 2048), (301, 4096, 4096), (301, 300, 14336)]
+         (130, 2048, 2048), (301, 4096, 4096), (301, 300, 14336), (32, 127, 256), (32, 128, 252), (1, 128, 256), (160, 129, 320),
+         (161, 300, 1028), (97, 4096, 4100), (500, 640, 2048), (40, 16, 4096),
+         (200, 1, 640), (3201, 130, 14336)]
 
 
 @pytest.mark.parametrize("m,n,k", CASES)
@@ -21,7 +23,8 @@ def test_gemm_f32(m, n, k, pitch):
     w = torch.randn((n, k + pitch), generator=g, device="cuda")[:, :k]
     y = ops.linear(x, w)
     want = x.double() @ w.double().T
-    # k roundings of partial sums that never exceed the sum of the absolute products
+    # k roundings of partial sums that never exceed the sum of the absolute products; the products of parts that are left out are
+    # below 2^-21 of a product
     bound = (k + 8) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
     assert y.shape == (m, n) and y.dtype == torch.float32
     assert ((y.double() - want).abs() <= bound).all()
@@ -38,3 +41,32 @@ def test_rows_do_not_depend_on_the_others():
     y = ops.linear(x, w)
     keep = [i for i in range(70) if i not in (3, 69)]
     assert torch.equal(y[keep], clean[keep]) and y[3].isnan().all() and not y[69].isfinite().any()
+
+
+def test_error_is_that_of_ordinary_sums():
+    g = torch.Generator(device="cuda").manual_seed(5)
+    for m, n, k in ((301, 512, 4096), (17, 256, 14336)):
+        x, w = torch.randn((m, k), generator=g, device="cuda"), torch.randn((n, k), generator=g, device="cuda")
+        want = x.double() @ w.double().T
+        # one running fp32 sum per result has about 0.3 sqrt(k) 2^-24 (1.1e-6 at 4096); slabs of 64 stay well below
+        assert float((ops.linear(x, w).double() - want).norm() / want.norm()) < 0.3 * k ** 0.5 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("n,k", [(256, 512), (100, 64)])
+def test_infinities_and_exact_parts(n, k):
+    """One infinity gives infinities of the weights' signs although its lower parts are zero; values with short significands
+    give exact products."""
+    g = torch.Generator(device="cuda").manual_seed(9)
+    x = torch.randint(-8, 9, (40, k), generator=g, device="cuda").float()
+    w = torch.randint(1, 9, (n, k), generator=g, device="cuda").float()
+    w[1::2] *= -1
+    assert torch.equal(ops.linear(x, w), (x.double() @ w.double().T).float())
+    x[2, 7] = float("inf")
+    w[3, 9] = float("-inf")
+    x[:, 9] = 1.0
+    y = ops.linear(x, w)
+    sign = torch.sign(w[:, 7])
+    rows = [j for j in range(n) if j != 3]
+    assert torch.equal(y[2, rows], sign[rows] * float("inf"))
+    assert (y[[i for i in range(40) if i != 2], 3] == float("-inf")).all()
+    ops.raise_on_device_error()
