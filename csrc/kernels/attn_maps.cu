@@ -432,14 +432,25 @@ struct MapsSimpleParams {
   const int *block_table, *q_start, *q_lens, *context_lens;
   void* out;
   int batch, max_blocks;
+  int vec;                   // keys are read in pieces of four
 };
 
 constexpr int kSimpleWarps = 4;
 
-// COLS: value columns per lane
+// four consecutive elements
+__device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 load4(const __nv_bfloat16* p) {
+  const uint2 r = *reinterpret_cast<const uint2*>(p);
+  const float2 a = unpack_bf16x2(r.x), b = unpack_bf16x2(r.y);
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+
+// COLS: value columns per lane.  Bound by the accesses to keys: a lane has a key of its own, so they go through the cache one
+// sector per lane, sixteen bytes at a time where the sizes allow it (`vec`), and by the chain of a value's loads, four of which are on
+// their way; the products keep their order.  301 tokens, 32 heads, fp32: 822 -> 274 us.
 template <typename T, int MAPS, int COLS>
 __global__ void __launch_bounds__(kSimpleWarps * 32) maps_simple_kernel(const __grid_constant__ MapsSimpleParams p) {
-  extern __shared__ float sm[];      // q [MAPS][dim_p], o [warps][MAPS][vdim_p], m [warps][MAPS], l [warps][MAPS], red[warps]
+  extern __shared__ __align__(16) float sm[];      // q [MAPS][dim_p], o [warps][MAPS][vdim_p], m [warps][MAPS], l [warps][MAPS], red[warps]
   const int t = blockIdx.x, h = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kw = MAPS * p.a.dim_p, VP = p.a.vdim_p, v_ld = p.a.v_ld;
@@ -493,7 +504,18 @@ __global__ void __launch_bounds__(kSimpleWarps * 32) maps_simple_kernel(const __
     for (int mp = 0; mp < MAPS; ++mp) {
       float s = 0.f;
       if (vis) {
-        for (int c = 0; c < p.a.dim; ++c) s = fmaf(q_s[mp * p.a.dim_p + c], cast_in<T>(kr[mp * p.a.dim_p + c]), s);
+        if (p.vec) {
+#pragma unroll 8
+          for (int c = 0; c < p.a.dim; c += 4) {
+            const float4 x = *reinterpret_cast<const float4*>(q_s + mp * p.a.dim_p + c), y = load4(kr + mp * p.a.dim_p + c);
+            s = fmaf(x.x, y.x, s);
+            s = fmaf(x.y, y.y, s);
+            s = fmaf(x.z, y.z, s);
+            s = fmaf(x.w, y.w, s);
+          }
+        } else {
+          for (int c = 0; c < p.a.dim; ++c) s = fmaf(q_s[mp * p.a.dim_p + c], cast_in<T>(kr[mp * p.a.dim_p + c]), s);
+        }
         s *= p.a.scale;
         if (p.a.softcap > 0.f) s = p.a.softcap * tanhf(s / p.a.softcap);
         if (p.a.dist_a) s -= da * log1pf(db * float(pos - key));
@@ -508,6 +530,7 @@ __global__ void __launch_bounds__(kSimpleWarps * 32) maps_simple_kernel(const __
 #pragma unroll
       for (int i = 0; i < COLS; ++i) o[mp][i] *= alpha;
     }
+#pragma unroll 4
     for (int j = 0; j < nvis; ++j) {
       float pj[MAPS];
 #pragma unroll
@@ -969,6 +992,7 @@ static int launch_simple(const MapsSimpleParams& p, dim3 grid, size_t smem, cuda
   const dim3 block(kSimpleWarps * 32);
   if (p.a.maps == 2)
     return p.a.vdim_p <= 256 ? launch_pdl(maps_simple_kernel<T, 2, 8>, grid, block, smem, s, p) : -2;
+  if (p.a.vdim_p <= 128) return launch_pdl(maps_simple_kernel<T, 1, 4>, grid, block, smem, s, p);
   if (p.a.vdim_p <= 256) return launch_pdl(maps_simple_kernel<T, 1, 8>, grid, block, smem, s, p);
   if (p.a.vdim_p <= 1024) return launch_pdl(maps_simple_kernel<T, 1, 32>, grid, block, smem, s, p);
   return -2;
@@ -986,6 +1010,7 @@ extern "C" int nkb_maps_attn_simple(const NkbMapsArgs* a, const void* q, const v
   p.a = *a; p.q = q; p.k_cache = k_cache; p.v_cache = v_cache;
   p.block_table = block_table; p.q_start = q_start; p.q_lens = q_lens; p.context_lens = context_lens;
   p.out = out; p.batch = batch; p.max_blocks = max_blocks_per_seq;
+  p.vec = ((a->dim | a->dim_p) & 3) == 0 && (reinterpret_cast<uintptr_t>(k_cache) & 15) == 0;
   const int kw = a->maps * a->dim_p;
   if (!p.a.q_token) { p.a.q_token = (long long)a->heads * kw; p.a.q_head = kw; }
   if (!p.a.o_token) { p.a.o_token = (long long)a->heads * a->vdim; p.a.o_head = a->vdim; }

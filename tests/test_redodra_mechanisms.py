@@ -520,3 +520,16 @@ def test_gated_group_norm(device, dtype, W, parts):
         got = ops.gated_group_norm(y.to(device), Proj(g.to(device), 8, W), "silu", w.to(device), parts, 1e-3, dtype)
         z = (y.double() * O.silu(gv[:, 8:])).view(5, parts, -1)
         close(got, O.rms(z, 1e-3).reshape(5, W) * w.double(), TOL[dtype])
+
+
+@on_devices
+@pytest.mark.parametrize("H,G,d,n", [(2, 1, 30, 128), (2, 2, 63, 130), (2, 1, 4, 4), (1, 1, 132, 136)])
+def test_attention_of_32_bit_rows_with_and_without_whole_pieces(device, H, G, d, n):
+    """Queries and keys of whole pieces of four values and others, values up to 128 columns and beyond."""
+    lens = [70, 33]
+    spec = MapsSpec(H, G, d, n, d ** -0.5, tiled=False)
+    seqs = [(heads(T, H, d, 10 + i, 1.5), heads(T, G, d, 20 + i), heads(T, G, n, 30 + i)) for i, T in enumerate(lens)]
+    want = [O.softmax_attention(*(x.double() for x in s), spec.scale, O.causal_mask(len(s[0]))) for s in seqs]
+    for plan in ([lens], [[37, 33], [1, 0], [32, 0]]):
+        for g, w in zip(attend(spec, seqs, device, torch.float32, plan), want):
+            close(g, w, 2e-5)            # as for the other 32-bit attentions here
