@@ -83,3 +83,39 @@ def test_argmax(rows, vocab, dtype):
     z[rows - 1, vocab // 3:] = 0.0                    # zeros of either sign are a tie
     got = ops.argmax(z.cuda()).cpu().tolist()
     assert got[rows - 1] == 0 and (rows == 1 or got[0] == vocab // 2)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_argmax_of_rows_masked_with_the_lowest_value(dtype):
+    low = torch.finfo(dtype).min
+    z = torch.full((3, 4096), low, dtype=dtype)
+    z[1, 4093], z[2, 5], z[2, 6:] = low / 2, 0.0, float("-inf")
+    assert ops.argmax(z.cuda()).cpu().tolist() == [0, 4093, 5]
+
+
+@pytest.mark.parametrize("hidden", [8, 72, 256, 260, 2048])
+@pytest.mark.parametrize("tokens,experts,k", [(1, 4, 1), (37, 8, 3), (130, 12, 9), (1501, 16, 7)])
+def test_expert_rows_and_their_sums(tokens, experts, k, hidden):
+    """Pairs around whole blocks of four, more pairs per token than are on their way at a time, rows with and without whole pieces."""
+    g = torch.Generator().manual_seed(tokens + hidden)
+    ids = torch.stack([torch.randperm(experts, generator=g)[:k] for _ in range(tokens)]).to(torch.int32)
+    x, w = rnd(tokens, hidden), torch.rand((tokens, k), generator=g)
+    lo, local = 1, experts - 1                         # the first expert is another rank's
+    here = (ids >= lo).flatten()
+    for scale in (None, w):
+        rows, offsets, pos = ops.moe_dispatch(x.cuda(), ids.cuda(), lo, local, weights=None if scale is None else scale.cuda())
+        at, n = pos.cpu().long().flatten(), int(here.sum())
+        assert offsets[-1] == n and (at[~here] == -1).all() and at[here].sort().values.tolist() == list(range(n))
+        want = x.repeat_interleave(k, 0)[here]
+        if scale is not None:
+            want = (scale.flatten()[here, None] * want.float()).to(torch.bfloat16)
+        assert torch.equal(rows.cpu()[at[here]], want)
+        by_row = torch.empty(n, dtype=torch.int32)
+        by_row[at[here]] = ids.flatten()[here]
+        assert torch.equal(by_row, by_row.sort().values)
+    if hidden % 8 == 0:
+        rows, _, pos = ops.moe_dispatch(x.cuda(), ids.cuda(), lo, local)
+        got = ops.moe_combine(rows, pos, w.cuda(), tokens).double().cpu()
+        terms = (w * here.view(tokens, k)).double()[:, :, None] * x.double()[:, None]
+        # k products summed in 32 bits, then one rounding to bf16
+        assert ((got - terms.sum(1)).abs() <= (2.0 ** -8 + k * 2.0 ** -23) * terms.abs().sum(1)).all()
