@@ -77,7 +77,7 @@ int nkb_gemm_bf16(const void* A, const void* B, void* out, int rows, int cols, i
 int nkb_gemm_effective_splits(int k, int splits);
 int nkb_gemm_bf16_2cta(const void* A, const void* B, void* out, int m, int n, int k, long long lda, long long ldb,
                        long long ldo, const void* bias, const void* residual, int gated, int gate_off, int act,
-                       float act_a, float act_b, int splits, long long split_stride, int static_b, void* stream);
+                       float act_a, float act_b, int splits, long long split_stride, int static_b, int tile_n, void* stream);
 int nkb_gemm_bf16_2cta_grouped(const void* weights, const void* x_sorted, void* out, const int* group_offsets, int num_groups,
                                int features, int k, int total_rows, long long ldx, long long ldo, int gated, int gate_off,
                                const void* bias, long long bias_group_stride, float act_limit, float act_alpha,

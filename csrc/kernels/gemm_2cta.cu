@@ -1,4 +1,4 @@
-// bf16 GEMM on CTA pairs: D[m, n] = A[m, k] * B[n, k]^T with 256 x 256 output tiles.
+// bf16 GEMM on CTA pairs: D[m, n] = A[m, k] * B[n, k]^T with output tiles of 256 x 256, or less wide ones.
 //
 // Two CTAs of a cluster (one SM each) work on one tile with `tcgen05.mma.cta_group::2`: CTA r of
 // the pair holds rows [128 r, 128 r + 128) of the A tile and rows [128 r, 128 r + 128) of the B tile in
@@ -17,6 +17,10 @@
 //   tempty[a] lives in the first CTA, count 8: the four epilogue warps of both CTAs arrive.
 // Loads are plain (non-broadcast) tiled TMA copies of this GPU's memory.
 //
+// Tile width: a round of tiles takes as long on 40 SM pairs as on all of them, and products of some hundred rows have two to five rounds.
+// Narrower tiles let the last round come out even (the caller picks the width): 414 rows of 2 x 14336 gate / up rows, 4096 of k, 3.03
+// rounds of 256 columns 126 us, 4.9 of 160 columns 106 us; at the same number of rounds per column the widest tile is the fastest.
+//
 // Reference parity: same role as gemm_tcgen05.cuh (the `dot` lowering target, prefill orientation).
 #include "gemm_tcgen05.cuh"
 #include "api.h"
@@ -26,7 +30,8 @@ namespace nkb {
 
 struct Gemm2Args {            // <= 128 bytes (see GemmArgs)
   int m, n, k;
-  int tiles_m, tiles_n;       // 256 x 256 tiles
+  int tiles_m, tiles_n;       // tiles of 256 x tile_n
+  int tile_n;                 // multiple of 32 up to 256; gated: half of it gate columns, half up columns
   int kb_total, stages;
   int group_m;                // row tiles that share one sweep over the column tiles (L2 reuse)
   int gated;                  // B holds [gate; up] rows: the pair's first CTA loads gate rows, the second up rows
@@ -45,7 +50,7 @@ struct Gemm2Args {            // <= 128 bytes (see GemmArgs)
 };
 static_assert(sizeof(Gemm2Args) <= 128, "Gemm2Args grew past the fast kernel-parameter size");
 
-constexpr int k2TileN = 256;
+constexpr int k2TileN = 256;                      // widest tile
 constexpr int k2StageBytes = 2 * kATileBytes;     // A rows + B rows of this CTA, 16 KB each
 
 // Rows of A sorted by group, one weight matrix per group (stacked in B): tile t of the list is rows [256 ct, 256 ct + 256) of a
@@ -110,6 +115,8 @@ __device__ __forceinline__ void gemm2_body(const CUtensorMap& tmA, const CUtenso
   const uint32_t rank = cluster_ctarank();        // 0 = issues the MMAs
   const int stages = args.stages;
   constexpr uint32_t tmem_cols = 2 * k2TileN;     // two accumulators of 256 columns
+  const int tile_n = GROUPED ? k2TileN : args.tile_n, half_n = tile_n / 2;     // half_n: rows of B per CTA
+  const uint32_t stage_tx = 2u * uint32_t(kATileBytes + half_n * kBlockK * 2);
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmA);
@@ -146,7 +153,7 @@ __device__ __forceinline__ void gemm2_body(const CUtensorMap& tmA, const CUtenso
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (both CTAs)
     auto b_row_of = [&](const Work2& t) {
-      return t.b_row0 + (args.gated ? (int(rank) * args.gate_off + t.tn * 128) : (t.tn * 256 + int(rank) * 128));
+      return t.b_row0 + (args.gated ? (int(rank) * args.gate_off + t.tn * half_n) : (t.tn * tile_n + int(rank) * half_n));
     };
     // Weight tiles do not depend on the preceding kernel: the first fill of the ring takes them before the wait.  (The second
     // CTA's bytes may arrive before the first one has announced them: a barrier's phase ends only with the announcement.)
@@ -156,7 +163,7 @@ __device__ __forceinline__ void gemm2_body(const CUtensorMap& tmA, const CUtenso
       pre = min(stages, t.kb1 - t.kb0);
       if (lane == 0)
         for (int i = 0; i < pre; ++i) {
-          if (rank == 0) mbar_expect_tx(&ctrl->full[i], 2 * k2StageBytes);
+          if (rank == 0) mbar_expect_tx(&ctrl->full[i], stage_tx);
           tma_load_2d_pair(tiles + i * k2StageBytes + kATileBytes, &tmB, map_to_cta(&ctrl->full[i], 0), (t.kb0 + i) * kBlockK,
                            b_row_of(t));
         }
@@ -180,7 +187,7 @@ __device__ __forceinline__ void gemm2_body(const CUtensorMap& tmA, const CUtenso
           // (its loads of this phase cannot start before the barrier entered the phase: they wait for the
           // stage to be released, which follows the previous phase's completion)
           const bool ahead = w == pair && kb - t.kb0 < pre;
-          if (rank == 0 && !ahead) mbar_expect_tx(&ctrl->full[stage], 2 * k2StageBytes);
+          if (rank == 0 && !ahead) mbar_expect_tx(&ctrl->full[stage], stage_tx);
           tma_load_2d_pair(a_ptr, &tmA, full0, kb * kBlockK, a_row);
           if (!ahead) tma_load_2d_pair(a_ptr + kATileBytes, &tmB, full0, kb * kBlockK, b_row);
         }
@@ -192,7 +199,7 @@ __device__ __forceinline__ void gemm2_body(const CUtensorMap& tmA, const CUtenso
     // ------------------------------------------------------------------ MMA issuer (first CTA of the pair)
     // One elected thread runs the whole loop alone: the tensor pipe queues only a few MMAs, so warp votes,
     // reconvergence and descriptor arithmetic between two k-blocks are time in which it drains.
-    constexpr uint32_t idesc = make_idesc_bf16(256, k2TileN, 0, 0);
+    const uint32_t idesc = make_idesc_bf16(256, tile_n, 0, 0);
     if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
@@ -249,21 +256,21 @@ __device__ __forceinline__ void gemm2_body(const CUtensorMap& tmA, const CUtenso
       const uint32_t t0 = tmem_base + (uint32_t(quad * 32) << 16) + uint32_t(acc * k2TileN);
       const int row = work.a_row0 + int(rank) * 128 + quad * 32 + lane;
       if (args.gated) {
-        // accumulator columns [0, 128) = gate, [128, 256) = up: out[:, tn * 128 + j] = silu(gate_j) * up_j
-        const int gcol0 = tn * 128;
+        // accumulator columns [0, half_n) = gate, [half_n, tile_n) = up: out[:, tn * half_n + j] = silu(gate_j) * up_j
+        const int gcol0 = tn * half_n, cend = min(args.n, gcol0 + half_n);
 #pragma unroll 1
-        for (int c = 0; c < 128; c += 32) {
+        for (int c = 0; c < half_n; c += 32) {
           uint32_t v[32], u[32];
           tmem_ld_32x32(t0 + c, v);
-          tmem_ld_32x32(t0 + 128 + c, u);
+          tmem_ld_32x32(t0 + half_n + c, u);
           tmem_ld_wait();
-          if (c + 32 >= 128) {
+          if (c + 32 >= half_n) {
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(map_to_cta(&ctrl->tempty[acc], 0));
           }
           const int cbase = gcol0 + c;
-          if (row >= work.row_end || cbase >= args.n) continue;
+          if (row >= work.row_end || cbase >= cend) continue;
           if constexpr (GROUPED) {
             if (bias) {
 #pragma unroll
@@ -291,30 +298,32 @@ __device__ __forceinline__ void gemm2_body(const CUtensorMap& tmA, const CUtenso
               v[j] = __float_as_uint(silu_f(__uint_as_float(v[j])) * __uint_as_float(u[j]));
           }
           const long long off = (long long)row * args.ldo + cbase;
-          if (cbase + 32 <= args.n && ((off & 7) == 0)) {
-            uint4* p = reinterpret_cast<uint4*>(out_h + off);
 #pragma unroll
-            for (int q = 0; q < 4; ++q)
-              p[q] = make_uint4(pack_bf16x2(__uint_as_float(v[8 * q]), __uint_as_float(v[8 * q + 1])),
-                                pack_bf16x2(__uint_as_float(v[8 * q + 2]), __uint_as_float(v[8 * q + 3])),
-                                pack_bf16x2(__uint_as_float(v[8 * q + 4]), __uint_as_float(v[8 * q + 5])),
-                                pack_bf16x2(__uint_as_float(v[8 * q + 6]), __uint_as_float(v[8 * q + 7])));
-          } else {
-            for (int j = 0; j < 32; ++j)
-              if (cbase + j < args.n) out_h[off + j] = __float2bfloat16(__uint_as_float(v[j]));
+          for (int q = 0; q < 4; ++q) {
+            if (cbase + 8 * q + 8 <= cend && (off & 7) == 0) {
+              reinterpret_cast<uint4*>(out_h + off)[q] =
+                  make_uint4(pack_bf16x2(__uint_as_float(v[8 * q]), __uint_as_float(v[8 * q + 1])),
+                             pack_bf16x2(__uint_as_float(v[8 * q + 2]), __uint_as_float(v[8 * q + 3])),
+                             pack_bf16x2(__uint_as_float(v[8 * q + 4]), __uint_as_float(v[8 * q + 5])),
+                             pack_bf16x2(__uint_as_float(v[8 * q + 6]), __uint_as_float(v[8 * q + 7])));
+            } else {
+#pragma unroll
+              for (int j = 8 * q; j < 8 * q + 8; ++j)
+                if (cbase + j < cend) out_h[off + j] = __float2bfloat16(__uint_as_float(v[j]));
+            }
           }
         }
         acc ^= 1;
         if (acc == 0) acc_phase ^= 1u;
         continue;
       }
-      const int col0 = tn * k2TileN;
+      const int col0 = tn * tile_n;
 #pragma unroll 1
-      for (int c = 0; c < k2TileN; c += 32) {
+      for (int c = 0; c < tile_n; c += 32) {
         uint32_t v[32];
         tmem_ld_32x32(t0 + c, v);
         tmem_ld_wait();
-        if (c + 32 >= k2TileN) {
+        if (c + 32 >= tile_n) {
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive_cluster(map_to_cta(&ctrl->tempty[acc], 0));
@@ -454,7 +463,7 @@ static int ring2(Gemm2Args& a) {
 using namespace nkb;
 
 // out[m, n] = A[m, k] * B[n, k]^T (+ bias[n]) (+ residual[m, n]); bf16 in and out, row strides in elements.
-// For m, n of at least a few hundred; the launcher returns -5 for shapes it does not take (callers then use
+// tile_n: columns per tile, a multiple of 32 up to 256 (gated: half of them gate, half up).  For m, n of at least a few hundred; the launcher returns -5 for shapes it does not take (callers then use
 // the single-CTA kernel).
 // Number of CTA pairs that can be resident at once (0 before the first launch).
 static int g_pairs_last = 0;
@@ -466,17 +475,19 @@ extern "C" int nkb_gemm_2cta_pairs() { return g_pairs_last; }
 extern "C" int nkb_gemm_bf16_2cta(const void* A, const void* B, void* out, int m, int n, int k, long long lda,
                                   long long ldb, long long ldo, const void* bias, const void* residual, int gated,
                                   int gate_off, int act, float act_a, float act_b, int splits, long long split_stride,
-                                  int static_b, void* stream) {
+                                  int static_b, int tile_n, void* stream) {
   if (splits < 1 || (splits > 1 && (gated || bias || residual || act))) return -2;
   if (act < 0 || (act > 2 && act != 7) || (act >= 2 && gated)) return -2;
   if (!status_word() && nkb_init() != 0) return -1;
   if (m <= 0 || n <= 0 || k <= 0) return -2;
   if ((k & 7) || (lda & 7) || (ldb & 7)) return -2;
+  if (tile_n < 32 || tile_n > k2TileN || (tile_n & 31)) return -2;
   if (n < 256) return -5;
   Gemm2Args a{};
   a.m = m; a.n = n; a.k = k;
   a.tiles_m = (m + 255) / 256;
-  a.tiles_n = gated ? (n + 127) / 128 : (n + 255) / 256;
+  a.tile_n = tile_n;
+  a.tiles_n = gated ? (n + tile_n / 2 - 1) / (tile_n / 2) : (n + tile_n - 1) / tile_n;
   a.gated = gated ? 1 : 0;
   a.gate_off = gate_off;
   a.act = act;
@@ -504,7 +515,7 @@ extern "C" int nkb_gemm_bf16_2cta(const void* A, const void* B, void* out, int m
   const int smem = ring2(a);
   CUtensorMap ta, tb;
   if (encode_tmap_bf16_2d(&ta, A, k, m, lda, kBlockK, kTileRows)) return -4;
-  if (encode_tmap_bf16_2d(&tb, B, k, gated ? uint64_t(gate_off) + n : uint64_t(n), ldb, kBlockK, kTileRows)) return -4;
+  if (encode_tmap_bf16_2d(&tb, B, k, gated ? uint64_t(gate_off) + n : uint64_t(n), ldb, kBlockK, tile_n / 2)) return -4;
   static int resident = 0;
   return launch_pairs(gemm2_kernel, &resident, a.tiles_m * a.tiles_n * splits, smem, reinterpret_cast<cudaStream_t>(stream),
                       &g_pairs_last, ta, tb, a);

@@ -88,29 +88,43 @@ def _check_bf16(*tensors):
 _USE_2CTA = os.environ.get("NKIPY_B200_GEMM_2CTA", "1") == "1"
 
 
-def _pair_tiles(rows: int, cols: int, gated: bool) -> int:
-    """256 x 256 tiles of the CTA-pair kernel (gated: 128 columns of gate and up each)."""
-    return -(-rows // 256) * -(-cols // (128 if gated else 256))
+# us that a round of 74 tiles of 256 rows takes on CTA pairs per 4096 of k, by columns per tile.  A narrower tile has fewer
+# multiply-adds per load, so its time falls less than its width; below 128 it would not fall at all.
+_PAIR_ROUND_US = {256: 24.0, 224: 21.1, 192: 18.5, 160: 16.2, 128: 15.6}
+
+
+@functools.lru_cache(maxsize=4096)
+def _pair_width(rows: int, cols: int, gated: bool, splits: int = 1) -> Tuple[int, float]:
+    """(columns per tile, us per 4096 of a split's k) of a product on CTA pairs; gated: half of the columns gate, half up.  An SM pair
+    runs its tiles one after another, so a narrower tile wins where it makes the rounds come out even.  4096 of k: 414 rows of
+    2 x 14336 gate / up 126 us at 256 columns and 106 at 160; 414 of 6144 29 and 23 at 192; 1500 of 4096 49 and 40 at 192; 2048 of 16448
+    207 and 192 at 224; 640 of 6144 29 at 256, 32 to 41 at the others."""
+    tiles_m, n = -(-rows // 256) * splits, cols * (2 if gated else 1)
+    best, best_us = 256, None
+    for width, round_us in _PAIR_ROUND_US.items():
+        us = -(-tiles_m * -(-n // width) // 74) * round_us
+        if best_us is None or us < 0.97 * best_us:
+            best, best_us = width, us
+    return best, best_us
 
 
 def _use_pairs(rows: int, cols: int, gated: bool) -> bool:
-    """Whether CTA pairs on 256 x 256 tiles beat single CTAs on 128 x 256 ones.  A round of pairs (74 tiles) takes about 24 us per
-    4096 of k, one of single CTAs (148 half-size tiles, three quarters of the loads per multiply-add more) about 31, so only
-    rounding decides: 300 rows of a 2 x 14336 gate / up product take 108 us on single CTAs and 120 on pairs, 414 rows 140 and
-    122, 200 rows 79 and 68."""
+    """Whether CTA pairs on tiles of 256 rows beat single CTAs on 128 x 256 ones, of which a round (148 tiles, three quarters of the
+    loads per multiply-add more) takes about 31 us per 4096 of k: 200 rows of a 2 x 14336 gate / up product take 79 us on single CTAs
+    and 61 on pairs, 414 rows 140 and 106."""
     if rows <= 128 or cols < 256 or not _USE_2CTA:
         return False
     single = -(-rows // 128) * -(-cols // (128 if gated else 256))
-    return rows >= 2048 or -(-_pair_tiles(rows, cols, gated) // 74) * 24 <= -(-single // 148) * 31
+    return rows >= 2048 or _pair_width(rows, cols, gated)[1] <= -(-single // 148) * 31
 
 
 def prefill_plan(rows: int, cols: int, k: int) -> Tuple[bool, int]:
     """(swap, splits) of a product whose consumer can sum split-K partials, for a packed step of `rows` tokens.
 
     Up to 128 rows a decode step's form (weights on the 128-row side, `models.transformer.pick_splits`); above, pairs of CTAs
-    split over k while their tiles leave SMs idle: a round takes 0.4 us per 64 of k, and partials are written and read once
-    at some 4 TB/s; a gain of less than 3 us is left alone.  414 rows of 14336 -> 4096: 74 us whole, 48 us in two; 130 rows: 71 and 32 us in four; 414 rows of
-    4096 -> 6144 stay whole (30 us, 33 in three)."""
+    split over k while their tiles leave SMs idle; partials are written and read once at some 4 TB/s, and a gain of less than 3 us is
+    left alone.  414 rows of 14336 -> 4096: 55 us whole, 48 in two; 130 rows: 57 and 34 us in three; 414 rows of 4096 -> 4096 stay
+    whole (19 us, 22 in two)."""
     if rows <= 128:
         from ..models.transformer import pick_splits
 
@@ -120,13 +134,13 @@ def prefill_plan(rows: int, cols: int, k: int) -> Tuple[bool, int]:
 
 @functools.lru_cache(maxsize=1024)
 def _pair_splits(rows: int, cols: int, k: int) -> int:
-    slabs, tiles = -(-k // 64), _pair_tiles(rows, cols, False)
-    best, best_cost = 1, -(-tiles // 74) * slabs * 0.4 - 3.0
+    slabs = -(-k // 64)
+    best, best_cost = 1, _pair_width(rows, cols, False)[1] * slabs / 64 - 3.0
     for s in range(2, 9):
         per = -(-slabs // s)
         if per < 8 or -(-slabs // per) != s:
             continue
-        cost = -(-tiles * s // 74) * per * 0.4 + s * rows * cols * 8 / 4e6
+        cost = _pair_width(rows, cols, False, s)[1] * per / 64 + s * rows * cols * 8 / 4e6
         if cost < best_cost:
             best, best_cost = s, cost
     return best
@@ -247,10 +261,10 @@ def linear(
     if (not swap and not fp32_out and (ldo & 7) == 0 and not (gated and (bias is not None or residual is not None))
             and (_use_pairs(M, N, gated) if splits <= 1 else
                  eff > 1 and M > 128 and N >= 256 and _USE_2CTA and bias is None and residual is None)):
-        # prefill-sized: CTA pairs on 256 x 256 tiles (csrc/kernels/gemm_2cta.cu)
+        # prefill-sized: CTA pairs on tiles of 256 rows (csrc/kernels/gemm_2cta.cu)
         rc = L.nkb_gemm_bf16_2cta(xp, wp, out_view.data_ptr(), M, N, K, ldx, ldw,
                                   ldo, _ptr(bias), _ptr(residual), 1 if gated else 0, N if gated else 0, act_code, epi.a, epi.b,
-                                  eff, split_stride, 1 if weights_static else 0, _stream())
+                                  eff, split_stride, 1 if weights_static else 0, _pair_width(M, N, gated, eff)[0], _stream())
         if rc != -5:
             _lib.check(rc, "nkb_gemm_bf16_2cta")
             _launches += 1

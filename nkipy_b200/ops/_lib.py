@@ -103,7 +103,7 @@ _SIGNATURES = {
          c_int, c_int, _P, c_int, _P, c_int, c_int, c_int, c_int, c_int, c_float, c_float, _P],
     ),
     "nkb_gemm_bf16_2cta": (c_int, [_P, _P, _P, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, _P, _P, c_int,
-                                   c_int, c_int, c_float, c_float, c_int, c_longlong, c_int, _P]),
+                                   c_int, c_int, c_float, c_float, c_int, c_longlong, c_int, c_int, _P]),
     "nkb_gemm_bf16_2cta_grouped": (c_int, [_P, _P, _P, _P, c_int, c_int, c_int, c_int, c_longlong, c_longlong, c_int, c_int, _P,
                                            c_longlong, c_float, c_float, _P, _P, c_int, _P]),
     "nkb_gemm_simt": (c_int, [_P, c_int, _P, c_int, _P, c_int, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong,

@@ -94,3 +94,32 @@ def test_one_partial_of_a_requested_split():
     assert y.shape == (1, 130, 256) and y.dtype == torch.float32
     assert ((y[0] - x.double() @ w.double().T).abs() <= 64 * 2.0 ** -23 * (x.double().abs() @ w.double().abs().T)).all()
     ops.raise_on_device_error()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("width", [32, 64, 96, 128, 160, 192, 224])
+@pytest.mark.parametrize("m,n,k", [(257, 256, 192), (130, 1000, 264), (600, 4104, 64)])
+def test_tile_widths(width, m, n, k):
+    """The width of a tile only says which CTA computes a value: every form gives the bits of the widest tile."""
+    from nkipy_b200.ops import _lib
+
+    g = torch.Generator(device="cuda").manual_seed(m + width)
+    bf = lambda *shape: torch.randn(shape, generator=g, device="cuda").to(torch.bfloat16)
+    x, w, bias, res = bf(m, k), bf(2 * n, k), bf(n), bf(m, n)
+
+    def run(tile_n, gated, act, splits, b=None, r=None):
+        pad = 8                                        # a row pitch: columns behind the result stay as they are
+        out = torch.full((splits, m, n + pad), 7.0, dtype=torch.float32 if splits > 1 else torch.bfloat16, device="cuda")
+        rc = _lib.lib().nkb_gemm_bf16_2cta(x.data_ptr(), w.data_ptr(), out.data_ptr(), m, n, k, k, k, n + pad,
+                                           b.data_ptr() if b is not None else None, r.data_ptr() if r is not None else None, int(gated),
+                                           n if gated else 0, act, 0.0, 0.0, splits, m * (n + pad) if splits > 1 else 0, 1, tile_n,
+                                           torch.cuda.current_stream().cuda_stream)
+        assert rc == 0 and (out[..., n:] == 7).all()
+        return out
+
+    res = torch.nn.functional.pad(res, (0, 8))         # rows of the residual lie as those of the output
+    forms = [(False, 0, 1), (False, 2, 1), (True, 0, 1), (True, 1, 1)] + ([(False, 0, 2)] if k > 64 else [])
+    for form in forms:
+        assert torch.equal(run(width, *form), run(256, *form)), form
+    assert torch.equal(run(width, False, 0, 1, bias, res), run(256, False, 0, 1, bias, res))
+    ops.raise_on_device_error()
