@@ -27,6 +27,15 @@ __device__ __forceinline__ void argmax_combine(float& v, int& i, float ov, int o
   }
 }
 
+// argmax_combine over the warp's lanes, by integer reductions.  Values of at least -FLT_MAX (what the lanes start from), no NaN.
+__device__ __forceinline__ void warp_argmax(float& v, int& i) {
+  const uint32_t u = __float_as_uint(v + 0.f);                           // zeros of either sign are a tie
+  const uint32_t key = u & 0x80000000u ? ~u : u | 0x80000000u;           // ordered as the values are
+  const uint32_t top = __reduce_max_sync(0xffffffffu, key);
+  i = __reduce_min_sync(0xffffffffu, key == top ? i : 0x7fffffff);
+  v = __uint_as_float(top & 0x80000000u ? top & 0x7fffffffu : ~top);
+}
+
 __global__ void argmax_kernel(const void* __restrict__ logits, int is_fp32, int* __restrict__ out_ids,
                               float* __restrict__ out_vals, int vocab, long long ld) {
   __shared__ float sv[32];
@@ -283,7 +292,9 @@ __global__ void __launch_bounds__(256) softcap_kernel(float* __restrict__ x, lon
 // largest single score take part.  The weights are multiplied by `scale`.
 // ---------------------------------------------------------------------------
 // logits may be bf16 / fp32 [tokens, E] or fp32 split-K partials [splits, tokens, E] (summed here, plus bias), rows ld apart
-// kPer: experts per lane
+// kPer: experts per lane.  A chain of latencies, so the loads of a lane's experts are on their way together, the largest value of the
+// warp is found by two integer reductions, and the weights are taken after the picks, one lane each.  128 tokens of 128 experts in 8
+// partial sums, 8 picks: 11.6 -> 4.1 us in a decode step; five prompts of up to 900 tokens 19.5 -> 9.1 us.
 template <int kPer>
 __global__ void router_topk_kernel(const void* __restrict__ logits, int is_fp32, int splits, long long split_stride,
                                    long long ld, const __nv_bfloat16* __restrict__ bias, float* __restrict__ weights,
@@ -300,16 +311,26 @@ __global__ void router_topk_kernel(const void* __restrict__ logits, int is_fp32,
 #pragma unroll
   for (int j = 0; j < kPer; ++j) {
     const int e = j * 32 + lane;
-    if (j < per && e < num_experts) {
-      float a = load_logit(logits, is_fp32, warp * ld + e);
-#pragma unroll 8
-      for (int s = 1; s < splits; ++s)
-        a += reinterpret_cast<const float*>(logits)[s * split_stride + warp * ld + e];
-      if (bias) a += __bfloat162float(bias[e]);
-      v[j] = a;
-    } else {
-      v[j] = -FLT_MAX;
+    v[j] = j < per && e < num_experts ? load_logit(logits, is_fp32, warp * ld + e) : -FLT_MAX;
+  }
+  constexpr int kAhead = kPer <= 8 ? 16 / kPer : 1;
+  for (int s0 = 1; s0 < splits; s0 += kAhead) {
+    float t[kAhead][kPer];
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i) {
+      const float* part = reinterpret_cast<const float*>(logits) + min(s0 + i, splits - 1) * split_stride + warp * ld;
+#pragma unroll
+      for (int j = 0; j < kPer; ++j) t[i][j] = part[min(j * 32 + lane, num_experts - 1)];
     }
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i)
+#pragma unroll
+      for (int j = 0; j < kPer; ++j)
+        if (s0 + i < splits && j < per && j * 32 + lane < num_experts) v[j] += t[i][j];
+  }
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    if (bias && j < per && j * 32 + lane < num_experts) v[j] += __bfloat162float(bias[j * 32 + lane]);
     mx = fmaxf(mx, v[j]);
   }
   mx = warp_max(mx);
@@ -331,12 +352,7 @@ __global__ void router_topk_kernel(const void* __restrict__ logits, int is_fp32,
 #pragma unroll
       for (int j = 0; j < kPer; ++j)
         if (j < per && !((open_bits >> j) & 1u)) argmax_combine(best, bi, v[j], j * 32 + lane);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        float ov = __shfl_xor_sync(0xffffffffu, best, o);
-        int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        argmax_combine(best, bi, ov, oi);
-      }
+      warp_argmax(best, bi);
       const int g = bi / n;
 #pragma unroll
       for (int j = 0; j < kPer; ++j)
@@ -346,8 +362,7 @@ __global__ void router_topk_kernel(const void* __restrict__ logits, int is_fp32,
     for (int j = 0; j < kPer; ++j)
       if (!((open_bits >> j) & 1u)) v[j] = -FLT_MAX;
   }
-  float sel_sum = 0.f;
-  float my_w = 0.f;
+  float my_v = 0.f;
   int my_e = 0;
   for (int r = 0; r < top_k; ++r) {
     float best = -FLT_MAX;
@@ -355,22 +370,18 @@ __global__ void router_topk_kernel(const void* __restrict__ logits, int is_fp32,
 #pragma unroll
     for (int j = 0; j < kPer; ++j)
       if (j < per) argmax_combine(best, bi, v[j], j * 32 + lane);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      float ov = __shfl_xor_sync(0xffffffffu, best, o);
-      int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      argmax_combine(best, bi, ov, oi);
-    }
-    // mode 0 weight = softmax prob; mode 1 weight = exp(logit - max selected) (first pick is the max)
-    const float wgt = mode == 2 ? 1.f / (1.f + expf(-best)) : (mode == 0) ? expf(best - mx) / denom : expf(best - mx);
-    sel_sum += wgt;
-    if (lane == r % 32 && r / 32 == 0) { my_w = wgt; my_e = bi; }
+    warp_argmax(best, bi);
+    if (lane == r) { my_v = best; my_e = bi; }
     if ((bi & 31) == lane) {
 #pragma unroll
       for (int j = 0; j < kPer; ++j)
         if (j == (bi >> 5)) v[j] = -FLT_MAX;
     }
   }
+  // mode 0 weight = softmax prob; mode 1 weight = exp(logit - max selected) (first pick is the max)
+  const float my_w = mode == 2 ? 1.f / (1.f + expf(-my_v)) : (mode == 0) ? expf(my_v - mx) / denom : expf(my_v - mx);
+  float sel_sum = 0.f;
+  for (int r = 0; r < top_k; ++r) sel_sum += __shfl_sync(0xffffffffu, my_w, r);
   if (lane < top_k) {
     weights[(long long)warp * top_k + lane] = (mode == 2 ? my_w : my_w / (sel_sum + 1e-20f)) * scale;
     experts[(long long)warp * top_k + lane] = my_e;

@@ -119,3 +119,28 @@ def test_expert_rows_and_their_sums(tokens, experts, k, hidden):
         terms = (w * here.view(tokens, k)).double()[:, :, None] * x.double()[:, None]
         # k products summed in 32 bits, then one rounding to bf16
         assert ((got - terms.sum(1)).abs() <= (2.0 ** -8 + k * 2.0 ** -23) * terms.abs().sum(1)).all()
+
+
+@pytest.mark.parametrize("experts,k,splits", [(8, 2, 1), (32, 4, 3), (60, 5, 20), (128, 8, 8), (128, 32, 17), (200, 6, 2), (1000, 8, 4)])
+@pytest.mark.parametrize("mode", ["softmax_topk", "topk_softmax", "sigmoid_topk"])
+def test_router_picks(experts, k, splits, mode):
+    """Partial sums around what is loaded ahead, experts per lane of every instance, ties, infinities and a NaN."""
+    g = torch.Generator().manual_seed(experts + splits)
+    z = torch.randn((splits, 37, experts), generator=g)
+    z[:, 3] = 0.0
+    z[0, 3, 1::2] = -0.0                              # zeros of either sign are a tie: the first experts
+    z[0, 5, experts // 2], z[0, 6, 1] = float("-inf"), float("nan")
+    w, e = ops.router_topk(z.cuda(), k, mode)
+    total = z[0].clone()
+    for s in range(1, splits):
+        total += z[s]                                 # in the kernel's order
+    order = total.nan_to_num(nan=-3e38, neginf=-3.3e38).sort(dim=-1, descending=True, stable=True).indices[:, :k]
+    rows = [i for i in range(37) if not (experts == k and i in (5, 6))]
+    assert torch.equal(e.cpu().long()[rows], order[rows])
+    top = total.double().gather(1, order)
+    keep = total.double().masked_fill(total.isnan(), float("-inf"))
+    want = top.sigmoid() if mode == "sigmoid_topk" else (top - keep.amax(-1, keepdim=True)).exp()
+    if mode != "sigmoid_topk":
+        want = want / want.sum(-1, keepdim=True)
+    # exponentials of 32-bit differences of a few units, a sum of k and a division
+    assert ((w.cpu().double() - want).abs() <= 64 * 2.0 ** -24 * want + 1e-12)[rows].all()
