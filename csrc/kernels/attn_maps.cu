@@ -445,20 +445,24 @@ __device__ __forceinline__ float4 load4(const __nv_bfloat16* p) {
   return make_float4(a.x, a.y, b.x, b.y);
 }
 
-// COLS: value columns per lane.  Bound by the accesses to keys: a lane has a key of its own, so they go through the cache one
-// sector per lane, sixteen bytes at a time where the sizes allow it (`vec`), and by the chain of a value's loads, four of which are on
-// their way; the products keep their order.  301 tokens, 32 heads, fp32: 822 -> 274 us.
-template <typename T, int MAPS, int COLS>
+// COLS: value columns per lane; HEADS: query heads of one key head that a CTA takes together.  Bound by the accesses to keys and values:
+// with a key per lane every access touches 32 lines, so where sizes allow it (`vec`) eight lanes share a key and read whole lines;
+// what is left is traffic with L2, which heads of one key head share.  301 tokens, 32 heads on 8, fp32: 822 us a value at a time,
+// 274 with a key per lane in pieces of four, 194 with eight lanes per key, 121 with four heads together.
+template <typename T, int MAPS, int COLS, int HEADS>
 __global__ void __launch_bounds__(kSimpleWarps * 32) maps_simple_kernel(const __grid_constant__ MapsSimpleParams p) {
-  extern __shared__ __align__(16) float sm[];      // q [MAPS][dim_p], o [warps][MAPS][vdim_p], m [warps][MAPS], l [warps][MAPS], red[warps]
-  const int t = blockIdx.x, h = blockIdx.y;
+  static_assert(MAPS == 1 || HEADS == 1, "maps are combined per head");
+  constexpr int R = MAPS * HEADS;                  // rows of scores
+  // q [R][dim_p], o [warps][R][vdim_p], m [warps][R], l [warps][R], red[warps]
+  extern __shared__ __align__(16) float sm[];
+  const int t = blockIdx.x, h0 = blockIdx.y * HEADS;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kw = MAPS * p.a.dim_p, VP = p.a.vdim_p, v_ld = p.a.v_ld;
   float* q_s = sm;
-  float* o_s = q_s + kw;
-  float* m_s = o_s + kSimpleWarps * MAPS * VP;
-  float* l_s = m_s + kSimpleWarps * MAPS;
-  float* red = l_s + kSimpleWarps * MAPS;
+  float* o_s = q_s + R * p.a.dim_p;
+  float* m_s = o_s + kSimpleWarps * R * VP;
+  float* l_s = m_s + kSimpleWarps * R;
+  float* red = l_s + kSimpleWarps * R;
   griddep_wait();
   griddep_launch();
   int b = -1, pos = 0;
@@ -469,28 +473,31 @@ __global__ void __launch_bounds__(kSimpleWarps * 32) maps_simple_kernel(const __
       pos = p.context_lens[i] - p.q_lens[i] + r;
     }
   }
-  T* out = reinterpret_cast<T*>(p.out) + t * p.a.o_token + h * p.a.o_head;
+  T* out0 = reinterpret_cast<T*>(p.out) + t * p.a.o_token + h0 * p.a.o_head;
   if (b < 0 || pos < 0) {
-    for (int c = threadIdx.x; c < p.a.vdim; c += blockDim.x) out[c] = cast_out<T>(0.f);
+#pragma unroll
+    for (int u = 0; u < HEADS; ++u)
+      for (int c = threadIdx.x; c < p.a.vdim; c += blockDim.x) out0[u * p.a.o_head + c] = cast_out<T>(0.f);
     return;
   }
-  const T* q = reinterpret_cast<const T*>(p.q) + t * p.a.q_token + h * p.a.q_head;
-  for (int c = threadIdx.x; c < kw; c += blockDim.x) q_s[c] = cast_in<T>(q[c]);
+  const T* q = reinterpret_cast<const T*>(p.q) + t * p.a.q_token + h0 * p.a.q_head;
+#pragma unroll
+  for (int u = 0; u < HEADS; ++u)
+    for (int c = threadIdx.x; c < kw; c += blockDim.x) q_s[u * kw + c] = cast_in<T>(q[u * p.a.q_head + c]);
   __syncthreads();
-  const int g = h / (p.a.heads / p.a.kv_heads);
+  const int g = h0 / (p.a.heads / p.a.kv_heads);
   const int* table = p.block_table + (long long)b * p.max_blocks;
-  float o[MAPS][COLS], m[MAPS], l[MAPS];
+  float o[R][COLS], m[R], l[R];
 #pragma unroll
-  for (int mp = 0; mp < MAPS; ++mp) {
-    m[mp] = -INFINITY;
-    l[mp] = 0.f;
+  for (int r = 0; r < R; ++r) {
+    m[r] = -INFINITY;
+    l[r] = 0.f;
 #pragma unroll
-    for (int i = 0; i < COLS; ++i) o[mp][i] = 0.f;
+    for (int i = 0; i < COLS; ++i) o[r][i] = 0.f;
   }
   const int pages = pos / kMapsPage + 1;
   const int lo = nkb_first_visible(pos, p.a.window, p.a.chunk), page_lo = lo / kMapsPage;
   const int keep = p.a.keep_first, kept = min((keep + kMapsPage - 1) / kMapsPage, page_lo);   // pages of kept tokens before the window
-  const float da = p.a.dist_a ? p.a.dist_a[h] : 0.f, db = p.a.dist_a ? p.a.dist_b[h] : 0.f;
   for (int i = warp; i < kept + pages - page_lo; i += kSimpleWarps) {
     const int pg = i < kept ? i : i - kept + page_lo;
     const long long blk = table[pg];
@@ -499,97 +506,127 @@ __global__ void __launch_bounds__(kSimpleWarps * 32) maps_simple_kernel(const __
     const int key = pg * kMapsPage + lane;
     const bool vis = key <= pos && (key >= lo || key < keep);
     const int nvis = min(kMapsPage, pos + 1 - pg * kMapsPage);
-    float pr[MAPS];
+    float s[R], pr[R];
 #pragma unroll
-    for (int mp = 0; mp < MAPS; ++mp) {
-      float s = 0.f;
-      if (vis) {
-        if (p.vec) {
-#pragma unroll 8
-          for (int c = 0; c < p.a.dim; c += 4) {
-            const float4 x = *reinterpret_cast<const float4*>(q_s + mp * p.a.dim_p + c), y = load4(kr + mp * p.a.dim_p + c);
-            s = fmaf(x.x, y.x, s);
-            s = fmaf(x.y, y.y, s);
-            s = fmaf(x.z, y.z, s);
-            s = fmaf(x.w, y.w, s);
+    for (int r = 0; r < R; ++r) s[r] = 0.f;
+    if (p.vec) {
+      // eight lanes per key, four keys at a time; lane j gets the sums of key j.  Rows behind the last token are read and not used.
+#pragma unroll
+      for (int mp = 0; mp < MAPS; ++mp) {
+        const T* km = kr + ((lane >> 3) - lane) * kw + mp * p.a.dim_p;
+#pragma unroll(HEADS == 1 ? 4 : 2)
+        for (int it = 0; it < kMapsPage / 4; ++it) {
+          float d[HEADS];
+#pragma unroll
+          for (int u = 0; u < HEADS; ++u) d[u] = 0.f;
+#pragma unroll 4
+          for (int c = (lane & 7) * 4; c < p.a.dim; c += 32) {
+            const float4 y = load4(km + it * 4 * kw + c);
+#pragma unroll
+            for (int u = 0; u < HEADS; ++u) {
+              const float4 x = *reinterpret_cast<const float4*>(q_s + (u * MAPS + mp) * p.a.dim_p + c);
+              d[u] = fmaf(x.x, y.x, d[u]);
+              d[u] = fmaf(x.y, y.y, d[u]);
+              d[u] = fmaf(x.z, y.z, d[u]);
+              d[u] = fmaf(x.w, y.w, d[u]);
+            }
           }
-        } else {
-          for (int c = 0; c < p.a.dim; ++c) s = fmaf(q_s[mp * p.a.dim_p + c], cast_in<T>(kr[mp * p.a.dim_p + c]), s);
-        }
-        s *= p.a.scale;
-        if (p.a.softcap > 0.f) s = p.a.softcap * tanhf(s / p.a.softcap);
-        if (p.a.dist_a) s -= da * log1pf(db * float(pos - key));
-      } else {
-        s = -INFINITY;
-      }
-      const float mn = fmaxf(m[mp], warp_max(s));            // finite: every page read holds a visible token
-      const float alpha = expf(m[mp] - mn);
-      pr[mp] = expf(s - mn);
-      l[mp] = l[mp] * alpha + warp_sum(pr[mp]);
-      m[mp] = mn;
 #pragma unroll
-      for (int i = 0; i < COLS; ++i) o[mp][i] *= alpha;
+          for (int u = 0; u < HEADS; ++u) {
+#pragma unroll
+            for (int w = 4; w > 0; w >>= 1) d[u] += __shfl_xor_sync(0xffffffffu, d[u], w);
+            d[u] = __shfl_sync(0xffffffffu, d[u], (lane & 3) * 8);
+            if (lane >> 2 == it) s[u * MAPS + mp] = d[u];
+          }
+        }
+      }
+    } else if (vis) {
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        for (int c = 0; c < p.a.dim; ++c)
+          s[r] = fmaf(q_s[r * p.a.dim_p + c], cast_in<T>(kr[r % MAPS * p.a.dim_p + c]), s[r]);
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (vis) {
+        s[r] *= p.a.scale;
+        if (p.a.softcap > 0.f) s[r] = p.a.softcap * tanhf(s[r] / p.a.softcap);
+        if (p.a.dist_a) s[r] -= p.a.dist_a[h0 + r / MAPS] * log1pf(p.a.dist_b[h0 + r / MAPS] * float(pos - key));
+      } else {
+        s[r] = -INFINITY;
+      }
+      const float mn = fmaxf(m[r], warp_max(s[r]));          // finite: every page read holds a visible token
+      const float alpha = expf(m[r] - mn);
+      pr[r] = expf(s[r] - mn);
+      l[r] = l[r] * alpha + warp_sum(pr[r]);
+      m[r] = mn;
+#pragma unroll
+      for (int i = 0; i < COLS; ++i) o[r][i] *= alpha;
     }
 #pragma unroll 4
     for (int j = 0; j < nvis; ++j) {
-      float pj[MAPS];
+      float pj[R];
 #pragma unroll
-      for (int mp = 0; mp < MAPS; ++mp) pj[mp] = __shfl_sync(0xffffffffu, pr[mp], j);
+      for (int r = 0; r < R; ++r) pj[r] = __shfl_sync(0xffffffffu, pr[r], j);
 #pragma unroll
       for (int i = 0; i < COLS; ++i) {
         const int c = lane + 32 * i;
         if (c < VP) {
           const float v = cast_in<T>(vb[j * v_ld + c]);
 #pragma unroll
-          for (int mp = 0; mp < MAPS; ++mp) o[mp][i] = fmaf(pj[mp], v, o[mp][i]);
+          for (int r = 0; r < R; ++r) o[r][i] = fmaf(pj[r], v, o[r][i]);
         }
       }
     }
   }
 #pragma unroll
-  for (int mp = 0; mp < MAPS; ++mp) {
+  for (int r = 0; r < R; ++r) {
 #pragma unroll
     for (int i = 0; i < COLS; ++i)
-      if (lane + 32 * i < VP) o_s[(warp * MAPS + mp) * VP + lane + 32 * i] = o[mp][i];
+      if (lane + 32 * i < VP) o_s[(warp * R + r) * VP + lane + 32 * i] = o[r][i];
     if (lane == 0) {
-      m_s[warp * MAPS + mp] = m[mp];
-      l_s[warp * MAPS + mp] = l[mp];
+      m_s[warp * R + r] = m[r];
+      l_s[warp * R + r] = l[r];
     }
   }
   __syncthreads();
-  float ss = 0.f;
-  for (int c = threadIdx.x; c < p.a.vdim; c += blockDim.x) {
-    float a[MAPS];
 #pragma unroll
-    for (int mp = 0; mp < MAPS; ++mp) {
-      float mx = -INFINITY, acc = 0.f, den = 0.f;
-      for (int w = 0; w < kSimpleWarps; ++w) mx = fmaxf(mx, m_s[w * MAPS + mp]);
-      if (p.a.sinks) {
-        mx = fmaxf(mx, p.a.sinks[h]);
-        den = expf(p.a.sinks[h] - mx);
+  for (int u = 0; u < HEADS; ++u) {
+    T* out = out0 + u * p.a.o_head;
+    float ss = 0.f;
+    for (int c = threadIdx.x; c < p.a.vdim; c += blockDim.x) {
+      float a[MAPS];
+#pragma unroll
+      for (int mp = 0; mp < MAPS; ++mp) {
+        const int r = u * MAPS + mp;
+        float mx = -INFINITY, acc = 0.f, den = 0.f;
+        for (int w = 0; w < kSimpleWarps; ++w) mx = fmaxf(mx, m_s[w * R + r]);
+        if (p.a.sinks) {
+          mx = fmaxf(mx, p.a.sinks[h0 + u]);
+          den = expf(p.a.sinks[h0 + u] - mx);
+        }
+        for (int w = 0; w < kSimpleWarps; ++w) {
+          const float mw = m_s[w * R + r];
+          const float f = mw == -INFINITY ? 0.f : expf(mw - mx);
+          acc += f * o_s[(w * R + r) * VP + c];
+          den += f * l_s[w * R + r];
+        }
+        a[mp] = acc / den;
       }
-      for (int w = 0; w < kSimpleWarps; ++w) {
-        const float mw = m_s[w * MAPS + mp];
-        const float f = mw == -INFINITY ? 0.f : expf(mw - mx);
-        acc += f * o_s[(w * MAPS + mp) * VP + c];
-        den += f * l_s[w * MAPS + mp];
-      }
-      a[mp] = acc / den;
+      const float v = MAPS == 2 ? a[0] - p.a.lambda * a[MAPS - 1] : a[0];
+      ss += v * v;
+      if (MAPS == 2) o_s[c] = v;                   // warp 0's map 0 slot of this column: read above by this thread only
+      else out[c] = cast_out<T>(v);
     }
-    const float r = MAPS == 2 ? a[0] - p.a.lambda * a[MAPS - 1] : a[0];
-    ss += r * r;
-    o_s[c] = r;                      // warp 0's map 0 slot of this column: read above by this thread only
-  }
-  if (MAPS == 2) {
-    ss = warp_sum(ss);
-    if (lane == 0) red[warp] = ss;
-    __syncthreads();
-    float tot = 0.f;
-    for (int w = 0; w < kSimpleWarps; ++w) tot += red[w];
-    const float inv = p.a.out_scale / sqrtf(tot / float(p.a.vdim) + p.a.eps);
-    for (int c = threadIdx.x; c < p.a.vdim; c += blockDim.x) out[c] = cast_out<T>(o_s[c] * inv);
-  } else {
-    for (int c = threadIdx.x; c < p.a.vdim; c += blockDim.x) out[c] = cast_out<T>(o_s[c]);
+    if (MAPS == 2) {
+      ss = warp_sum(ss);
+      if (lane == 0) red[warp] = ss;
+      __syncthreads();
+      float tot = 0.f;
+      for (int w = 0; w < kSimpleWarps; ++w) tot += red[w];
+      const float inv = p.a.out_scale / sqrtf(tot / float(p.a.vdim) + p.a.eps);
+      for (int c = threadIdx.x; c < p.a.vdim; c += blockDim.x) out[c] = cast_out<T>(o_s[c] * inv);
+    }
   }
 }
 
@@ -988,13 +1025,21 @@ extern "C" int nkb_rope_norm_append(const NkbMapsArgs* a, const NkbProj* q, cons
 }
 
 template <typename T>
-static int launch_simple(const MapsSimpleParams& p, dim3 grid, size_t smem, cudaStream_t s) {
-  const dim3 block(kSimpleWarps * 32);
+static int launch_simple(const MapsSimpleParams& p, int total_q, cudaStream_t s) {
+  const dim3 block(kSimpleWarps * 32), grid(total_q, p.a.heads);
+  const auto bytes = [&](int rows) { return size_t(rows * p.a.dim_p + kSimpleWarps * (rows * (p.a.vdim_p + 2) + 1)) * sizeof(float); };
+  const size_t smem = bytes(p.a.maps);
+  if (smem > 48 * 1024) return -2;
   if (p.a.maps == 2)
-    return p.a.vdim_p <= 256 ? launch_pdl(maps_simple_kernel<T, 2, 8>, grid, block, smem, s, p) : -2;
-  if (p.a.vdim_p <= 128) return launch_pdl(maps_simple_kernel<T, 1, 4>, grid, block, smem, s, p);
-  if (p.a.vdim_p <= 256) return launch_pdl(maps_simple_kernel<T, 1, 8>, grid, block, smem, s, p);
-  if (p.a.vdim_p <= 1024) return launch_pdl(maps_simple_kernel<T, 1, 32>, grid, block, smem, s, p);
+    return p.a.vdim_p <= 256 ? launch_pdl(maps_simple_kernel<T, 2, 8, 1>, grid, block, smem, s, p) : -2;
+  if (p.a.vdim_p <= 128) {
+    // four heads of a key head share what is read of it, from two CTAs per SM on: below, a CTA per head is done sooner
+    if (p.a.heads / p.a.kv_heads % 4 == 0 && (long long)total_q * p.a.heads / 4 >= 2 * num_sms() && bytes(4) <= 48 * 1024)
+      return launch_pdl(maps_simple_kernel<T, 1, 4, 4>, dim3(total_q, p.a.heads / 4), block, bytes(4), s, p);
+    return launch_pdl(maps_simple_kernel<T, 1, 4, 1>, grid, block, smem, s, p);
+  }
+  if (p.a.vdim_p <= 256) return launch_pdl(maps_simple_kernel<T, 1, 8, 1>, grid, block, smem, s, p);
+  if (p.a.vdim_p <= 1024) return launch_pdl(maps_simple_kernel<T, 1, 32, 1>, grid, block, smem, s, p);
   return -2;
 }
 
@@ -1015,11 +1060,8 @@ extern "C" int nkb_maps_attn_simple(const NkbMapsArgs* a, const void* q, const v
   if (!p.a.q_token) { p.a.q_token = (long long)a->heads * kw; p.a.q_head = kw; }
   if (!p.a.o_token) { p.a.o_token = (long long)a->heads * a->vdim; p.a.o_head = a->vdim; }
   if (!p.a.v_ld) p.a.v_ld = a->vdim_p;
-  const size_t smem = size_t(kw + kSimpleWarps * (a->maps * a->vdim_p + 5)) * sizeof(float);
-  if (smem > 48 * 1024) return -2;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  const dim3 grid(total_q, a->heads);
-  return bf16 ? launch_simple<__nv_bfloat16>(p, grid, smem, s) : launch_simple<float>(p, grid, smem, s);
+  return bf16 ? launch_simple<__nv_bfloat16>(p, total_q, s) : launch_simple<float>(p, total_q, s);
 }
 
 extern "C" long long nkb_maps_decode_scratch_floats(const NkbMapsArgs* a, int batch, int num_splits) {

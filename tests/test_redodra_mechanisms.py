@@ -523,13 +523,15 @@ def test_gated_group_norm(device, dtype, W, parts):
 
 
 @on_devices
-@pytest.mark.parametrize("H,G,d,n", [(2, 1, 30, 128), (2, 2, 63, 130), (2, 1, 4, 4), (1, 1, 132, 136)])
+@pytest.mark.parametrize("H,G,d,n", [(2, 1, 30, 128), (2, 2, 63, 130), (2, 1, 4, 4), (1, 1, 132, 136), (8, 2, 128, 128), (12, 1, 36, 20),
+                                     (8, 1, 33, 7)])
 def test_attention_of_32_bit_rows_with_and_without_whole_pieces(device, H, G, d, n):
-    """Queries and keys of whole pieces of four values and others, values up to 128 columns and beyond."""
-    lens = [70, 33]
+    """Queries and keys of whole pieces of four values and others, values up to 128 columns and beyond, four heads of a key head
+    together (many tokens) and one."""
+    lens = [170, 33]
     spec = MapsSpec(H, G, d, n, d ** -0.5, tiled=False)
     seqs = [(heads(T, H, d, 10 + i, 1.5), heads(T, G, d, 20 + i), heads(T, G, n, 30 + i)) for i, T in enumerate(lens)]
     want = [O.softmax_attention(*(x.double() for x in s), spec.scale, O.causal_mask(len(s[0]))) for s in seqs]
-    for plan in ([lens], [[37, 33], [1, 0], [32, 0]]):
+    for plan in ([lens], [[37, 33], [1, 0], [132, 0]]):
         for g, w in zip(attend(spec, seqs, device, torch.float32, plan), want):
             close(g, w, 2e-5)            # as for the other 32-bit attentions here
