@@ -44,11 +44,12 @@ struct DecodeParams {
   const int* block_table;
   const int* context_lens;
   __nv_bfloat16* out;
-  float* scratch;            // partials (behind the counters); nullptr when num_splits == 1
+  float* scratch;            // partials (behind the counters), one per unit and kv head
   unsigned int* counters;    // arrival counters of the split merge
   const float* sinks;
   int* status;
-  int batch, q_len, nq, nkv, group, max_blocks, num_splits, window, chunk;
+  int batch, q_len, nq, nkv, group, max_blocks, window, chunk;
+  int units;                 // CTAs per kv head that the sequences' pages are divided among (`plan_pages`); 0: one CTA per sequence
   float scale_log2;
   // Fused mode (qkv_partials != nullptr, q_len == 1): the kernel takes the split-K partials of the fused QKV
   // projection [splits][batch][(nq + 2 nkv) * D] instead of finished queries.  Every CTA builds its group's
@@ -185,6 +186,70 @@ __device__ __forceinline__ float modified_score(float s, const DecodeParams& p, 
 }
 
 // MODS: scores are capped, lose a term that grows with the distance, or the first tokens stay visible outside the window.
+// Pages a sequence of ctx tokens has to be read (fused: all tokens but the new one), `kept` of them first tokens' ahead of the window's.
+template <bool MODS>
+__device__ __forceinline__ int pages_of(const DecodeParams& p, int ctx, int& page_lo, int& kept) {
+  const int first_tok = nkb_first_visible(max(ctx - p.q_len, 0), p.window, p.chunk);
+  page_lo = first_tok / kPage;
+  const int page_hi = ((p.qkv_partials ? ctx - 1 : ctx) + kPage - 1) / kPage;
+  kept = MODS ? min((p.mods.keep_first + kPage - 1) / kPage, page_lo) : 0;
+  return kept + max(page_hi - page_lo, 0);
+}
+
+// Divides the pages of all sequences among `units` CTAs: every CTA of a kv head takes up to `per` pages of one sequence, per the
+// same for all, so that long sequences get more CTAs and all of them end together.  (Divided into equal numbers of CTAs per sequence, a
+// batch waits for its longest one: 7 sequences of 3500 to 7000 tokens 38.5 us, 33.7 here; one of 32000 36 and 30.)  At least `least`
+// pages each, because partial results cost a merge: one sequence of 203 tokens in single pages 15.5 us, as a whole 6.2.
+// units >= 2 * batch; returns false for a CTA without work.  One warp's lanes agree on everything.
+struct PagePlan {
+  int b, split, splits, per;
+};
+template <bool MODS>
+__device__ __forceinline__ bool plan_pages(const DecodeParams& p, int unit, int least, int lane, PagePlan& o) {
+  constexpr uint32_t kAll = 0xffffffffu;
+  int lo, kept, total = 0, mine = 0;
+  for (int i = lane; i < p.batch; i += 32) {
+    const int n = pages_of<MODS>(p, p.context_lens[i], lo, kept);
+    total += n;
+    if (i < 32) mine = n;
+  }
+  total = __reduce_add_sync(kAll, total);
+  // lane i tries first + first * i / 31 pages; the last one, twice the mean, always does: sum ceil(n / per) <= total / per + batch
+  const int first = max((total + p.units - 1) / p.units, least), per_i = first + (first * lane + 30) / 31;
+  const float inv = 1.f / float(per_i);
+  float count = 0.f;
+  for (int i0 = 0; i0 < p.batch; i0 += 32) {
+    if (i0 > 0) mine = i0 + lane < p.batch ? pages_of<MODS>(p, p.context_lens[i0 + lane], lo, kept) : 0;
+    const int m = min(p.batch - i0, 32);
+    for (int i = 0; i < m; ++i)          // (n - 1/2) / per lies half a part off any whole number, far beyond the rounding
+      count += fmaxf(ceilf((float(__shfl_sync(kAll, mine, i)) - 0.5f) * inv), 1.f);
+  }
+  const uint32_t fits = __ballot_sync(kAll, count <= float(p.units)) | 0x80000000u;
+  o.per = __shfl_sync(kAll, per_i, __ffs(fits) - 1);
+  int base = 0;                          // units of the sequences before i0
+  for (int i0 = 0; i0 < p.batch; i0 += 32) {
+    const bool in = i0 + lane < p.batch;
+    const int n = in ? pages_of<MODS>(p, p.context_lens[i0 + lane], lo, kept) : 0;
+    const int want = in ? max((n + o.per - 1) / o.per, 1) : 0;
+    int end = want;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int x = __shfl_up_sync(kAll, end, d);
+      if (lane >= d) end += x;
+    }
+    const uint32_t past = __ballot_sync(kAll, in && unit < base + end);
+    if (past) {
+      const int at = __ffs(past) - 1;
+      o.b = i0 + at;
+      o.splits = __shfl_sync(kAll, want, at);
+      o.split = unit - base - (__shfl_sync(kAll, end, at) - o.splits);
+      return true;
+    }
+    base += __shfl_sync(kAll, end, 31);
+  }
+  return false;
+}
+
 template <int D, int kDecWarps, bool MODS>
 __global__ void __launch_bounds__(kDecWarps * 32)
 paged_attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
@@ -200,7 +265,7 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
-  const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
+  const int kvh = blockIdx.y;
   const int rows = p.q_len * p.group;
 
   if (threadIdx.x == 0) {
@@ -215,24 +280,22 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
   __syncthreads();
   griddep_wait();   // q, the cache and the tables come from the preceding kernels
   griddep_launch();
+  PagePlan plan{int(blockIdx.z), 0, 1, 0x3fffffff};
+  if (p.units && !plan_pages<MODS>(p, blockIdx.x, 2 * kDecWarps, lane, plan)) return;
+  const int b = plan.b, split = plan.split;
   const int ctx = p.context_lens[b];
   const bool fused = p.qkv_partials != nullptr;       // then q_len == 1
   const bool owner = fused && split == 0 && ctx > 0;   // this CTA handles the new token's key and value
-  // tokens that are read from the cache pages: all of them, or all but the new one
-  const int ctx_paged = fused ? ctx - 1 : ctx;
 
   // ---- page range of this split
-  const int first_tok = nkb_first_visible(max(ctx - p.q_len, 0), p.window, p.chunk);
-  const int page_lo = first_tok / kPage, page_hi = (ctx_paged + kPage - 1) / kPage;
   // pages of kept first tokens come ahead of the window's (those that are not among them): walk position x is page page_at(x)
   // (without MODS the walk counts pages themselves)
-  const int kept = MODS ? min((p.mods.keep_first + kPage - 1) / kPage, page_lo) : 0;
+  int page_lo, kept;
+  const int npages = pages_of<MODS>(p, ctx, page_lo, kept);
   const int walk0 = MODS ? 0 : page_lo, shift = page_lo - kept;
   const auto page_at = [&](int x) { return !MODS || x < kept ? x : x + shift; };
-  const int npages = kept + max(page_hi - page_lo, 0);
-  const int per_split = (npages + p.num_splits - 1) / p.num_splits;
-  const int p0 = walk0 + split * per_split;
-  const int p1 = min(walk0 + npages, p0 + per_split);
+  const int p0 = walk0 + split * (plan.splits > 1 ? plan.per : 0);
+  const int p1 = min(walk0 + npages, p0 + plan.per);
   const int* table = p.block_table + (long long)b * p.max_blocks;
 
   float o[D / 8][4];
@@ -241,9 +304,8 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
   float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
 
   uint8_t* my_smem = smem + warp * kDecStages * kStageBytes;
-  auto issue = [&](int at, int stage) {
+  auto issue = [&](int blk, int stage) {
     if (lane == 0) {
-      const int blk = table[page_at(at)];
       uint8_t* dst = my_smem + stage * kStageBytes;
       mbar_expect_tx(&bars[warp][stage], kStageBytes);
 #pragma unroll
@@ -256,11 +318,15 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
 
   // ---- prologue
   const int my_first = p0 + warp;
+  int blks[kDecStages];
 #pragma unroll
   for (int s = 0; s < kDecStages; ++s) {
     const int pg = my_first + s * kDecWarps;
-    if (pg < p1) issue(pg, s);
+    blks[s] = pg < p1 ? table[page_at(pg)] : 0;
   }
+#pragma unroll
+  for (int s = 0; s < kDecStages; ++s)
+    if (my_first + s * kDecWarps < p1) issue(blks[s], s);
   // (the first pages are in flight while the queries are built)
   __shared__ __align__(16) __nv_bfloat16 q_s[16 * D]; // the group's query rows (fused mode)
   __shared__ float kn_s[D], vn_s[D], snew_s[16];
@@ -364,6 +430,9 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
   int stage = 0;
   uint32_t phase = 0;
   for (int pg = my_first; pg < p1; pg += kDecWarps) {
+    // the table is read ahead: between the last use of a stage and its next load the warp would wait for it
+    const int next = pg + kDecStages * kDecWarps;
+    const int next_blk = next < p1 ? table[page_at(next)] : 0;
     bool ok = mbar_wait(&bars[warp][stage], phase, &abort_flag, p.status, ERR_WAIT_SMEM_FULL);
     if (!__all_sync(0xffffffffu, ok)) break;
     const uint32_t kbase = smem_u32(my_smem + stage * kStageBytes);
@@ -458,8 +527,7 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
       }
     }
     __syncwarp();
-    const int next = pg + kDecStages * kDecWarps;
-    if (next < p1) issue(next, stage);
+    if (next < p1) issue(next_blk, stage);
     if (++stage == kDecStages) { stage = 0; phase ^= 1u; }
   }
   // quad-reduce the row sums
@@ -489,9 +557,7 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
     ml[warp * 16 + g] = l0; ml[warp * 16 + g + 8] = l1;
   }
   __syncthreads();
-  float* part = p.scratch
-      ? p.scratch + (((long long)b * p.nkv + kvh) * p.num_splits + split) * (16 * D + 32)
-      : nullptr;
+  float* part = plan.splits > 1 ? p.scratch + ((long long)kvh * p.units + blockIdx.x) * (16 * D + 32) : nullptr;
   for (int idx = threadIdx.x; idx < rows * D; idx += blockDim.x) {
     const int r = idx / D, d = idx % D;
     float mf = -INFINITY;
@@ -512,7 +578,7 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
       acc += sc * vn_s[d];
       l += sc;
     }
-    if (p.num_splits == 1) {
+    if (plan.splits == 1) {
       const int head = kvh * p.group + r % p.group;
       if (p.sinks) {
         const float sk = p.sinks[head] * 1.4426950408889634f;
@@ -531,7 +597,7 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
       }
     }
   }
-  if (p.num_splits == 1) return;
+  if (plan.splits == 1) return;
 
   // ---- split merge by the CTA that arrives last at this (sequence, kv head)'s counter
   __shared__ int is_last;
@@ -540,36 +606,59 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
   if (threadIdx.x == 0) {
     unsigned int* ctr = p.counters + (long long)b * p.nkv + kvh;
     const unsigned int old = atomicAdd(ctr, 1u);
-    const int last = old == unsigned(p.num_splits - 1);
+    const int last = old == unsigned(plan.splits - 1);
     if (last) *ctr = 0u;           // ready for the next call (the next kernel starts after this grid)
     is_last = last;
   }
   __syncthreads();
   if (!is_last) return;
   __threadfence();
-  const float* base = p.scratch + (((long long)b * p.nkv + kvh) * p.num_splits) * (16 * D + 32);
-  for (int idx = threadIdx.x; idx < rows * D; idx += blockDim.x) {
-    const int r = idx / D, d = idx % D;
-    float mf = -INFINITY;
-    for (int s = 0; s < p.num_splits; ++s) mf = fmaxf(mf, __ldcg(base + s * (16 * D + 32) + 16 * D + r));
-    float acc = 0.f, l = 0.f;
-    for (int s = 0; s < p.num_splits; ++s) {
-      const float* ps = base + s * (16 * D + 32);
-      const float ms = __ldcg(ps + 16 * D + r);
-      const float sc = (ms == -INFINITY) ? 0.f : exp2f(ms - mf);
-      acc += sc * __ldcg(ps + r * D + d);
-      l += sc * __ldcg(ps + 16 * D + 16 + r);
+  const float* base = p.scratch + ((long long)kvh * p.units + blockIdx.x - split) * (16 * D + 32);
+  // four columns per thread, the partials of eight splits on their way together: the merge is a chain of latencies
+  constexpr int kAhead = 8;
+  for (int idx = threadIdx.x; idx < rows * (D / 4); idx += blockDim.x) {
+    const int r = idx / (D / 4), d = idx % (D / 4) * 4;
+    float mf = -INFINITY, l = 0.f;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int s0 = 0; s0 < plan.splits; s0 += kAhead) {
+      float ms[kAhead], ls[kAhead];
+      float4 x[kAhead];
+#pragma unroll
+      for (int i = 0; i < kAhead; ++i) {
+        const float* ps = base + min(s0 + i, plan.splits - 1) * (16 * D + 32);
+        ms[i] = __ldcg(ps + 16 * D + r);
+        ls[i] = __ldcg(ps + 16 * D + 16 + r);
+        const float* v = ps + r * D + d;
+        x[i] = make_float4(__ldcg(v), __ldcg(v + 1), __ldcg(v + 2), __ldcg(v + 3));
+      }
+      float mn = mf;
+#pragma unroll
+      for (int i = 0; i < kAhead; ++i) mn = fmaxf(mn, ms[i]);
+      const float keep = mf == -INFINITY ? 0.f : exp2f(mf - mn);
+      acc.x *= keep; acc.y *= keep; acc.z *= keep; acc.w *= keep;
+      l *= keep;
+      mf = mn;
+#pragma unroll
+      for (int i = 0; i < kAhead; ++i) {
+        const float sc = s0 + i >= plan.splits || ms[i] == -INFINITY ? 0.f : exp2f(ms[i] - mn);
+        acc.x += sc * x[i].x; acc.y += sc * x[i].y; acc.z += sc * x[i].z; acc.w += sc * x[i].w;
+        l += sc * ls[i];
+      }
     }
     const int head = kvh * p.group + r % p.group;
     if (p.sinks) {
       const float sk = p.sinks[head] * 1.4426950408889634f;
       const float m2 = fmaxf(mf, sk);
       const float sc = (mf == -INFINITY) ? 0.f : exp2f(mf - m2);
-      acc *= sc;
+      acc.x *= sc; acc.y *= sc; acc.z *= sc; acc.w *= sc;
       l = l * sc + exp2f(sk - m2);
     }
-    const float v = l > 0.f ? acc / l : 0.f;
-    p.out[(((long long)b * p.q_len + r / p.group) * p.nq + head) * D + d] = __float2bfloat16(v);
+    const float inv = l > 0.f ? 1.f / l : 0.f;
+    __nv_bfloat16* out = p.out + (((long long)b * p.q_len + r / p.group) * p.nq + head) * D + d;
+    out[0] = __float2bfloat16(acc.x * inv);
+    out[1] = __float2bfloat16(acc.y * inv);
+    out[2] = __float2bfloat16(acc.z * inv);
+    out[3] = __float2bfloat16(acc.w * inv);
   }
 }
 
@@ -589,8 +678,17 @@ static int launch_decode(const CUtensorMap& tk, const CUtensorMap& tv, const Dec
     if (e != cudaSuccess) return int(e);
     attr_set[dev] = true;
   }
-  dim3 grid(p.num_splits, p.nkv, p.batch);
+  const dim3 grid = p.units ? dim3(p.units, p.nkv, 1) : dim3(1, p.nkv, p.batch);
   return launch_pdl(paged_attn_decode_kernel<D, kDecWarps, MODS>, grid, dim3(kDecWarps * 32), size_t(smem), s, tk, tv, p);
+}
+
+// Units of the page plan: num_splits per sequence, rounded up to one wave of one CTA per SM, or of two (the scratch, which is sized for nq
+// heads, has room for num_splits * group per sequence).
+static int plan_units(int batch, int nkv, int group, int num_splits) {
+  if (num_splits <= 1) return 0;
+  const int asked = batch * num_splits, one = num_sms() / nkv, two = 2 * num_sms() / nkv;
+  const int wave = asked <= one ? one : (asked <= two ? two : asked);
+  return wave < asked * group ? wave : asked * group;
 }
 
 // Warps per CTA: every warp streams its own pages through a private 3-stage ring (48 KB at D = 128), so an SM
@@ -598,8 +696,9 @@ static int launch_decode(const CUtensorMap& tk, const CUtensorMap& tv, const Dec
 // partly filled wave costs as much as a full one): four-warp CTAs while there is at most one CTA per SM, two-warp
 // CTAs up to two per SM, one-warp CTAs (four per SM) beyond.
 template <bool MODS = false>
-static int dispatch_decode(int head_dim, long long ctas, int sms, const CUtensorMap& tk, const CUtensorMap& tv,
-                           const DecodeParams& p, cudaStream_t s) {
+static int dispatch_decode(int head_dim, int sms, const CUtensorMap& tk, const CUtensorMap& tv, const DecodeParams& p,
+                           cudaStream_t s) {
+  const long long ctas = (long long)(p.units ? p.units : p.batch) * p.nkv;
   const int warps = ctas <= sms ? 4 : (ctas <= 2LL * sms ? 2 : 1);
   if (head_dim == 128) {
     if (warps == 4) return launch_decode<128, 4, MODS>(tk, tv, p, s);
@@ -649,7 +748,8 @@ extern "C" int nkb_paged_attn_decode(const void* q, const void* k_cache, const v
   p.sinks = sinks;
   p.status = status_word();
   p.batch = batch; p.q_len = q_len; p.nq = nq; p.nkv = nkv; p.group = group;
-  p.max_blocks = max_blocks_per_seq; p.num_splits = num_splits; p.window = window; p.chunk = chunk;
+  p.max_blocks = max_blocks_per_seq; p.window = window; p.chunk = chunk;
+  p.units = plan_units(batch, nkv, group, num_splits);
   if (mods) p.mods = *mods;
   p.scale_log2 = scale * 1.4426950408889634f;
   CUtensorMap tk, tv;
@@ -660,8 +760,7 @@ extern "C" int nkb_paged_attn_decode(const void* q, const void* k_cache, const v
   if (encode_tmap_bf16(&tk, k_cache, 4, dims, strides, box)) return -4;
   if (encode_tmap_bf16(&tv, v_cache, 4, dims, strides, box)) return -4;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  const long long ctas = (long long)batch * nkv * num_splits;
-  return mods ? dispatch_decode<true>(head_dim, ctas, num_sms(), tk, tv, p, s) : dispatch_decode(head_dim, ctas, num_sms(), tk, tv, p, s);
+  return mods ? dispatch_decode<true>(head_dim, num_sms(), tk, tv, p, s) : dispatch_decode(head_dim, num_sms(), tk, tv, p, s);
 }
 
 // Decode attention that starts from the split-K partials of the fused QKV projection: bias, QK-norm, RoPE and the
@@ -691,7 +790,8 @@ extern "C" int nkb_paged_attn_decode_fused(const float* qkv_partials, int qkv_sp
   p.sinks = sinks;
   p.status = status_word();
   p.batch = batch; p.q_len = 1; p.nq = nq; p.nkv = nkv; p.group = group;
-  p.max_blocks = max_blocks_per_seq; p.num_splits = num_splits; p.window = window;
+  p.max_blocks = max_blocks_per_seq; p.window = window;
+  p.units = plan_units(batch, nkv, group, num_splits);
   p.scale_log2 = scale * 1.4426950408889634f;
   p.qkv_partials = qkv_partials;
   p.qkv_split_stride = qkv_split_stride;
@@ -714,7 +814,7 @@ extern "C" int nkb_paged_attn_decode_fused(const float* qkv_partials, int qkv_sp
   if (encode_tmap_bf16(&tk, k_cache, 4, dims, strides, box)) return -4;
   if (encode_tmap_bf16(&tv, v_cache, 4, dims, strides, box)) return -4;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  return dispatch_decode(head_dim, (long long)batch * nkv * num_splits, num_sms(), tk, tv, p, s);
+  return dispatch_decode(head_dim, num_sms(), tk, tv, p, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -816,7 +916,8 @@ extern "C" int nkb_paged_attn_decode_noalloc(const void* q, const void* k_cache,
   p.sinks = sinks;
   p.status = d->status;
   p.batch = batch; p.q_len = q_len; p.nq = nq; p.nkv = nkv; p.group = group;
-  p.max_blocks = max_blocks_per_seq; p.num_splits = num_splits; p.window = window;
+  p.max_blocks = max_blocks_per_seq; p.window = window;
+  p.units = num_splits > 1 ? batch * num_splits : 0;      // what the scratch has room for
   p.scale_log2 = scale * 1.4426950408889634f;
   CUtensorMap tk, tv;
   const uint64_t dims[4] = {uint64_t(head_dim), uint64_t(kPage), uint64_t(nkv), uint64_t(num_blocks)};
@@ -825,5 +926,5 @@ extern "C" int nkb_paged_attn_decode_noalloc(const void* q, const void* k_cache,
   const uint32_t box[4] = {64, uint32_t(kPage), 1, 1};
   if (encode_tmap_bf16(&tk, k_cache, 4, dims, strides, box)) return -4;
   if (encode_tmap_bf16(&tv, v_cache, 4, dims, strides, box)) return -4;
-  return dispatch_decode(head_dim, (long long)batch * nkv * num_splits, d->sms, tk, tv, p, s);
+  return dispatch_decode(head_dim, d->sms, tk, tv, p, s);
 }

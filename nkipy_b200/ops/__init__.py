@@ -901,10 +901,10 @@ def _ref_attention(q, k, v, scale, q_pos0, causal, window, sinks, chunk=0, mods=
 
 
 def pick_kv_splits(ctas: int, max_pages: int, sms: int = 148) -> int:
-    """KV split count for decode attention.  Every warp of the kernel streams its own pages, an SM holds four
-    warps, and the kernel picks 4 / 2 / 1 warps per CTA so that the grid stays within one wave.  Splitting
-    only pays while the unsplit grid leaves SMs without a CTA: then split until about one four-warp CTA sits
-    on every SM, keeping at least two pages per warp."""
+    """KV split count for decode attention (of a sequence on average: the kernel gives long sequences more of them).  Every warp of the
+    kernel streams its own pages, an SM holds four warps, and the kernel picks 4 / 2 / 1 warps per CTA so that the grid stays within
+    one wave.  Splitting only pays while the unsplit grid leaves SMs without a CTA (16 sequences of 1000 to 2000 tokens on 8 kv
+    heads: 20.8 us unsplit, 23.7 divided): then split until about one four-warp CTA sits on every SM."""
     if ctas >= sms:
         return 1
     s = min(sms // ctas, max(max_pages // 8, 1), 16)
