@@ -18,7 +18,7 @@ partial sums the next kernel adds up; larger ones as tiled GEMMs with bf16 resul
 the epilogue.  Attention and recurrence have their own kernels for "one new token per sequence" and for packed
 prompts; both read and leave the same cache and state.
 
-`dtype` float32 runs the whole model in true 32-bit (weights, activations, cache; products on the CUDA cores).
+`dtype` float32 runs the whole model in true 32-bit (weights, activations, cache; products in 32 bits).
 """
 
 from __future__ import annotations

@@ -180,7 +180,7 @@ def linear(
     """``y = x @ w.T`` with optional fused epilogue.
 
     x: [M, K] bf16 (row stride may exceed K), w: [N, K] bf16; both fp32 for a model that runs in 32-bit, whose
-           products (and those of operands without a 16-byte row pitch) run on the CUDA cores (gemm_simt.cu).
+           products run in 32 bits (gemm_f32_split.cu, gemm_simt.cu); operands without a 16-byte row pitch run on the CUDA cores.
     gated: w is ``[2*I, K]`` holding gate rows then up rows; returns
            ``act(x @ gate.T) * (x @ up.T)`` of shape [M, I], act "silu" or "gelu_tanh".
     fp32_out: finished values in fp32 instead of bf16 (not with gated).

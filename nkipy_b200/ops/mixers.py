@@ -13,11 +13,11 @@
     heads_attention  attention with several score maps over shared values (differential attention), score soft cap;
                      with one map plain grouped-query attention, also through a sliding window (with kept first
                      tokens), inside chunks, with sinks and with a distance term
-    linear_simt      products on the CUDA cores: 32-bit models, operands TMA cannot describe
+    linear_simt      products of 32-bit models, and of operands TMA cannot describe
 
 All of them take the projections they consume as `Proj` slices, so a decode-sized batch hands over split-K partial
 sums and a prefill-sized one finished bf16 without a copy in between.  CUDA tensors run the kernels of
-csrc/kernels/{gated_residual,post_residual,recurrent,attn_maps,attn_maps_prefill,gemm_simt}.cu; CPU tensors run the PyTorch
+csrc/kernels/{gated_residual,post_residual,recurrent,attn_maps,attn_maps_prefill,gemm_simt,gemm_f32_split}.cu; CPU tensors run the PyTorch
 statement of the same op.
 """
 

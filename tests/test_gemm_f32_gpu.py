@@ -6,8 +6,8 @@ from nkipy_b200 import ops
 
 pytestmark = pytest.mark.gpu
 
-# rows around the tiles of 16, 32 and 64; columns around 256 and without whole vectors; k of one slab, a ragged one, and long
-# enough to be split over a cluster
+# rows around tiles of 32 to 160 and pieces of 3200, columns around 128, k around 256, in ragged slabs of 64 and in several ranges; sizes
+# and pitches that the CUDA cores keep
 CASES = [(1, 256, 4), (15, 255, 8), (16, 257, 12), (17, 1000, 260), (33, 4096, 4096), (64, 512, 20), (65, 770, 1028),
          (130, 2048, 2048), (301, 4096, 4096), (301, 300, 14336), (32, 127, 256), (32, 128, 252), (1, 128, 256), (160, 129, 320),
          (161, 300, 1028), (97, 4096, 4100), (500, 640, 2048), (40, 16, 4096),
