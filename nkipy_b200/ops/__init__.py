@@ -988,16 +988,20 @@ def paged_attn_decode(
     return out
 
 
-# Decode attention can read the fused QKV projection's split-K partials itself (bias, QK-norm, RoPE and the cache append
-# included) instead of running after a separate RoPE + append launch.  "1" = always, "0" and "auto" (default) = never: every CTA
-# rebuilds its group's queries before it can start, which costs more than the launch.  Decode steps fused and apart, us: 4 Llama-3-8B
-# layers 583 and 576 for one sequence, 912 and 908 for 64, 738 either way for 7 of 7000 tokens; 4 Qwen3-30B-A3B layers 1506 and 1484 for
-# 128; 4 GPT-OSS-20B layers 600 and 593 for one.
+# Decode attention reads the fused QKV projection's split-K partials itself (bias, QK-norm, RoPE and the cache append
+# included) instead of running after a separate RoPE + append launch.  "1" = always, "0" = never, "auto" (default) = on one
+# rank only: its multi-rank runs have not been re-validated.  The newest key, which usually weighs most, then takes part with its
+# probability in fp32; read from the cache like the others it would be rounded to bf16.  That is what the fused form is for: every
+# CTA rebuilds its group's queries before it can start, which costs a little more than the launch.  Decode steps fused and apart,
+# us: 4 Llama-3-8B layers 583 and 576 for one sequence, 912 and 908 for 64, 738 either way for 7 of 7000 tokens; 4 Qwen3-30B-A3B
+# layers 1506 and 1484 for 128; 4 GPT-OSS-20B layers 600 and 593 for one.
 FUSED_ROPE_ATTN = os.environ.get("NKIPY_B200_FUSED_ROPE_ATTN", "auto")
 
 
 def fused_rope_attn_enabled(world_size: int) -> bool:
-    return FUSED_ROPE_ATTN not in ("auto", "0")
+    if FUSED_ROPE_ATTN == "auto":
+        return world_size == 1
+    return FUSED_ROPE_ATTN != "0"
 
 
 def rope_attn_decode(
