@@ -1,12 +1,12 @@
 // 32-bit products on the tensor cores: out[m, n] = sum_k x[m, k] * w[n, k], all fp32.
 //
 // A 24-bit significand is exactly three 8-bit ones, so an fp32 value is the sum of three bf16 values without rounding
-// (truncation, subtraction, truncation, subtraction).  Of the nine products of two such sums the six of the largest orders are
-// taken (a1 b1, a1 b2, a2 b1, a1 b3, a2 b2, a3 b1); the others are below 2^-21 of a product at the very most and 2^-23 on
-// average.  Products of bf16 values are exact in fp32; what is not is the tensor core's accumulation, which truncates: a long sum
-// would lose a unit in the last place per step, always towards zero.  So an accumulator only ever holds one slab of 64 k, small
-// products first, and warps add the slabs up in registers with ordinary rounding.  Error against 64 bits (norm of the difference)
-// at 4096 k: 1.9e-7, one running sum in fp32 1.1e-6.
+// (truncation, subtraction, truncation, subtraction).  Of the nine products of two such sums all but the last (a3 b3, below 2^-30 of the
+// product) are taken.  Products of bf16 values are exact in fp32; what is not is the tensor core's accumulation, which truncates: a
+// long sum would lose a unit in the last place per step, always towards zero.  So an accumulator only ever holds one slab of 64 k,
+// small products first, and warps add the slabs up in registers with ordinary rounding.  Error against 64 bits (norm of the
+// difference) at 4096 k: 1.2e-7, one running sum in fp32 1.1e-6; a single product is good to 2^-23 (a multiply-add to 2^-24).  (The
+// six largest products alone, a sixth faster at 160 rows: 1.5e-7, a single product 2^-21.)
 //
 // A CTA owns 128 rows of w, BN rows of x and a range of k:
 //   warps 0-7   add finished slabs from tensor memory (two accumulators in turn): 128 rows x BN / 2 columns per four warps
@@ -14,14 +14,14 @@
 //               operand (two buffers in turn)
 //   warp 12     brings w as it is (TMA, a ring of three to six slabs)
 //   warp 13     brings the three tiles of x (TMA, two stages), which a kernel before this one has split once
-//   warp 14     issues the slab's 24 MMAs
+//   warp 14     issues the slab's 32 MMAs
 // The ranges of k of one tile go to separate planes that a last kernel adds in order.
 //
-// Bound by the six MMAs per product (1.0 us per slab of 160 rows, 1.5 with everything around them) or, with few rows, by the
+// Bound by the eight MMAs per product (1.35 us per slab of 160 rows, 1.75 with everything around them) or, with few rows, by the
 // splitting (0.95 us per slab, 3.8 TB/s of w over all SMs).  w's parts go through tensor memory because shared memory is full: with
 // w and x in stages of their own nothing waits for a load.  (w split into shared memory by the warps that loaded it, stages shared
-// with x: 385 us for 301 x 16448 x 4096, 202 here.)  4096 k, in us, before (64 x 64 tiles of multiply-adds) and now: 301 x 16448 1746
-// and 202, 301 x 4096 772 and 56, 1 x 16448 398 and 71, 301 x 4096 of 14336 k 2732 and 190.
+// with x: 385 us for six products of 301 x 16448 x 4096, 202 in this form.)  4096 k, in us behind a flushed L2, on the CUDA cores (64 x 64 tiles of
+// multiply-adds) and here: 301 x 16448 1746 and 232, 301 x 4096 772 and 71, 1 x 16448 398 and 77, 301 x 4096 of 14336 k 2732 and 204.
 //
 // Values below 2^-100 lose low bits (their third parts are below bf16's range).  A result that is not a number is computed again
 // with ordinary multiply-adds: an infinity times a part that is zero is none.
@@ -298,9 +298,9 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
         tc_fence_after();
         const uint32_t d = tmem + uint32_t(i * BN), w0 = tmem + uint32_t(2 * BN + i * kPartCols);
         const uint32_t x0 = smem_u32(x_tiles) + i * kXStage;
-        constexpr int kA[6] = {2, 1, 0, 1, 0, 0}, kB[6] = {0, 1, 2, 0, 1, 0};        // small products first
+        constexpr int kA[8] = {2, 1, 2, 1, 0, 1, 0, 0}, kB[8] = {1, 2, 0, 1, 2, 0, 1, 0};        // small products first
 #pragma unroll
-        for (int t = 0; t < 6; ++t) {
+        for (int t = 0; t < 8; ++t) {
           const uint64_t db = make_smem_desc_sw128(x0 + kB[t] * kBTile, 0, 1024);
 #pragma unroll
           for (int k = 0; k < kBlockK / 16; ++k)

@@ -183,11 +183,11 @@ def _ptr_array(ts: Sequence[Optional[torch.Tensor]]):
 @functools.lru_cache(maxsize=1024)
 def f32_split_plan(rows: int, cols: int, k: int) -> Tuple[int, int]:
     """(rows of x per tile, splits of k) of a 32-bit product on the tensor cores (gemm_f32_split.cu).  An SM runs one tile at a time; a
-    slab of 64 k takes 1 us with few rows of x and 1.5 with 160, a tile some three slabs' time around its own, and planes of partial
+    slab of 64 k takes 1 us with few rows of x and 1.75 with 160, a tile some three slabs' time around its own, and planes of partial
     sums go through the cache once more."""
     tiles = -(-rows // 160)
     block = next(b for b in (32, 64, 96, 128, 160) if b >= -(-rows // tiles))
-    slabs, slab_us = -(-k // 64), 0.9 + 0.004 * block
+    slabs, slab_us = -(-k // 64), 0.8 + 0.006 * block
     best, best_cost = 1, None
     for s in range(1, 17):
         per = -(-slabs // s)
@@ -203,7 +203,7 @@ def linear_simt(x: torch.Tensor, w: torch.Tensor, *, gated: bool = False, act: s
                 fp32_out: bool = False) -> torch.Tensor:
     """``x @ w.T`` with fp32 accumulation; x and w both fp32 or both bf16.  Products of 256 k or more of fp32 operands whose rows lie on
     16 bytes run on the tensor cores as sums of exact bf16 parts, the others on the CUDA cores.  (The error of the parts does not grow
-    with k, 1.9e-7 of the result; that of a running sum is 1.1e-6 at 4096 k and would be the smaller one for very short sums.)"""
+    with k, 1.2e-7 of the result; that of a running sum is 1.1e-6 at 4096 k and 2.9e-7 at 256.)"""
     M, K = x.shape
     N = w.shape[0]
     f32 = x.dtype == torch.float32

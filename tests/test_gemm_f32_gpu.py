@@ -23,8 +23,8 @@ def test_gemm_f32(m, n, k, pitch):
     w = torch.randn((n, k + pitch), generator=g, device="cuda")[:, :k]
     y = ops.linear(x, w)
     want = x.double() @ w.double().T
-    # k roundings of partial sums that never exceed the sum of the absolute products; the products of parts that are left out are
-    # below 2^-21 of a product
+    # k roundings of partial sums that never exceed the sum of the absolute products; the product of parts that is left out is
+    # below 2^-30 of a product
     bound = (k + 8) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
     assert y.shape == (m, n) and y.dtype == torch.float32
     assert ((y.double() - want).abs() <= bound).all()
@@ -69,4 +69,21 @@ def test_infinities_and_exact_parts(n, k):
     rows = [j for j in range(n) if j != 3]
     assert torch.equal(y[2, rows], sign[rows] * float("inf"))
     assert (y[[i for i in range(40) if i != 2], 3] == float("-inf")).all()
+    ops.raise_on_device_error()
+
+
+@pytest.mark.parametrize("terms", [1, 2])
+def test_few_terms_keep_all_their_bits(terms):
+    """Rows in which one or two products count: nothing averages out what is left out of a product."""
+    g = torch.Generator(device="cuda").manual_seed(13)
+    m, n, k = 160, 512, 4096
+    x, w = torch.zeros((m, k), device="cuda"), torch.randn((n, k), generator=g, device="cuda")
+    for i in range(terms):
+        x[torch.arange(m), (torch.arange(m) * (17 + 14 * i) + 7 * i) % k] = torch.randn(m, generator=g, device="cuda")
+    x, w = (t.view(torch.int32).bitwise_or(0xff).view(torch.float32) for t in (x, w))   # full significands
+    x[x.abs() < 1e-30] = 0.0
+    want, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    # the product left out and truncations of the accumulator while it holds lower parts, its truncation per whole product, and the
+    # rounding of the sum of two slabs
+    assert ((ops.linear(x, w).double() - want).abs() <= (2.0 ** -27 + terms * 2.0 ** -23 + (terms - 1) * 2.0 ** -24) * size).all()
     ops.raise_on_device_error()
