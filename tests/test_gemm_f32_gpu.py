@@ -87,3 +87,55 @@ def test_few_terms_keep_all_their_bits(terms):
     # rounding of the sum of two slabs
     assert ((ops.linear(x, w).double() - want).abs() <= (2.0 ** -27 + terms * 2.0 ** -23 + (terms - 1) * 2.0 ** -24) * size).all()
     ops.raise_on_device_error()
+
+
+def test_not_a_number_costs_no_more_than_numbers():
+    """Results that are not numbers are found to be none without a multiply-add for every element of their rows."""
+    g = torch.Generator(device="cuda").manual_seed(17)
+    x, w = torch.randn((301, 4096), generator=g, device="cuda"), torch.randn((2048, 4096), generator=g, device="cuda")
+    nans, column = torch.full_like(x, float("nan")), w.clone()
+    column[:, 4090] = float("nan")
+
+    def best_ms(x, w):
+        times = []
+        for _ in range(5):
+            a, b = torch.cuda.Event(True), torch.cuda.Event(True)
+            a.record()
+            y = ops.linear(x, w)
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times), y
+
+    plain, _ = best_ms(x, w)
+    for slow, y in (best_ms(nans, w), best_ms(x, column)):
+        assert y.isnan().all()
+        # 80 results of a warp, each a few loads on top of the product (thousands without the early end)
+        assert slow < 100 * plain
+    ops.raise_on_device_error()
+
+
+@pytest.mark.parametrize("splits", [1, 3])
+def test_only_infinities_are_summed_again(splits):
+    """Infinities against whole numbers (whose lower parts are zero) in rows and columns on both sides of tiles, beside NaNs."""
+    from nkipy_b200.ops import mixers
+
+    g = torch.Generator(device="cuda").manual_seed(19)
+    m, n, k = 170, 140, 1100
+    x = torch.randint(1, 9, (m, k), generator=g, device="cuda").float()
+    w = torch.randint(1, 9, (n, k), generator=g, device="cuda").float()
+    for i, j in ((0, 0), (159, 700), (160, 1099), (169, 64)):
+        x[i, j] = float("inf")
+    for i, j in ((31, 5), (127, 1098), (128, 900), (139, 64)):
+        w[i, j] = float("-inf")
+    x[100, 1099] = float("nan")
+    w[130, 3] = float("nan")
+    plan = mixers.f32_split_plan
+    mixers.f32_split_plan = lambda *a: (160, splits)
+    try:
+        y = ops.linear(x, w)
+    finally:
+        mixers.f32_split_plan = plan
+    want = (x.double() @ w.double().T).float()
+    assert torch.equal(y.isnan(), want.isnan()) and torch.equal(y.nan_to_num(7.0), want.nan_to_num(7.0))
+    ops.raise_on_device_error()
