@@ -23,8 +23,10 @@
 // with x: 385 us for six products of 301 x 16448 x 4096, 202 in this form.)  4096 k, in us behind a flushed L2, on the CUDA cores (64 x 64 tiles of
 // multiply-adds) and here: 301 x 16448 1746 and 232, 301 x 4096 772 and 71, 1 x 16448 398 and 77, 301 x 4096 of 14336 k 2732 and 204.
 //
-// Values below 2^-100 lose low bits (their third parts are below bf16's range).  A result that is not a number is computed again
-// with ordinary multiply-adds (`fs_again`): an infinity times a part that is zero is none.
+// A result that is not a number is computed again with ordinary multiply-adds (`fs_again`): an infinity times a part that is zero is
+// none.  So is one below 2^-100: the third parts of values below 2^-110 lie under bf16's smallest numbers (2^-133), and products of parts
+// under those of fp32.  Larger results do not see what is lost there, unless the other operand is beyond 2^10.  Values below 2^-133
+// count as zeros.
 #include "common.cuh"
 #include "gemm_args.h"
 #include "api.h"
@@ -118,8 +120,10 @@ __global__ void __launch_bounds__(256) f32_sum_planes_kernel(const float* __rest
   }
 }
 
-// Results in rows [r0, r0 + 32) of w and [t0, t1) of x that are not numbers, again by multiply-adds over [k0, k1), a result at a time by the
-// whole warp.  Rows that hold a NaN are left as they are, a sum that has become one ends there.  (301 x 16448 x
+// Whether a result is computed again.
+__device__ __forceinline__ bool fs_doubtful(float y) { return !(fabsf(y) >= 0x1p-100f) && y != 0.f; }
+
+// Doubtful results in rows [r0, r0 + 32) of w and [t0, t1) of x, again by multiply-adds over [k0, k1), a result at a time by the whole warp.  Rows that hold a NaN are left as they are, a sum that has become one ends there.  (301 x 16448 x
 // 4096 with every row of x NaN 0.75 ms, with a NaN in every row of w 3.4 ms, with one infinity 0.28 ms; by a thread per row of w, its
 // loads 32 rows apart, 104, 104 and 0.55 ms.)
 __device__ __noinline__ void fs_again(const float* x, const float* w, float* out, long long ldx, long long ldw, long long ldo, int r0, int n,
@@ -147,7 +151,7 @@ __device__ __noinline__ void fs_again(const float* x, const float* w, float* out
 #pragma unroll 1
   for (int t = t0; t < t1; ++t) {
     const float y = r0 + lane < n ? out[t * ldo + r0 + lane] : 0.f;
-    uint32_t bad = __ballot_sync(kAll, y != y);
+    uint32_t bad = __ballot_sync(kAll, fs_doubtful(y));
     const float* xr = x + t * ldx;
     if (bad && holds_nan(xr)) bad = 0;
 #pragma unroll 1
@@ -266,7 +270,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
       for (int j = 0; j < kCols; ++j) {
         const int t = m0 + c0 + j;
         if (t < a.m) out[t * a.ldo] = acc[j];
-        bad |= t < a.m && acc[j] != acc[j];
+        bad |= t < a.m && fs_doubtful(acc[j]);
       }
     }
     if (__any_sync(0xffffffffu, bad))

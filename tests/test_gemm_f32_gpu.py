@@ -139,3 +139,24 @@ def test_only_infinities_are_summed_again(splits):
     want = (x.double() @ w.double().T).float()
     assert torch.equal(y.isnan(), want.isnan()) and torch.equal(y.nan_to_num(7.0), want.nan_to_num(7.0))
     ops.raise_on_device_error()
+
+
+@pytest.mark.parametrize("ex,ew", [(-90, 0), (-100, 0), (-105, 0), (-110, 0), (-115, 0), (-120, 0), (-126, 0), (0, -110), (0, -120), (-60, -60), (-66, -66)])
+def test_tiny_values_keep_their_bits(ex, ew):
+    """Down to results at fp32's smallest normal numbers, where parts and their products would lie below what they can hold."""
+    g = torch.Generator(device="cuda").manual_seed(-ex - 2 * ew)
+    m, n, k = 170, 140, 516
+    x, w = (torch.randn((r, k), generator=g, device="cuda", dtype=torch.float64) * 2.0 ** e for r, e in ((m, ex), (n, ew)))
+    x, w = x.float(), w.float()
+    x[3] = 0.0
+    x[5] *= 2.0 ** 40                                       # a row of another size beside the small ones
+    y = ops.linear(x, w)
+    want, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    # ordinary sums: a rounding per term, of a number that may be denormal
+    assert ((y.double() - want).abs() <= (k + 8) * (2.0 ** -24 * size + 2.0 ** -150)).all()
+    # and no worse in the norm than one running sum per result (0.3 sqrt(k) 2^-24), wherever most terms are normal numbers
+    rows = [i for i in range(m) if i not in (3, 5)]
+    if ex + ew >= -120:
+        assert float((y[rows].double() - want[rows]).norm() / want[rows].norm()) < 0.3 * k ** 0.5 * 2.0 ** -24
+    assert (y[3] == 0).all()
+    ops.raise_on_device_error()
