@@ -176,7 +176,7 @@ def bench_moe_a2a(tp, m, args, pk, flush, g):
     def base():
         full = tp.all_gather(x).reshape(m, H)
         w_all, e_all = blk.route(lw, full)
-        plan = ops.moe_dispatch(full, e_all, blk.expert_lo, blk.num_local)
+        plan = ops.moe_dispatch(full, e_all, blk.expert_lo, blk.num_local, num_experts=E)
         h = ops.grouped_linear(plan.x_sorted, lw.gate_up, plan.offsets, max_rows_per_group=m, gated=True,
                                tiles=plan.tiles)
         y_sorted = ops.grouped_linear(h, lw.down, plan.offsets, max_rows_per_group=m, tiles=plan.tiles)

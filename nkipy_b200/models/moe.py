@@ -41,7 +41,7 @@ class MoEBlock:
         cfg = self.cfg
         T = x.shape[0]
         weights, experts = self.route(lw, x)
-        plan = ops.moe_dispatch(x, experts, self.expert_lo, self.num_local)
+        plan = ops.moe_dispatch(x, experts, self.expert_lo, self.num_local, num_experts=cfg.num_experts)
         h = ops.grouped_linear(plan.x_sorted, lw.gate_up, plan.offsets, max_rows_per_group=T, gated=True,
                                bias=lw.gate_up_bias, act_limit=cfg.swiglu_limit, act_alpha=cfg.swiglu_alpha,
                                tiles=plan.tiles)

@@ -1173,11 +1173,17 @@ def moe_tile_widths(tokens: int, per_group: float = 0.0):
     return 64, 128
 
 
+def rows_per_expert(pairs: int, expert_lo: int, num_local: int, num_experts: int = 0) -> float:
+    """Mean rows of an expert.  pairs counts those of all ranks' experts, of which there are at least expert_lo + num_local."""
+    return pairs / max(num_experts, expert_lo + num_local)
+
+
 def moe_dispatch(x: torch.Tensor, experts: torch.Tensor, expert_lo: int, num_local: int, gather: bool = True,
-                 weights: Optional[torch.Tensor] = None) -> MoEPlan:
+                 weights: Optional[torch.Tensor] = None, num_experts: int = 0) -> MoEPlan:
     """Sort the (token, expert) pairs routed to local experts [expert_lo, expert_lo + num_local) by
     expert and gather their token rows.  x [T, H] bf16 or fp32, experts [T, k] int32 (global ids); weights [T, k] fp32:
-    gathered rows are multiplied by their pair's weight.
+    gathered rows are multiplied by their pair's weight.  num_experts: experts of all ranks, where there are more than the local
+    ones (the tiles of the grouped products are chosen for the mean rows per expert).
     Returns a `MoEPlan` (unpacks to x_sorted [T * k, H], offsets int32 [num_local + 1], pair_pos int32
     [T * k]); rows past offsets[-1] of x_sorted are unspecified, pair_pos is -1 for pairs of other
     ranks' experts.  gather False: x_sorted is x itself and `row_token` names the token of every sorted row (any type and
@@ -1205,7 +1211,7 @@ def moe_dispatch(x: torch.Tensor, experts: torch.Tensor, expert_lo: int, num_loc
         x_sorted[:n_local] = rows if weights is None else (rows.float() * weights.reshape(-1)[order[:n_local], None]).to(x.dtype)
         return MoEPlan(x_sorted, offsets, pair_pos, None, T, row_token)
     global _launches
-    bn_a, bn_b = moe_tile_widths(T, pairs / num_local)
+    bn_a, bn_b = moe_tile_widths(T, rows_per_expert(pairs, expert_lo, num_local, num_experts))
     cap_a, cap_b = num_local + pairs // bn_a + 1, num_local + pairs // bn_b + 1
     if weights is not None and (not gather or weights.dtype != torch.float32 or not weights.is_contiguous()):
         raise ValueError("weights are contiguous fp32 and scale gathered rows")
