@@ -1252,8 +1252,11 @@ def grouped_linear(x_sorted: torch.Tensor, w: torch.Tensor, offsets: torch.Tenso
                    arrive: Optional[int] = None, arrive_target: int = 0) -> torch.Tensor:
     """Per-group ``y[r] = x_sorted[r] @ w[g(r)].T`` for rows sorted by group (group g owns rows
     offsets[g] .. offsets[g + 1]).  w [G, N, K] bf16 (gated: [G, 2 * I, K], gate rows then up
-    rows, output ``act(gate) * up`` of width I).  bias [G, N] is added before the activation."""
+    rows, output ``act(gate) * up`` of width I).  bias [G, N] is added before the activation.  arrive: arrival counters that the
+    tiles of the weight-side kernel wait on until they read arrive_target; not with tiles of the CTA-pair kernel."""
     R, K = x_sorted.shape
+    if arrive is not None and tiles is not None and 256 in tiles:
+        raise ValueError("the CTA-pair kernel does not wait for arrivals")
     G = w.shape[0]
     N = w.shape[1] // 2 if gated else w.shape[1]
     if not _native(x_sorted):

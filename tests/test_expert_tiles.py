@@ -33,6 +33,13 @@ def test_width_follows_the_rows_of_an_expert(monkeypatch, ranks, tokens, widths,
     assert seen["widths"] == widths
 
 
+def test_pair_tiles_refuse_arrival_counters():
+    x, w = torch.zeros((4, 64), dtype=torch.bfloat16), torch.zeros((1, 256, 64), dtype=torch.bfloat16)
+    offsets = torch.tensor([0, 4], dtype=torch.int32)
+    with pytest.raises(ValueError):
+        ops.grouped_linear(x, w, offsets, max_rows_per_group=4, tiles={256: (None, None, 1)}, arrive=1, arrive_target=1)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("lo,tokens,wide", [(0, 128, False), (12, 128, False), (0, 600, True), (8, 600, True), (12, 600, True)])
 def test_some_of_the_experts(lo, tokens, wide):
