@@ -65,7 +65,7 @@ class GenerationStats:
 
 @dataclass
 class StepEntry:
-    """New tokens of one sequence in a step, and the places among them whose logits are wanted."""
+    """New tokens of one sequence in a step, and the places among them whose logits are wanted (negative: from their end)."""
     seq: SequenceState
     tokens: Sequence[int]
     want: Sequence[int] = ()
@@ -101,6 +101,17 @@ def _token_arrays(entries: Sequence[StepEntry]) -> List[np.ndarray]:
     for e in entries:
         out.append(flat[n:n + len(e.tokens)])
         n += len(e.tokens)
+    return out
+
+
+def _wanted_places(entries: Sequence[StepEntry]) -> List[List[int]]:
+    """Wanted places of every entry among its own tokens."""
+    out = []
+    for e in entries:
+        n, places = len(e.tokens), [int(w) for w in e.want]
+        if any(not -n <= w < n for w in places):
+            raise IndexError("a wanted place lies outside its entry's tokens")
+        out.append([w % n for w in places])
     return out
 
 
@@ -356,6 +367,7 @@ class GenerationEngine:
                 raise RuntimeError(f"sequence would exceed max_seq_len={self.max_seq_len}")
         if not entries:
             return None
+        places = _wanted_places(entries)
         news = _token_arrays(entries)
         try:
             for e, new in zip(entries, news):
@@ -369,24 +381,17 @@ class GenerationEngine:
         decode = self.model.tp.world_size == 1 and all(len(e.tokens) == 1 and e.seq.num_computed > 0 for e in entries)
         logits = None
         if decode:
-            logits = self._decode_rows(entries)
+            logits = self._decode_rows(entries, [e.seq.slot for e, at in zip(entries, places) for _ in at])
         else:
-            # places count through the entries as they were given; single tokens lie ahead of portions in the batch, where
-            # attention takes them together
+            # single tokens lie ahead of portions in the batch, where attention takes them together
             order = sorted(range(len(entries)), key=lambda i: len(entries[i].tokens) > 1)
-            starts, total = np.zeros((len(entries),), dtype=np.int64), 0
+            starts, total = [0] * len(entries), 0
             for i in order:
                 starts[i] = total
                 total += len(entries[i].tokens)
-            place = np.concatenate([starts[i] + np.arange(len(e.tokens)) for i, e in enumerate(entries)])
-            rows, off = [], 0
-            for e in entries:
-                rows += [off + int(w) for w in e.want]
-                off += len(e.tokens)
-            if any(not -total <= r < total for r in rows):
-                raise IndexError("a wanted place lies outside the step's tokens")
+            rows = [starts[i] + w for i, at in enumerate(places) for w in at]
             parts = [(e.seq, e.seq.num_computed, len(e.seq.tokens)) for e in entries]
-            hidden, want = self._packed([parts[i] for i in order], [news[i] for i in order], place[rows] if rows else [])
+            hidden, want = self._packed([parts[i] for i in order], [news[i] for i in order], rows)
             if rows:
                 logits = self.model.logits(hidden.index_select(0, want))
         for e in entries:
@@ -399,8 +404,8 @@ class GenerationEngine:
             torch.cuda.current_stream().synchronize()
         return logits
 
-    def _decode_rows(self, entries: Sequence[StepEntry]) -> Optional[torch.Tensor]:
-        """A decode step of the rows in `entries` only; the other rows are inactive in it.  Returns the wanted rows' logits."""
+    def _decode_rows(self, entries: Sequence[StepEntry], rows: Sequence[int]) -> Optional[torch.Tensor]:
+        """A decode step of the rows in `entries` only; the other rows are inactive in it.  Returns the logits of `rows`."""
         self._ensure_graph()
         B, pitch = self.max_batch, self._pitch
         inputs = torch.empty((3 * pitch,), dtype=torch.int32, pin_memory=self.device.type == "cuda")
@@ -410,13 +415,16 @@ class GenerationEngine:
         ctx.fill(-1)
         ctx[slots] = [e.seq.num_computed for e in entries]
         ids[slots] = [e.seq.tokens[-1] for e in entries]
-        rows = [e.seq.slot for e in entries if len(e.want)]
         wanted = len(rows)
         host[:B] = ids
-        host[2 * pitch:2 * pitch + wanted] = rows
+        if wanted <= pitch:
+            host[2 * pitch:2 * pitch + wanted] = rows
         self._inputs.copy_(inputs, non_blocking=True)
         self.decode_step_device()
-        logits = self.step_logits.index_select(0, self._inputs[2 * pitch:2 * pitch + wanted]) if wanted else None
+        logits = None
+        if wanted:
+            at = self._inputs[2 * pitch:2 * pitch + wanted] if wanted <= pitch else self._to_device(np.array(rows, dtype=np.int32))[0]
+            logits = self.step_logits.index_select(0, at)
         if len(entries) < len(self.active):
             # the rows that were left out become active again; the others have been counted on by the step
             full = np.full((B,), -1, dtype=np.int32)

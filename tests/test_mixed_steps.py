@@ -79,3 +79,27 @@ def test_tables_and_lengths_follow_growth_and_release(device):
     with pytest.raises((OutOfBlocks, RuntimeError)):
         e.run_step([StepEntry(seqs[1], ids(300, 1))])
     assert e.cache.allocator.num_free() == free
+
+
+@pytest.mark.parametrize("device", DEVICES)
+def test_places_are_those_of_their_entry(device):
+    """In packed and in decode steps: negative places count from the entry's own end, a place wanted twice comes twice, and one
+    outside the entry is refused before anything has changed."""
+    e = engine(device)
+    a, b = e.open_request(), e.open_request()
+    p, q = ids(40, 1), ids(9, 2)
+    both = e.run_step([StepEntry(a, p, [-1, 3, 39]), StepEntry(b, q, [-9, -1])]).float()
+    assert both.shape[0] == 5
+    a.num_computed = b.num_computed = 0
+    same = e.run_step([StepEntry(a, p, [39, 3, 39]), StepEntry(b, q, [0, 8])]).float()
+    assert torch.equal(both, same)
+    free, tokens = e.cache.allocator.num_free(), (list(a.tokens), list(b.tokens))
+    for entries in ([StepEntry(a, ids(100, 3), [0]), StepEntry(b, ids(2, 4), [2])], [StepEntry(a, [5], [0]), StepEntry(b, [6], [1])],
+                    [StepEntry(a, [5], [-2])]):
+        with pytest.raises(IndexError):
+            e.run_step(entries)
+        assert (a.tokens, b.tokens) == tokens and e.cache.allocator.num_free() == free
+    once = e.run_step([StepEntry(a, [5], [0]), StepEntry(b, [6], [-1])])
+    a.num_computed, b.num_computed = 40, 9
+    many = e.run_step([StepEntry(a, [5], [0] * 70), StepEntry(b, [6], [0, 0])])
+    assert once.shape[0] == 2 and torch.equal(many, once[[0] * 70 + [1] * 2])
