@@ -368,7 +368,7 @@ class GenerationEngine:
         if not entries:
             return None
         places = _wanted_places(entries)
-        news = _token_arrays(entries)
+        news = _token_arrays(entries)        # from here on instead of the entries' tokens, which may be a sequence's own list
         try:
             for e, new in zip(entries, news):
                 tokens = e.seq.tokens
@@ -378,17 +378,17 @@ class GenerationEngine:
                     self.cache.ensure_capacity(e.seq, len(tokens), flush=False)
         finally:
             self.cache.flush()
-        decode = self.model.tp.world_size == 1 and all(len(e.tokens) == 1 and e.seq.num_computed > 0 for e in entries)
+        decode = self.model.tp.world_size == 1 and all(len(new) == 1 and e.seq.num_computed > 0 for e, new in zip(entries, news))
         logits = None
         if decode:
             logits = self._decode_rows(entries, [e.seq.slot for e, at in zip(entries, places) for _ in at])
         else:
             # single tokens lie ahead of portions in the batch, where attention takes them together
-            order = sorted(range(len(entries)), key=lambda i: len(entries[i].tokens) > 1)
+            order = sorted(range(len(entries)), key=lambda i: len(news[i]) > 1)
             starts, total = [0] * len(entries), 0
             for i in order:
                 starts[i] = total
-                total += len(entries[i].tokens)
+                total += len(news[i])
             rows = [starts[i] + w for i, at in enumerate(places) for w in at]
             parts = [(e.seq, e.seq.num_computed, len(e.seq.tokens)) for e in entries]
             hidden, want = self._packed([parts[i] for i in order], [news[i] for i in order], rows)

@@ -103,3 +103,18 @@ def test_places_are_those_of_their_entry(device):
     a.num_computed, b.num_computed = 40, 9
     many = e.run_step([StepEntry(a, [5], [0] * 70), StepEntry(b, [6], [0, 0])])
     assert once.shape[0] == 2 and torch.equal(many, once[[0] * 70 + [1] * 2])
+
+
+@pytest.mark.parametrize("device", DEVICES)
+def test_a_sequence_takes_the_tokens_of_another(device):
+    """The tokens of an entry may be another sequence's list, which the step itself makes longer."""
+    p = ids(12, 1)
+    got = []
+    for own in (False, True):
+        e = engine(device)
+        a, b, c = (e.open_request() for _ in range(3))
+        e.run_step([StepEntry(a, p)])
+        got.append(e.run_step([StepEntry(a, [7], [0]), StepEntry(b, a.tokens if own else list(p), [11]),
+                               StepEntry(c, ids(20, 5), [0, 4])]).float())
+        assert a.tokens == p + [7] and b.tokens == p and b.num_computed == 12
+    assert torch.equal(*got)
