@@ -421,8 +421,12 @@ gemm2_grouped_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
 
 // Launches `pairs` CTA pairs, at most as many as can be resident at once (the persistent loop strides by their number, and
 // pairs need two SMs of one GPC: not every SM can be paired) and as there are tiles.
+// resident: of each device, 0 before its first launch.
+constexpr int kMaxDevices = 64;
 template <typename K, typename... Args>
-static int launch_pairs(K kernel, int* resident, int total, int smem, cudaStream_t stream, int* used, const Args&... args) {
+static int launch_pairs(K kernel, int (&resident)[kMaxDevices], int total, int smem, cudaStream_t stream, int* used, const Args&... args) {
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return -1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * (num_sms() / 2));
   cfg.blockDim = dim3(kGemmThreads);
@@ -437,14 +441,14 @@ static int launch_pairs(K kernel, int* resident, int total, int smem, cudaStream
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (*resident == 0) {
+  if (resident[dev] == 0) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
     if (e != cudaSuccess) return int(e);
     int n = 0;
     e = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
-    *resident = (e == cudaSuccess && n > 0) ? n : num_sms() / 4;
+    resident[dev] = (e == cudaSuccess && n > 0) ? n : num_sms() / 4;
   }
-  const int pairs = *resident < total ? *resident : total;
+  const int pairs = resident[dev] < total ? resident[dev] : total;
   if (used) *used = pairs;
   cfg.gridDim = dim3(2 * pairs);
   cfg.numAttrs = pdl_enabled() ? 2 : 1;
@@ -463,8 +467,8 @@ static int ring2(Gemm2Args& a) {
 using namespace nkb;
 
 // out[m, n] = A[m, k] * B[n, k]^T (+ bias[n]) (+ residual[m, n]); bf16 in and out, row strides in elements.
-// tile_n: columns per tile, a multiple of 32 up to 256 (gated: half of them gate, half up).  For m, n of at least a few hundred; the launcher returns -5 for shapes it does not take (callers then use
-// the single-CTA kernel).
+// tile_n: columns per tile, a multiple of 32 up to 256 (gated: half of them gate, half up).  The launcher returns -5
+// for n below 256, which it does not take (callers then use the single-CTA kernel, as they do for 128 rows or fewer).
 // Number of CTA pairs that can be resident at once (0 before the first launch).
 static int g_pairs_last = 0;
 extern "C" int nkb_gemm_2cta_pairs() { return g_pairs_last; }
@@ -516,8 +520,8 @@ extern "C" int nkb_gemm_bf16_2cta(const void* A, const void* B, void* out, int m
   CUtensorMap ta, tb;
   if (encode_tmap_bf16_2d(&ta, A, k, m, lda, kBlockK, kTileRows)) return -4;
   if (encode_tmap_bf16_2d(&tb, B, k, gated ? uint64_t(gate_off) + n : uint64_t(n), ldb, kBlockK, tile_n / 2)) return -4;
-  static int resident = 0;
-  return launch_pairs(gemm2_kernel, &resident, a.tiles_m * a.tiles_n * splits, smem, reinterpret_cast<cudaStream_t>(stream),
+  static int resident[kMaxDevices] = {0};
+  return launch_pairs(gemm2_kernel, resident, a.tiles_m * a.tiles_n * splits, smem, reinterpret_cast<cudaStream_t>(stream),
                       &g_pairs_last, ta, tb, a);
 }
 
@@ -558,7 +562,7 @@ extern "C" int nkb_gemm_bf16_2cta_grouped(const void* weights, const void* x_sor
   CUtensorMap ta, tb;
   if (encode_tmap_bf16_2d(&ta, x_sorted, k, total_rows, ldx, kBlockK, kTileRows)) return -4;
   if (encode_tmap_bf16_2d(&tb, weights, k, uint64_t(w_rows) * num_groups, k, kBlockK, kTileRows)) return -4;
-  static int resident = 0;
-  return launch_pairs(gemm2_grouped_kernel, &resident, max_tiles * a.tiles_n, smem, reinterpret_cast<cudaStream_t>(stream),
+  static int resident[kMaxDevices] = {0};
+  return launch_pairs(gemm2_grouped_kernel, resident, max_tiles * a.tiles_n, smem, reinterpret_cast<cudaStream_t>(stream),
                       nullptr, ta, tb, a, g);
 }
