@@ -194,7 +194,7 @@ def linear(
            swapped / decode orientation: lets the next kernel's prefetch overlap this one's tail).
     weights_static: w is not written by the kernels launched just before this one, so its
            tiles may be fetched before the preceding kernel has finished (set False when w is
-           itself a fresh activation).
+           itself a fresh activation).  Whole products of 512 rows or more on CTA pairs wait in any case.
     """
     M, K = x.shape
     N = w.shape[0] // 2 if gated else w.shape[0]
@@ -261,10 +261,12 @@ def linear(
     if (not swap and not fp32_out and (ldo & 7) == 0 and not (gated and (bias is not None or residual is not None))
             and (_use_pairs(M, N, gated) if splits <= 1 else
                  eff > 1 and M > 128 and N >= 256 and _USE_2CTA and bias is None and residual is None)):
-        # prefill-sized: CTA pairs on tiles of 256 rows (csrc/kernels/gemm_2cta.cu)
+        # prefill-sized: CTA pairs on tiles of 256 rows (csrc/kernels/gemm_2cta.cu).  From 512 rows on a ring of weight tiles ahead of
+        # the wait is a hundredth of the product, less than a w that is not static after all is worth.
+        ahead = weights_static and (M < 512 or splits > 1)
         rc = L.nkb_gemm_bf16_2cta(xp, wp, out_view.data_ptr(), M, N, K, ldx, ldw,
                                   ldo, _ptr(bias), _ptr(residual), 1 if gated else 0, N if gated else 0, act_code, epi.a, epi.b,
-                                  eff, split_stride, 1 if weights_static else 0, _pair_width(M, N, gated, eff)[0], _stream())
+                                  eff, split_stride, 1 if ahead else 0, _pair_width(M, N, gated, eff)[0], _stream())
         if rc != -5:
             _lib.check(rc, "nkb_gemm_bf16_2cta")
             _launches += 1
