@@ -18,7 +18,7 @@ from __future__ import annotations
 import os
 import time
 from dataclasses import dataclass, field
-from typing import Dict, List, Optional, Sequence
+from typing import Dict, Iterable, List, Optional, Sequence
 
 import numpy as np
 import torch
@@ -473,8 +473,9 @@ class GenerationEngine:
         self.release(seqs)
         return outs
 
-    def release(self, seqs: Sequence[SequenceState]) -> None:
-        if not len(seqs):
+    def release(self, seqs: Iterable[SequenceState]) -> None:
+        seqs = list(seqs)
+        if not seqs:
             return
         # runs of neighbouring rows
         slots = sorted(s.slot for s in seqs)

@@ -118,3 +118,15 @@ def test_a_sequence_takes_the_tokens_of_another(device):
                                StepEntry(c, ids(20, 5), [0, 4])]).float())
         assert a.tokens == p + [7] and b.tokens == p and b.num_computed == 12
     assert torch.equal(*got)
+
+
+@pytest.mark.parametrize("device", DEVICES)
+def test_release_takes_any_iterable(device):
+    e = engine(device)
+    seqs = [e.open_request() for _ in range(4)]
+    e.run_step([StepEntry(s, ids(40, i)) for i, s in enumerate(seqs)])
+    e.release(s for s in seqs[:2])
+    assert set(e.active) == {s.slot for s in seqs[2:]} and e.context_lens[:4].tolist().count(-1) == 2
+    e.release(e.active.values())
+    e.release(iter(()))
+    assert not e.active and e.context_lens.tolist() == [-1] * 6
