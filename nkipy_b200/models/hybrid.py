@@ -28,14 +28,13 @@ from typing import Dict, List, Optional
 import torch
 
 from .. import ops
-from ..ops import Branch, Norm, Proj
+from ..ops import Branch, Norm, Proj, pick_splits
 from ..ops.mixers import History
 from ..parallel.comm import TPGroup
 from .config import LayerSpec, ModelConfig, RopeSpec, rope_frequencies
 from .kv_cache import BLOCK_SIZE, PagedKVCache
 from .mixers import MIXERS, Tensors, padded_rows
 from .moe import RoutedExperts
-from .transformer import pick_splits
 
 SMALL_BATCH = 128
 

@@ -21,28 +21,16 @@ over ranks, examples/models/qwen3/kernels/sampling.py:127-147).
 from __future__ import annotations
 
 import math
-import os
 from typing import Dict, List, Optional
 
 import torch
 
 from .. import ops
+from ..ops import pick_splits
 from ..parallel.comm import TPGroup
 from .config import ModelConfig, yarn_inv_freq
 from .kv_cache import PagedKVCache
 from .weights import kv_heads_for_rank, to_device_layout
-
-
-def pick_splits(n_out: int, k: int, sms: int = 148) -> int:
-    """Split-K factor for a decode-sized GEMM.  Two CTAs share an SM in that orientation,
-    so aim for about two CTAs per SM while each split still streams at least 512
-    contraction elements."""
-    tiles = (n_out + 127) // 128
-    if tiles >= 2 * sms * 3 // 4:
-        return 1
-    want = max(1, (2 * sms) // tiles)
-    min_k = int(os.environ.get("NKIPY_B200_SPLIT_MIN_K", "512"))
-    return max(1, min(want, k // min_k, 8))
 
 
 def pick_cluster_splits(tiles: int, k: int, tokens: int, sms: int = 148) -> int:

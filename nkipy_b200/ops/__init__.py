@@ -30,7 +30,7 @@ from ._lib import KernelLibraryError, device_status, raise_on_device_error
 
 __all__ = [
     "linear", "decode_linear", "qkv_rope_append", "reduce_partials", "rmsnorm", "add_rmsnorm", "silu_mul", "embedding", "rope_kv_append",
-    "argmax", "sample", "decode_advance", "router_topk", "moe_dispatch", "grouped_linear", "moe_combine", "paged_attn_decode", "flash_attn_prefill", "packed_attention", "leading_singles", "rope_table",
+    "argmax", "sample", "decode_advance", "router_topk", "moe_dispatch", "grouped_linear", "moe_combine", "paged_attn_decode", "flash_attn_prefill", "packed_attention", "leading_singles", "pick_splits", "rope_table",
     "Branch", "MapsSpec", "Norm", "Proj", "activation", "gate_heads", "gated_act", "gated_residual", "hgrn2", "maps_append",
     "heads_attention", "maps_attention", "row_norm_append", "rope_norm_append", "head_linear", "softcap",
     "LatentSpec", "latent_append", "latent_attention", "latent_gather", "latent_prefill", "latent_queries",
@@ -118,16 +118,26 @@ def _use_pairs(rows: int, cols: int, gated: bool) -> bool:
     return rows >= 2048 or _pair_width(rows, cols, gated)[1] <= -(-single // 148) * 31
 
 
+def pick_splits(n_out: int, k: int, sms: int = 148) -> int:
+    """Split-K factor for a decode-sized GEMM.  Two CTAs share an SM in that orientation,
+    so aim for about two CTAs per SM while each split still streams at least 512
+    contraction elements."""
+    tiles = (n_out + 127) // 128
+    if tiles >= 2 * sms * 3 // 4:
+        return 1
+    want = max(1, (2 * sms) // tiles)
+    min_k = int(os.environ.get("NKIPY_B200_SPLIT_MIN_K", "512"))
+    return max(1, min(want, k // min_k, 8))
+
+
 def prefill_plan(rows: int, cols: int, k: int) -> Tuple[bool, int]:
     """(swap, splits) of a product whose consumer can sum split-K partials, for a packed step of `rows` tokens.
 
-    Up to 128 rows a decode step's form (weights on the 128-row side, `models.transformer.pick_splits`); above, pairs of CTAs
+    Up to 128 rows a decode step's form (weights on the 128-row side, `pick_splits`); above, pairs of CTAs
     split over k while their tiles leave SMs idle; partials are written and read once at some 4 TB/s, and a gain of less than 3 us is
     left alone.  414 rows of 14336 -> 4096: 55 us whole, 48 in two; 130 rows: 57 and 34 us in three; 414 rows of 4096 -> 4096 stay
     whole (19 us, 22 in two)."""
     if rows <= 128:
-        from ..models.transformer import pick_splits
-
         return True, pick_splits(cols, k)
     return False, _pair_splits(rows, cols, k) if cols >= 256 and _USE_2CTA and k % 8 == 0 else 1
 
