@@ -1,14 +1,15 @@
 // Paged-KV decode attention (flash-decoding) for sm_100a.
 //
-// One CTA per (kv split, kv head, sequence).  The query rows of a CTA are the
+// One CTA per (sequence, kv head), or, for batches that would leave SMs without one, as many CTAs per kv head as
+// fill a wave, among which the pages of all its sequences are divided (`plan_pages`).  The query rows of a CTA are the
 // q_len new tokens x the GQA group of this kv head (at most 16 rows), held as
-// MMA A-fragments in registers for the whole kernel.  Each of the four warps
+// MMA A-fragments in registers for the whole kernel.  Each of its one, two or four warps
 // walks its own subset of 32-token KV pages: the page is fetched with TMA
 // (128-byte swizzle, through the per-sequence block table) into a private
 // 3-stage shared-memory ring, scores and P*V run on the tensor cores with
 // m16n8k16 fragments fed by ldmatrix, and the online-softmax state stays in
-// registers.  Warps are merged through shared memory; for long contexts the KV
-// range is split over several CTAs, each writes its partial (accumulator, running
+// registers.  Warps are merged through shared memory; where the pages of a sequence
+// are divided among several CTAs, each writes its partial (accumulator, running
 // maximum, denominator) to a scratch buffer and the CTA that arrives last at a
 // per-(sequence, kv head) counter merges them, so the whole op is one launch.
 //
@@ -55,8 +56,8 @@ struct DecodeParams {
   // projection [splits][batch][(nq + 2 nkv) * D] instead of finished queries.  Every CTA builds its group's
   // query rows itself (sum, bias, QK-norm, rotate-halves RoPE); the CTA of split 0 also builds the new
   // token's key and value, writes them to their cache slot for later steps and adds them to the softmax
-  // as one extra key, so the pages it streams stop one token earlier.  This removes the separate
-  // RoPE + append launch from every layer of a decode step.
+  // as one extra key, so the pages it streams stop one token earlier.  The newest key's probability and value stay in fp32 that
+  // way (those of cached keys are bf16 fragments), and the separate RoPE + append launch is gone from every layer.
   const float* qkv_partials;
   long long qkv_split_stride;
   const __nv_bfloat16* qkv_bias;

@@ -10,8 +10,8 @@
 //            the query of map 0 only in the first half of the contraction and that of map 1 only in the second, one
 //            accumulator receives both maps' scores, and both maps share every value fragment.  TMA page ring,
 //            splits and their merge as in attn_decode.cu; the maps are combined and normalised after the merge.
-//   simple   any sizes, any storage type, any number of new tokens: one CTA per (token, head), scores and softmax
-//            on the CUDA cores in fp32.  Serves 32-bit models and head sizes the tiled kernels do not take.
+//   simple   any sizes, any storage type, any number of new tokens: a CTA per token and head, or per token and four heads of a
+//            key head, scores and softmax on the CUDA cores in fp32.  Serves 32-bit models and head sizes the tiled kernels do not take.
 // Cache: keys [block, kv_head, 32, maps * dim_p], values [block, kv_head, 32, vdim_p]; padding columns are zero.
 #include "common.cuh"
 #include "mma_frag.cuh"

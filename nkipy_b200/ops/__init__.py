@@ -1172,6 +1172,11 @@ class MoEPlan:
         return iter((self.x_sorted, self.offsets, self.pair_pos))
 
 
+# Rows per expert from which the CTA-pair kernel takes the experts' products.  Its tiles have 256 token rows, so its time hardly depends
+# on the rows below that; that of the weight-side kernel grows with its tiles of 32 to 128 tokens.  Both products, us, weight side
+# and pairs: 128 experts of 2048 x 768 224 and 242 at 48 rows, 243 and 247 at 64, 287 and 250 at 96, 450 and 275 at 192; 32 of 2880 x
+# 2880 320 and 336 at 48, 350 and 330 at 64, 332 and 340 at 80, 425 and 360 at 128; 8 of 4096 x 14336 680 and 565 at 48, 790 and 575 at 64.
+# Between 64 and 112 rows either is ahead, by up to a tenth, from one shape and routing to the next.
 MOE_PAIR_ROWS = 64
 
 
