@@ -80,8 +80,8 @@ class Sampling:
     seed: int = 0
 
 
-def _token_arrays(entries: Sequence[StepEntry]) -> List[np.ndarray]:
-    """Token ids of every entry as int32."""
+def _token_arrays(entries: Sequence[StepEntry], lens: Sequence[int]) -> List[np.ndarray]:
+    """Token ids of every entry as int32; lens: how many each has."""
     def one(tokens) -> np.ndarray:
         try:
             a = np.asarray(tokens)
@@ -91,28 +91,25 @@ def _token_arrays(entries: Sequence[StepEntry]) -> List[np.ndarray]:
             a = np.array([int(t) for t in tokens], dtype=np.int64)
         return a
 
-    if all(len(e.tokens) == 1 for e in entries):
+    if max(lens) == 1:
         flat = one([e.tokens[0] for e in entries])
     else:
         flat = np.concatenate([one(e.tokens) for e in entries])
     if flat.size and not -2 ** 31 <= int(flat.min()) <= int(flat.max()) < 2 ** 31:
         raise ValueError("token ids are 32-bit numbers")
     flat, out, n = flat.astype(np.int32), [], 0
-    for e in entries:
-        out.append(flat[n:n + len(e.tokens)])
-        n += len(e.tokens)
+    for k in lens:
+        out.append(flat[n:n + k])
+        n += k
     return out
 
 
-def _wanted_places(entries: Sequence[StepEntry]) -> List[List[int]]:
-    """Wanted places of every entry among its own tokens."""
-    out = []
-    for e in entries:
-        n, places = len(e.tokens), [int(w) for w in e.want]
-        if any(not -n <= w < n for w in places):
-            raise IndexError("a wanted place lies outside its entry's tokens")
-        out.append([w % n for w in places])
-    return out
+def _places(want: List[int], n: int) -> List[int]:
+    """Wanted places among n tokens, from the front."""
+    places = [int(w) for w in want]
+    if any(not -n <= w < n for w in places):
+        raise IndexError("a wanted place lies outside its entry's tokens")
+    return [w % n for w in places]
 
 
 class GenerationEngine:
@@ -360,15 +357,22 @@ class GenerationEngine:
         as they are."""
         if len({e.seq.slot for e in entries}) != len(entries):
             raise ValueError("a sequence may have one entry in a step")
+        lens, places, decode = [], [], self.model.tp.world_size == 1
         for e in entries:
-            if not len(e.tokens):
+            n, done, at = len(e.tokens), e.seq.num_computed, [*e.want]
+            if not n:
                 raise ValueError("an entry needs at least one token")
-            if e.seq.num_computed + len(e.tokens) > self.max_seq_len:
+            if done + n > self.max_seq_len:
                 raise RuntimeError(f"sequence would exceed max_seq_len={self.max_seq_len}")
+            if len(at) != 1 or type(at[0]) is not int or not 0 <= at[0] < n:        # anything but one place from the front
+                at = _places(at, n)
+            if n > 1 or done <= 0:
+                decode = False
+            lens.append(n)
+            places.append(at)
         if not entries:
             return None
-        places = _wanted_places(entries)
-        news = _token_arrays(entries)        # from here on instead of the entries' tokens, which may be a sequence's own list
+        news = _token_arrays(entries, lens)        # the entries' tokens themselves may be a sequence's own list, which grows now
         try:
             for e, new in zip(entries, news):
                 tokens = e.seq.tokens
@@ -378,17 +382,16 @@ class GenerationEngine:
                     self.cache.ensure_capacity(e.seq, len(tokens), flush=False)
         finally:
             self.cache.flush()
-        decode = self.model.tp.world_size == 1 and all(len(new) == 1 and e.seq.num_computed > 0 for e, new in zip(entries, news))
         logits = None
         if decode:
             logits = self._decode_rows(entries, [e.seq.slot for e, at in zip(entries, places) for _ in at])
         else:
             # single tokens lie ahead of portions in the batch, where attention takes them together
-            order = sorted(range(len(entries)), key=lambda i: len(news[i]) > 1)
+            order = sorted(range(len(entries)), key=lambda i: lens[i] > 1)
             starts, total = [0] * len(entries), 0
             for i in order:
                 starts[i] = total
-                total += len(news[i])
+                total += lens[i]
             rows = [starts[i] + w for i, at in enumerate(places) for w in at]
             parts = [(e.seq, e.seq.num_computed, len(e.seq.tokens)) for e in entries]
             hidden, want = self._packed([parts[i] for i in order], [news[i] for i in order], rows)
