@@ -574,9 +574,10 @@ static int launch_rec(const NkbHeadRec& p, bool async, cudaStream_t s) {
 // TH threads hold 128 columns of the state at a time, in blocks of TH / 8.  Bound by streaming the state twice; what keeps it from
 // that is the time in which a CTA's loads are back and the convolution, norms and gates of its head are not.  512 threads with
 // half the columns each do that part in one pass and hold two heads per SM in 64 registers a thread: 64 sequences of 32 heads of
-// 128 x 128, 84 -> 79 us with the delta rule and 78 -> 65 us without (256 threads held one head per SM).
+// 128 x 128, 84 -> 79 us with the delta rule and 78 -> 65 us without (256 threads held one head per SM).  With 256 threads no number
+// of CTAs per SM is asked for (0): asked for one, the compiler takes twice the registers, 64 x 64 34 -> 60 us.
 template <int TH, int CH, bool DELTA, typename OutT>
-__global__ void __launch_bounds__(TH, TH == 512 ? 2 : 1) head_rec_step_kernel(const __grid_constant__ NkbHeadRec p) {
+__global__ void __launch_bounds__(TH, TH == 512 ? 2 : 0) head_rec_step_kernel(const __grid_constant__ NkbHeadRec p) {
   constexpr int D8 = 8 * CH, kCols = TH / 8, kBlocks = 128 / kCols;
   __shared__ __align__(16) float qs[D8], ks[D8];
   __shared__ float red[TH / 32], gates[3];      // decay, step size, write strength
@@ -913,7 +914,10 @@ extern "C" int nkb_head_rec_step(const NkbHeadRec* a, void* stream) {
     return -2;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (a->dim <= 32) return launch_rec_step<256, 4>(*a, s);
-  if (a->dim <= 64) return launch_rec_step<512, 8>(*a, s);
+  // 512 threads hold 128 columns in two blocks, so fewer leave half of them idle: 64 sequences of 32 heads of 64 x 64 with the delta
+  // rule, 256 and 512 threads, 36.9 and 39.3 us; of 64 x 96 39.4 and 42.4, of 64 x 128 44.9 and 45.4, of 64 x 256 68.6 and 62.2, of 96 x 64
+  // 51.9 and 49.1.
+  if (a->dim <= 64) return a->vdim < 128 ? launch_rec_step<256, 8>(*a, s) : launch_rec_step<512, 8>(*a, s);
   if (a->dim <= 128) return launch_rec_step<512, 16>(*a, s);
   return launch_rec_step<256, 32>(*a, s);
 }

@@ -428,6 +428,15 @@ def test_gated_delta_rule(device, dtype, H, G, d, n, taps, decay, strength, plan
 
 @on_devices
 @in_dtypes
+@pytest.mark.parametrize("H,G,d,n", [(2, 1, 33, 72), (2, 2, 64, 127), (2, 1, 48, 128), (3, 1, 36, 130)])
+@pytest.mark.parametrize("plan", PLANS)
+def test_delta_rule_of_small_keys(device, dtype, H, G, d, n, plan):
+    """Up to 127 value columns a step has 256 threads for a head, beyond them 512."""
+    test_gated_delta_rule(device, dtype, H, G, d, n, 4, -3.0, 0.5, plan)
+
+
+@on_devices
+@in_dtypes
 @pytest.mark.parametrize("H,G,N,n,taps,parts,decay", [
     (4, 2, 16, 24, 4, 2, 0.0), (2, 1, 128, 64, 4, 1, -3.0), (6, 6, 64, 40, 2, 3, -6.0), (3, 1, 7, 11, 3, 1, -2.0),
     (4, 1, 24, 8, 1, 16, 3.0), (2, 2, 160, 136, 5, 4, -5.0), (8, 2, 32, 128, 4, 2, -4.0), (12, 3, 8, 5, 3, 12, 0.0)])
