@@ -500,9 +500,12 @@ extern "C" int nkb_add_rmsnorm(const float* partials, int splits, long long spli
   if (nvec <= 1024) threads = (nvec + 31) / 32 * 32;
   if (threads > 1024) threads = 1024;
   if (!partials) splits = 0;
-  // From about seven warps per SM on a row per warp; fewer rows need the loads of a whole block per row in flight.
+  // From about seven warps per SM on a row per warp; fewer rows need the loads of a whole block per row in flight.  With a residual, which
+  // a lane reads behind x and not with it, from twice the rows on and up to 3072 columns: blocks and warps at 1024 rows of 2048 3.9 and
+  // 5.1 us, 4096 of 2048 11.5 and 10.5, 4096 of 2880 26.0 and 20.8, 4096 of 4096 32.1 and 43.0.
   const int lane_vecs = (nvec + 31) / 32;
-  if (!partials && x && !bias && w && normed_out && rows >= 1024 && lane_vecs <= 16 && !residual_in == !residual_out) {
+  if (!partials && x && !bias && w && normed_out && !residual_in == !residual_out &&
+      (residual_in ? rows >= 2048 && lane_vecs <= 12 : rows >= 1024 && lane_vecs <= 16)) {
     const dim3 grid((rows + 3) / 4), block(128);
     auto go = [&](auto kernel) {
       return launch_pdl(kernel, grid, block, 0, S(stream), (const __nv_bfloat16*)x, (const __nv_bfloat16*)residual_in,
