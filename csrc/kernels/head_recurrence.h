@@ -31,4 +31,5 @@ struct NkbHeadRec {
   int taps, channels, q_col, k_col, v_col, gate_act, bf16;
   int batch, tokens, heads, groups, dim, vdim;
   float q_scale, eps, unit_eps;
+  int longest;              // scan: most new tokens of a sequence, 0 where the caller does not know
 };

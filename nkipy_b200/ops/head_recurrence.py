@@ -147,7 +147,7 @@ def _recur_ref(r: HeadRecurrence, y, a, b, state, spans):
 def head_recurrence(r: HeadRecurrence, x: Proj, conv: ShortConv, a: Proj, b: Optional[Proj], gate: Proj, norm_w: torch.Tensor,
                     state: torch.Tensor, conv_state: torch.Tensor, context_lens: torch.Tensor, *, parts: int = 0,
                     gate_act: str = "silu", q_start: Optional[torch.Tensor] = None, q_lens: Optional[torch.Tensor] = None,
-                    rows: Optional[torch.Tensor] = None, dtype: torch.dtype = torch.bfloat16) -> torch.Tensor:
+                    rows: Optional[torch.Tensor] = None, dtype: torch.dtype = torch.bfloat16, max_q_len: int = 0) -> torch.Tensor:
     """The convolution of the channels x, the recurrence over them with decay logits a [T, heads] and write strengths b
     [T, heads] (delta rule only), and the norm and gate of its results o [T, heads * vdim], returned in `dtype`:
 
@@ -156,7 +156,8 @@ def head_recurrence(r: HeadRecurrence, x: Proj, conv: ShortConv, a: Proj, b: Opt
 
     state [slots, heads, vdim, dim_p] and conv_state [slots, taps, channels], fp32, are read and written in place at slot
     rows[b] (rows None: b).  context_lens counts the new tokens; a sequence whose tokens are all new starts from zero, one with
-    a negative length is skipped.  q_lens None: one new token per sequence (a decode step)."""
+    a negative length is skipped.  q_lens None: one new token per sequence (a decode step).  max_q_len: most new tokens of a sequence,
+    where the caller knows it (it decides how the tokens are worked off)."""
     T, inner = x.t.shape[-2], r.heads * r.vdim
     if r.delta != (b is not None):
         raise ValueError("the delta rule has write strengths, the state-space form has none")
@@ -202,6 +203,7 @@ def head_recurrence(r: HeadRecurrence, x: Proj, conv: ShortConv, a: Proj, b: Opt
     y = short_conv(x, conv, conv_state, context_lens, q_start, q_lens, rows, dtype=dtype)
     out = torch.empty((T, inner), dtype=dtype, device=state.device)
     arg.x, arg.q_start, arg.q_lens, arg.out = Proj(y, 0, y.shape[1]).arg(), q_start.data_ptr(), q_lens.data_ptr(), out.data_ptr()
+    arg.longest = max_q_len
     _lib.check(L.nkb_head_rec_scan(ctypes.byref(arg), _stream()), "nkb_head_rec_scan")
     _count_launch()
     if parts:
