@@ -151,6 +151,9 @@ int nkb_rope_kv_append(const void* qkv_bf16, const float* qkv_partials, int spli
                        void* stream);
 int nkb_decode_advance(int* context_lens, const int* block_table, int* positions, int* slots, int batch, int q_len,
                        int max_blocks, int block_size, void* stream);
+// Positions and cache slots of the tokens of a packed step (sequences one behind another without gaps, each with its row of the table).
+int nkb_packed_positions(const int* q_start, const int* q_lens, const int* context_lens, const int* block_table, int* positions, int* slots,
+                         int batch, int tokens, int max_blocks, int block_size, void* stream);
 int nkb_argmax(const void* logits, int is_fp32, int* out_ids, float* out_vals, int rows, int vocab, long long ld,
                void* stream);
 int nkb_sample(const void* logits, int is_fp32, int* out_ids, int rows, int vocab, long long ld, float temperature,

@@ -16,6 +16,7 @@ prompt portions and single decoded tokens of open sequences as one batch.
 from __future__ import annotations
 
 import os
+import struct
 import time
 from dataclasses import dataclass, field
 from typing import Dict, Iterable, List, Optional, Sequence
@@ -91,13 +92,22 @@ def _token_arrays(entries: Sequence[StepEntry], lens: Sequence[int]) -> List[np.
             a = np.array([int(t) for t in tokens], dtype=np.int64)
         return a
 
-    if max(lens) == 1:
-        flat = one([e.tokens[0] for e in entries])
-    else:
-        flat = np.concatenate([one(e.tokens) for e in entries])
-    if flat.size and not -2 ** 31 <= int(flat.min()) <= int(flat.max()) < 2 ** 31:
-        raise ValueError("token ids are 32-bit numbers")
-    flat, out, n = flat.astype(np.int32), [], 0
+    flat, single = None, max(lens) == 1
+    ids = [e.tokens[0] for e in entries] if single else None
+    if single or all(type(e.tokens) is list for e in entries):
+        # lists of whole numbers, a quarter of the time (1024 numbers 14 us); anything else, and numbers of more bits, below
+        try:
+            flat = struct.pack(f"{len(ids)}i", *ids) if single else b"".join(
+                [struct.pack(f"{n}i", *e.tokens) for n, e in zip(lens, entries)])
+            flat = np.frombuffer(flat, dtype=np.int32)
+        except (struct.error, TypeError, ValueError, RuntimeError):
+            flat = None
+    if flat is None:
+        flat = one(ids) if single else np.concatenate([one(e.tokens) for e in entries])
+        if flat.size and not -2 ** 31 <= int(flat.min()) <= int(flat.max()) < 2 ** 31:
+            raise ValueError("token ids are 32-bit numbers")
+        flat = flat.astype(np.int32)
+    out, n = [], 0
     for k in lens:
         out.append(flat[n:n + k])
         n += k
@@ -142,6 +152,7 @@ class GenerationEngine:
         self.ids_host = torch.zeros((B,), dtype=torch.int32, pin_memory=pin)
         self.out_host = torch.zeros((B,), dtype=torch.int32, pin_memory=pin)
         self.active: Dict[int, SequenceState] = {}     # table row -> sequence
+        self._opened: set = set()                      # rows whose length on the device may not be -1
         self._graph = None
         self.step_logits: Optional[torch.Tensor] = None   # logits of the last decode step [max_batch, V] (one rank)
         tp = model.tp
@@ -163,16 +174,18 @@ class GenerationEngine:
     def _to_device(self, *arrays: np.ndarray) -> List[torch.Tensor]:
         """int32 arrays on the device, brought over by one copy from pinned memory (the allocator keeps that until the copy
         is done); each starts on 256 bytes."""
-        starts, n = [], 0
+        sizes, n = [], 0
         for a in arrays:
-            starts.append(n)
-            n += (a.size + 63) // 64 * 64
+            pad = -a.size % 64
+            sizes += (a.size, pad)
+            n += a.size + pad
         host = torch.empty((n,), dtype=torch.int32, pin_memory=self.device.type == "cuda")
-        flat = host.numpy()
-        for a, o in zip(arrays, starts):
-            flat[o:o + a.size] = a.reshape(-1)
-        there = host.to(self.device, non_blocking=True)
-        return [there[o:o + a.size].view(a.shape) for a, o in zip(arrays, starts)]
+        flat, o = host.numpy(), 0
+        for a, k, pad in zip(arrays, sizes[::2], sizes[1::2]):
+            flat[o:o + k] = a.reshape(-1)
+            o += k + pad
+        there = host.to(self.device, non_blocking=True).split(sizes)[::2]
+        return [t if a.ndim == 1 else t.view(a.shape) for a, t in zip(arrays, there)]
 
     def _packed(self, parts: Sequence[tuple], ids: Optional[List[np.ndarray]] = None, want: Optional[List[int]] = None) -> tuple:
         """Run tokens [start, end) of each (sequence, start, end) as one packed batch; returns (final-normed hidden
@@ -183,14 +196,11 @@ class GenerationEngine:
             ids = [np.array(s.tokens[c:n], dtype=np.int32) for s, c, n in parts]
         lens = np.array([n - c for _, c, n in parts], dtype=np.int32)
         ends = np.cumsum(lens, dtype=np.int32)
-        pos = np.concatenate([np.arange(c, n, dtype=np.int32) for _, c, n in parts])
         rows = np.array([s.slot for s, _, _ in parts], dtype=np.int32)
-        table = cache.table_rows(rows)
-        page = np.repeat(np.arange(len(parts)), lens), pos // BLOCK_SIZE
-        ids_d, pos_d, slots_d, qs_d, ql_d, ctx_d, rows_d, want_d, table_d = self._to_device(
-            np.concatenate(ids), pos, table[page] * BLOCK_SIZE + pos % BLOCK_SIZE, ends - lens, lens,
-            np.array([n for _, _, n in parts], dtype=np.int32), rows, ends - 1 if want is None else np.array(want, dtype=np.int32),
-            table)
+        ids_d, qs_d, ql_d, ctx_d, rows_d, want_d, table_d = self._to_device(
+            np.concatenate(ids), ends - lens, lens, np.array([n for _, _, n in parts], dtype=np.int32), rows,
+            ends - 1 if want is None else np.array(want, dtype=np.int32), cache.table_rows(rows))
+        pos_d, slots_d = ops.packed_positions(qs_d, ql_d, ctx_d, table_d, int(ends[-1]), BLOCK_SIZE)
         hidden = m.prefill(ids_d, pos_d, slots_d, cache, table_d, qs_d, ql_d, ctx_d, int(lens.max()), rows=rows_d,
                            spans=[(c, n) for _, c, n in parts])
         return hidden, want_d
@@ -254,6 +264,7 @@ class GenerationEngine:
         ctx_host = self.context_lens.cpu()
         for s in seqs:
             ctx_host[s.slot] = s.num_computed
+            self._opened.add(s.slot)
         self.context_lens.copy_(ctx_host)
         self.ids.copy_(self.ids_host, non_blocking=True)
 
@@ -357,79 +368,90 @@ class GenerationEngine:
         as they are."""
         if len({e.seq.slot for e in entries}) != len(entries):
             raise ValueError("a sequence may have one entry in a step")
-        lens, places, decode = [], [], self.model.tp.world_size == 1
+        lens, places, decode, limit = [], [], self.model.tp.world_size == 1, self.max_seq_len
         for e in entries:
-            n, done, at = len(e.tokens), e.seq.num_computed, [*e.want]
+            n, done, at = len(e.tokens), e.seq.num_computed, e.want
             if not n:
                 raise ValueError("an entry needs at least one token")
-            if done + n > self.max_seq_len:
-                raise RuntimeError(f"sequence would exceed max_seq_len={self.max_seq_len}")
-            if len(at) != 1 or type(at[0]) is not int or not 0 <= at[0] < n:        # anything but one place from the front
-                at = _places(at, n)
+            if done + n > limit:
+                raise RuntimeError(f"sequence would exceed max_seq_len={limit}")
+            # anything but a list of one place from the front
+            if type(at) is not list or len(at) != 1 or type(at[0]) is not int or not 0 <= at[0] < n:
+                at = _places([*at], n)
             if n > 1 or done <= 0:
                 decode = False
             lens.append(n)
             places.append(at)
         if not entries:
             return None
-        news = _token_arrays(entries, lens)        # the entries' tokens themselves may be a sequence's own list, which grows now
+        news = _token_arrays(entries, lens)        # the entries' tokens themselves may be a sequence's own list, which grows below
+        cache, logits = self.cache, None
+        # what the device does not wait for comes behind the launches: the sequences' tokens, and (packed steps bring their own rows)
+        # the device's block table
+        reached = 0
         try:
-            for e, new in zip(entries, news):
+            for e, n in zip(entries, lens):
+                reached += 1
+                if e.seq.num_computed + n > len(e.seq.blocks) * BLOCK_SIZE:
+                    cache.ensure_capacity(e.seq, e.seq.num_computed + n, flush=False)
+            if decode:
+                cache.flush()
+                logits = self._decode_rows(entries, [int(a[0]) for a in news],
+                                           [e.seq.slot for e, at in zip(entries, places) for _ in at])
+            else:
+                # single tokens lie ahead of portions in the batch, where attention takes them together
+                order = sorted(range(len(entries)), key=lambda i: lens[i] > 1)
+                starts, total = [0] * len(entries), 0
+                for i in order:
+                    starts[i] = total
+                    total += lens[i]
+                rows = [starts[i] + w for i, at in enumerate(places) for w in at]
+                parts = [(e.seq, e.seq.num_computed, e.seq.num_computed + n) for e, n in zip(entries, lens)]
+                hidden, want = self._packed([parts[i] for i in order], [news[i] for i in order], rows)
+                if rows:
+                    logits = self.model.logits(hidden.index_select(0, want))
+        finally:
+            cache.flush()
+            for e, new in zip(entries[:reached], news):
                 tokens = e.seq.tokens
                 del tokens[e.seq.num_computed:]
                 tokens.extend(new.tolist())
-                if len(tokens) > len(e.seq.blocks) * BLOCK_SIZE:
-                    self.cache.ensure_capacity(e.seq, len(tokens), flush=False)
-        finally:
-            self.cache.flush()
-        logits = None
-        if decode:
-            logits = self._decode_rows(entries, [e.seq.slot for e, at in zip(entries, places) for _ in at])
-        else:
-            # single tokens lie ahead of portions in the batch, where attention takes them together
-            order = sorted(range(len(entries)), key=lambda i: lens[i] > 1)
-            starts, total = [0] * len(entries), 0
-            for i in order:
-                starts[i] = total
-                total += lens[i]
-            rows = [starts[i] + w for i, at in enumerate(places) for w in at]
-            parts = [(e.seq, e.seq.num_computed, len(e.seq.tokens)) for e in entries]
-            hidden, want = self._packed([parts[i] for i in order], [news[i] for i in order], rows)
-            if rows:
-                logits = self.model.logits(hidden.index_select(0, want))
         for e in entries:
             if decode:
                 e.seq.num_computed += 1
             else:
-                self.cache.mark_computed(e.seq, len(e.seq.tokens))
+                cache.mark_computed(e.seq, len(e.seq.tokens))
         if self.device.type == "cuda":
             # the block table and the step's inputs are copied from pinned memory that the next step or release may rewrite
             torch.cuda.current_stream().synchronize()
         return logits
 
-    def _decode_rows(self, entries: Sequence[StepEntry], rows: Sequence[int]) -> Optional[torch.Tensor]:
-        """A decode step of the rows in `entries` only; the other rows are inactive in it.  Returns the logits of `rows`."""
+    def _decode_rows(self, entries: Sequence[StepEntry], tokens: Sequence[int], rows: Sequence[int]) -> Optional[torch.Tensor]:
+        """A decode step of the rows in `entries` only, by their new tokens; the other rows are inactive in it.  Returns the logits of
+        `rows`."""
         self._ensure_graph()
         B, pitch = self.max_batch, self._pitch
         inputs = torch.empty((3 * pitch,), dtype=torch.int32, pin_memory=self.device.type == "cuda")
         host = inputs.numpy()
         ids, ctx = self.ids_host.numpy(), host[pitch:pitch + B]
-        slots = np.array([e.seq.slot for e in entries])
+        slots = [e.seq.slot for e in entries]
         ctx.fill(-1)
         ctx[slots] = [e.seq.num_computed for e in entries]
-        ids[slots] = [e.seq.tokens[-1] for e in entries]
+        ids[slots] = tokens
         wanted = len(rows)
         host[:B] = ids
         if wanted <= pitch:
             host[2 * pitch:2 * pitch + wanted] = rows
         self._inputs.copy_(inputs, non_blocking=True)
         self.decode_step_device()
+        self._opened.update(slots)
         logits = None
         if wanted:
             at = self._inputs[2 * pitch:2 * pitch + wanted] if wanted <= pitch else self._to_device(np.array(rows, dtype=np.int32))[0]
             logits = self.step_logits.index_select(0, at)
         if len(entries) < len(self.active):
             # the rows that were left out become active again; the others have been counted on by the step
+            self._opened.update(self.active)
             full = np.full((B,), -1, dtype=np.int32)
             for s in self.active.values():
                 full[s.slot] = s.num_computed
@@ -480,13 +502,14 @@ class GenerationEngine:
         seqs = list(seqs)
         if not seqs:
             return
-        # runs of neighbouring rows
-        slots = sorted(s.slot for s in seqs)
+        # runs of neighbouring rows, of those that decode steps have given a length
+        slots = sorted({s.slot for s in seqs} & self._opened)
         first = 0
         for i in range(1, len(slots) + 1):
             if i == len(slots) or slots[i] != slots[i - 1] + 1:
                 self.context_lens[slots[first]:slots[i - 1] + 1].fill_(-1)
                 first = i
+        self._opened.difference_update(slots)
         if self.device.type == "cuda":
             # steps in flight still read the blocks and table rows that are given back here
             torch.cuda.current_stream().synchronize()

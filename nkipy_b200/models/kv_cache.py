@@ -132,6 +132,13 @@ class BlockAllocator:
     def extend(self, blocks: List[int], new_len: int) -> int:
         """Grow a block list to cover new_len tokens; returns the number of blocks added."""
         need = (new_len + self.block_size - 1) // self.block_size - len(blocks)
+        if 0 < need <= len(self.free):           # one by one from the end
+            taken = self.free[:-need - 1:-1]
+            del self.free[-need:]
+            for b in taken:
+                self.ref[b] = 1
+            blocks += taken
+            return need
         for _ in range(max(need, 0)):
             blocks.append(self._take())
         return max(need, 0)

@@ -30,7 +30,7 @@ from ._lib import KernelLibraryError, device_status, raise_on_device_error
 
 __all__ = [
     "linear", "decode_linear", "qkv_rope_append", "reduce_partials", "rmsnorm", "add_rmsnorm", "silu_mul", "embedding", "rope_kv_append",
-    "argmax", "sample", "decode_advance", "router_topk", "moe_dispatch", "grouped_linear", "moe_combine", "paged_attn_decode", "flash_attn_prefill", "packed_attention", "leading_singles", "pick_splits", "rope_table",
+    "argmax", "sample", "decode_advance", "packed_positions", "router_topk", "moe_dispatch", "grouped_linear", "moe_combine", "paged_attn_decode", "flash_attn_prefill", "packed_attention", "leading_singles", "pick_splits", "rope_table",
     "Branch", "MapsSpec", "Norm", "Proj", "activation", "gate_heads", "gated_act", "gated_residual", "hgrn2", "maps_append",
     "heads_attention", "maps_attention", "row_norm_append", "rope_norm_append", "head_linear", "softcap",
     "LatentSpec", "latent_append", "latent_attention", "latent_gather", "latent_prefill", "latent_queries",
@@ -728,6 +728,27 @@ def decode_advance(context_lens: torch.Tensor, block_table: torch.Tensor, positi
                                        slots.data_ptr(), B, q_len, block_table.stride(0), block_size, _stream())
     _lib.check(rc, "nkb_decode_advance")
     _launches += 2
+
+
+def packed_positions(q_start: torch.Tensor, q_lens: torch.Tensor, context_lens: torch.Tensor, block_table: torch.Tensor, tokens: int,
+                     block_size: int = 32) -> tuple:
+    """(positions, cache slots), int32 [tokens], of the tokens of a packed step: sequence b's q_lens[b] new tokens, in rows q_start[b]
+    on, are the last of its context_lens[b]; its blocks are row b of the table.  The sequences follow one another without gaps."""
+    positions = torch.empty((tokens,), dtype=torch.int32, device=q_start.device)
+    slots = torch.empty_like(positions)
+    if not _native(positions):
+        lens = q_lens.long()
+        seq = torch.repeat_interleave(torch.arange(len(lens)), lens)
+        pos = torch.arange(tokens) - q_start.long()[seq] + (context_lens.long() - lens)[seq]
+        positions.copy_(pos)
+        slots.copy_(block_table.long()[seq, pos // block_size] * block_size + pos % block_size)
+        return positions, slots
+    rc = _lib.lib().nkb_packed_positions(q_start.data_ptr(), q_lens.data_ptr(), context_lens.data_ptr(), block_table.data_ptr(),
+                                         positions.data_ptr(), slots.data_ptr(), q_start.shape[0], tokens, block_table.stride(0),
+                                         block_size, _stream())
+    _lib.check(rc, "nkb_packed_positions")
+    _count_launch()
+    return positions, slots
 
 
 # --------------------------------------------------------------------------- sampling / routing

@@ -191,6 +191,7 @@ _SIGNATURES = {
          c_int, _P],
     ),
     "nkb_decode_advance": (c_int, [_P, _P, _P, _P, c_int, c_int, c_int, c_int, _P]),
+    "nkb_packed_positions": (c_int, [_P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, _P]),
     "nkb_argmax": (c_int, [_P, c_int, _P, _P, c_int, c_int, c_longlong, _P]),
     "nkb_sample": (c_int, [_P, c_int, _P, c_int, c_int, c_longlong, c_float, c_int, c_float, c_ulonglong,
                            c_ulonglong, _P]),

@@ -1,7 +1,9 @@
 """Steps of an external scheduler: single tokens and portions in any order give what they give alone."""
+import numpy as np
 import pytest
 import torch
 
+from nkipy_b200 import ops
 from nkipy_b200.models import config as C
 from nkipy_b200.models.engine import GenerationEngine, StepEntry
 from nkipy_b200.models.kv_cache import BLOCK_SIZE, OutOfBlocks
@@ -130,3 +132,38 @@ def test_release_takes_any_iterable(device):
     e.release(e.active.values())
     e.release(iter(()))
     assert not e.active and e.context_lens.tolist() == [-1] * 6
+
+
+@pytest.mark.parametrize("device", DEVICES)
+@pytest.mark.parametrize("lens", [[1], [129], [1, 1, 1], [31, 33, 1, 64, 5], [1] * 70 + [300]])
+def test_positions_of_packed_tokens(device, lens):
+    """Positions and slots as counted out one by one, for new sequences and continued ones."""
+    done = [(37 * i) % 90 for i in range(len(lens))]
+    ends = [d + n for d, n in zip(done, lens)]
+    table = torch.randperm(len(lens) * 13, generator=torch.Generator().manual_seed(1)).reshape(len(lens), 13)
+    i32 = lambda x: torch.as_tensor(x, dtype=torch.int32).to(device)
+    pos, slots = ops.packed_positions(i32([sum(lens[:i]) for i in range(len(lens))]), i32(lens), i32(ends), i32(table), sum(lens))
+    want = [(b, p) for b, (d, e) in enumerate(zip(done, ends)) for p in range(d, e)]
+    assert pos.tolist() == [p for _, p in want]
+    assert slots.tolist() == [int(table[b, p // BLOCK_SIZE]) * BLOCK_SIZE + p % BLOCK_SIZE for b, p in want]
+
+
+def test_token_ids_of_all_kinds():
+    """Lists, tuples, arrays and tensors, of whole numbers and of what stands for them, alone and beside one another."""
+    e = engine("cpu")
+    p = ids(5, 3)
+    kinds = [p, tuple(p), np.array(p), np.array(p, dtype=np.uint8) if max(p) < 256 else np.array(p, dtype=np.int64), torch.tensor(p),
+             [float(t) for t in p], [np.int64(t) for t in p], [torch.tensor(t) for t in p]]
+    got = []
+    for k in kinds:
+        s = e.open_request()
+        got.append(e.run_step([StepEntry(s, k, [4])]))
+        assert s.tokens == p and all(type(t) is int for t in s.tokens)
+        e.release([s])
+    assert all(torch.equal(g, got[0]) for g in got)
+    a, b = e.open_request(), e.open_request()
+    assert torch.equal(e.run_step([StepEntry(a, kinds[0], [4]), StepEntry(b, kinds[4], [4])]), torch.cat([got[0]] * 2))
+    for bad in ([2 ** 31], [-2 ** 31 - 1], [1, 2 ** 40]):
+        with pytest.raises(ValueError):
+            e.run_step([StepEntry(a, bad, [0])])
+    assert a.num_computed == 5 and e.run_step([StepEntry(a, [np.int32(3)], [0])]).shape[0] == 1
