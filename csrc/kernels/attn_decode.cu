@@ -4,7 +4,7 @@
 // fill a wave, among which the pages of all its sequences are divided (`plan_pages`).  The query rows of a CTA are the
 // q_len new tokens x the GQA group of this kv head (at most 16 rows), held as
 // MMA A-fragments in registers for the whole kernel.  Each of its one, two or four warps
-// walks its own subset of 32-token KV pages: the page is fetched with TMA
+// walks its own subset of 32-token KV pages (further warps help before and after, `dec_helpers`): the page is fetched with TMA
 // (128-byte swizzle, through the per-sequence block table) into a private
 // 3-stage shared-memory ring, scores and P*V run on the tensor cores with
 // m16n8k16 fragments fed by ldmatrix, and the online-softmax state stays in
@@ -70,70 +70,88 @@ struct DecodeParams {
   __nv_bfloat16* v_cache;
   float norm_eps;
   int qkv_splits, max_pos;
+  int qkv_pairs;             // partials may be read two at a time
   NkbScoreMods mods;         // MODS only (not fused)
 };
 
-// One head row of the fused QKV output for token `tok`, in two steps so that a warp can have the loads of two
-// heads in flight at once: `load` issues every global read the row needs (the partials of up to kFuseChunk splits,
-// bias, norm weight, the cos / sin row), `finish` sums, normalises, rotates and rounds to bf16 the way the
-// stand-alone RoPE kernel does.  One warp; lane owns elements lane * PER + j of each half.
-constexpr int kFuseChunk = 8;
+// Rows of the fused QKV output of one token, two heads at a time, in two steps so that a warp has the loads of all of them in flight:
+// `load` issues every global read the rows need (the partials of up to C splits, bias), `finish` sums, normalises, rotates and rounds
+// to bf16 the way the stand-alone RoPE kernel does.  One warp; lane owns elements lane * PER + j of each half.  What all heads of a
+// kind share (cos / sin, norm weights) is loaded once, by `FusedShared`.
 template <int D>
-struct FusedRow {
+struct FusedShared {
   static constexpr int PER = D / 64;
-  float x[kFuseChunk][PER], y[kFuseChunk][PER];
-  float bx[PER], by[PER], wx[PER], wy[PER], c[PER], sn[PER];
-  long long base;
-  bool has_norm, rotate;
+  float c[PER], sn[PER], wq[2][PER], wk[2][PER];
 
-  __device__ __forceinline__ void load(const DecodeParams& p, int tok, int head, const __nv_bfloat16* norm_w,
-                                       bool rot, int lane) {
-    const int width = (p.nq + 2 * p.nkv) * D;
-    base = (long long)tok * width + (long long)head * D + lane * PER;
-    has_norm = norm_w != nullptr;
-    rotate = rot && p.cos_sin != nullptr;
-    int pos = rotate ? p.positions[tok] : 0;
-#pragma unroll
-    for (int q = 0; q < kFuseChunk; ++q) {
-      const bool on = q < p.qkv_splits;
-      const float* src = p.qkv_partials + (long long)q * p.qkv_split_stride + base;
-#pragma unroll
-      for (int j = 0; j < PER; ++j) {
-        x[q][j] = on ? __ldcg(src + j) : 0.f;
-        y[q][j] = on ? __ldcg(src + D / 2 + j) : 0.f;
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < PER; ++j) {
-      const int i = lane * PER + j;
-      bx[j] = p.qkv_bias ? __bfloat162float(p.qkv_bias[head * D + i]) : 0.f;
-      by[j] = p.qkv_bias ? __bfloat162float(p.qkv_bias[head * D + D / 2 + i]) : 0.f;
-      wx[j] = has_norm ? __bfloat162float(norm_w[i]) : 1.f;
-      wy[j] = has_norm ? __bfloat162float(norm_w[D / 2 + i]) : 1.f;
-    }
+  __device__ __forceinline__ void load(const DecodeParams& p, int pos, int lane) {
     pos = pos < 0 ? 0 : (pos >= p.max_pos ? p.max_pos - 1 : pos);
 #pragma unroll
     for (int j = 0; j < PER; ++j) {
       const int i = lane * PER + j;
-      c[j] = rotate ? p.cos_sin[(long long)pos * D + i] : 1.f;
-      sn[j] = rotate ? p.cos_sin[(long long)pos * D + D / 2 + i] : 0.f;
+      c[j] = p.cos_sin ? p.cos_sin[(long long)pos * D + i] : 1.f;
+      sn[j] = p.cos_sin ? p.cos_sin[(long long)pos * D + D / 2 + i] : 0.f;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        wq[h][j] = p.q_norm_w ? __bfloat162float(p.q_norm_w[h * (D / 2) + i]) : 1.f;
+        wk[h][j] = p.k_norm_w ? __bfloat162float(p.k_norm_w[h * (D / 2) + i]) : 1.f;
+      }
+    }
+  }
+};
+// The code runs once per CTA, so its instructions come from memory: two rows and eight splits a time keep it small (four rows of four
+// splits and two forms of loads: 29.0 us instead of 26.6 for the three kernels around one sequence of 203 tokens).
+template <int D>
+struct FusedRows {
+  static constexpr int PER = D / 64, R = 2, C = 8;
+  float x[R][C][2][PER], b[R][2][PER];
+  long long base[R];
+
+  // head[r] < 0: none
+  __device__ __forceinline__ void load(const DecodeParams& p, int tok, const int (&head)[R], int lane) {
+    const int width = (p.nq + 2 * p.nkv) * D;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      base[r] = (long long)tok * width + (long long)max(head[r], 0) * D + lane * PER;
+      const int ahead = head[r] >= 0 && p.qkv_pairs ? p.qkv_splits : 0;
+#pragma unroll
+      for (int q = 0; q < C; ++q) {
+        const float* src = p.qkv_partials + (long long)q * p.qkv_split_stride + base[r];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          if constexpr (PER == 2) {
+            const float2 v = q < ahead ? __ldcg(reinterpret_cast<const float2*>(src + h * (D / 2))) : make_float2(0.f, 0.f);
+            x[r][q][h][0] = v.x;
+            x[r][q][h][1] = v.y;
+          } else {
+            x[r][q][h][0] = q < ahead ? __ldcg(src + h * (D / 2)) : 0.f;
+          }
+        }
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int j = 0; j < PER; ++j)
+          b[r][h][j] = p.qkv_bias && head[r] >= 0 ? __bfloat162float(p.qkv_bias[head[r] * D + h * (D / 2) + lane * PER + j]) : 0.f;
     }
   }
 
-  __device__ __forceinline__ void finish(const DecodeParams& p, float (&lo)[PER], float (&hi)[PER]) {
+  // row r as a query (norm weights w) or key, or (rotate false, norm false) a value
+  __device__ __forceinline__ void finish(const DecodeParams& p, const FusedShared<D>& s, int r, const float (&w)[2][PER], bool norm,
+                                         bool rotate, float (&lo)[PER], float (&hi)[PER]) {
 #pragma unroll
     for (int j = 0; j < PER; ++j) lo[j] = hi[j] = 0.f;
 #pragma unroll
-    for (int q = 0; q < kFuseChunk; ++q) {
+    for (int q = 0; q < C; ++q) {
 #pragma unroll
       for (int j = 0; j < PER; ++j) {
-        lo[j] += x[q][j];
-        hi[j] += y[q][j];
+        lo[j] += x[r][q][0][j];
+        hi[j] += x[r][q][1][j];
       }
     }
-    // more splits than one chunk holds (rare): the rest in order, without the overlap
-    for (int q = kFuseChunk; q < p.qkv_splits; ++q) {
-      const float* src = p.qkv_partials + (long long)q * p.qkv_split_stride + base;
+    // more splits than one chunk holds (rare) and partials that do not lie in pairs: in order, without the overlap
+#pragma unroll 1
+    for (int q = p.qkv_pairs ? C : 0; q < p.qkv_splits; ++q) {
+      const float* src = p.qkv_partials + (long long)q * p.qkv_split_stride + base[r];
 #pragma unroll
       for (int j = 0; j < PER; ++j) {
         lo[j] += __ldcg(src + j);
@@ -142,10 +160,10 @@ struct FusedRow {
     }
 #pragma unroll
     for (int j = 0; j < PER; ++j) {
-      lo[j] += bx[j];
-      hi[j] += by[j];
+      lo[j] += b[r][0][j];
+      hi[j] += b[r][1][j];
     }
-    if (has_norm) {
+    if (norm) {
       float ss = 0.f;
 #pragma unroll
       for (int j = 0; j < PER; ++j) ss += lo[j] * lo[j] + hi[j] * hi[j];
@@ -153,16 +171,16 @@ struct FusedRow {
       const float inv = rsqrtf(ss / float(D) + p.norm_eps);
 #pragma unroll
       for (int j = 0; j < PER; ++j) {
-        lo[j] = __bfloat162float(__float2bfloat16(lo[j] * inv * wx[j]));
-        hi[j] = __bfloat162float(__float2bfloat16(hi[j] * inv * wy[j]));
+        lo[j] = __bfloat162float(__float2bfloat16(lo[j] * inv * w[0][j]));
+        hi[j] = __bfloat162float(__float2bfloat16(hi[j] * inv * w[1][j]));
       }
     }
-    if (rotate) {
+    if (rotate && p.cos_sin) {
 #pragma unroll
       for (int j = 0; j < PER; ++j) {
-        const float a = lo[j], b = hi[j];
-        lo[j] = a * c[j] - b * sn[j];
-        hi[j] = b * c[j] + a * sn[j];
+        const float u = lo[j], v = hi[j];
+        lo[j] = u * s.c[j] - v * s.sn[j];
+        hi[j] = v * s.c[j] + u * s.sn[j];
       }
     }
 #pragma unroll
@@ -251,11 +269,20 @@ __device__ __forceinline__ bool plan_pages(const DecodeParams& p, int unit, int 
   return false;
 }
 
+// Warps of a CTA beside those that stream pages: they take their share of the new token's rows (fused mode) and of the merge, for which
+// a single warp takes its time.  As many as the registers leave room for beside the rings of four warps per SM (heads of 64 columns:
+// eight).  QKV product, attention and output product of a layer one behind another, before and so, us: 128 sequences of 512, 32 heads on 4,
+// 68.0 -> 60.2; 64 of 1024, 32 on 8, 79.3 -> 74.8; 68 of 76 45.4 -> 40.6; 7 of 3500 to 7000 52.7 -> 51.5; one of 203 26.6 -> 24.1; one of
+// 128, 64 heads of 64 on 8, 21.9 -> 19.4.
+template <int D, int kDecWarps>
+__host__ __device__ constexpr int dec_helpers() { return kDecWarps == 1 && D == 128 ? 2 : kDecWarps; }
+
 template <int D, int kDecWarps, bool MODS>
-__global__ void __launch_bounds__(kDecWarps * 32)
+__global__ void __launch_bounds__((kDecWarps + dec_helpers<D, kDecWarps>()) * 32, 512 / D / kDecWarps)
 paged_attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                          const DecodeParams p) {
   constexpr int NH = D / 64;                 // 128-byte halves per row
+  constexpr int kAllWarps = kDecWarps + dec_helpers<D, kDecWarps>();
   constexpr int kHalfBytes = kPage * 128;    // one [32 x 64] swizzled slab
   constexpr int kMatBytes = NH * kHalfBytes; // K (or V) page
   constexpr int kStageBytes = 2 * kMatBytes;
@@ -304,7 +331,7 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
   for (int i = 0; i < D / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
   float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
 
-  uint8_t* my_smem = smem + warp * kDecStages * kStageBytes;
+  uint8_t* my_smem = smem + min(warp, kDecWarps - 1) * kDecStages * kStageBytes;
   auto issue = [&](int blk, int stage) {
     if (lane == 0) {
       uint8_t* dst = my_smem + stage * kStageBytes;
@@ -318,7 +345,8 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
   };
 
   // ---- prologue
-  const int my_first = p0 + warp;
+  const int new_pos = fused && p.cos_sin ? p.positions[b] : 0;
+  const int my_first = warp < kDecWarps ? p0 + warp : p1;       // helpers stream nothing
   int blks[kDecStages];
 #pragma unroll
   for (int s = 0; s < kDecStages; ++s) {
@@ -334,7 +362,7 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
   if (fused) {
     constexpr int PER = D / 64;
     // heads of this CTA: the group's queries, then (owner only) the key and the value of this kv head; a warp
-    // takes two of them per round so that both rows' loads are in flight together
+    // takes several of them per round so that all their loads are in flight together
     const int nheads = p.group + (owner ? 2 : 0);
     const int slot = p.slots ? p.slots[b] : -1;
     auto head_of = [&](int hh) { return hh < p.group ? kvh * p.group + hh : (hh == p.group ? p.nq + kvh : p.nq + p.nkv + kvh); };
@@ -365,24 +393,30 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
         }
       }
     };
-    for (int h0 = warp; h0 < nheads; h0 += 2 * kDecWarps) {
-      const int h1 = h0 + kDecWarps;
-      FusedRow<D> ra, rb;
-      float lo[PER], hi[PER];
-      ra.load(p, b, head_of(h0), h0 < p.group ? p.q_norm_w : (h0 == p.group ? p.k_norm_w : nullptr), h0 <= p.group, lane);
-      if (h1 < nheads)
-        rb.load(p, b, head_of(h1), h1 < p.group ? p.q_norm_w : (h1 == p.group ? p.k_norm_w : nullptr), h1 <= p.group, lane);
-      ra.finish(p, lo, hi);
-      store(h0, lo, hi);
-      if (h1 < nheads) {
-        rb.finish(p, lo, hi);
-        store(h1, lo, hi);
+    FusedShared<D> shared;
+    constexpr int R = FusedRows<D>::R;
+#pragma unroll 1
+    for (int h0 = warp; h0 < nheads; h0 += R * kAllWarps) {
+      FusedRows<D> rows;
+      int head[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) head[r] = h0 + r * kAllWarps < nheads ? head_of(h0 + r * kAllWarps) : -1;
+      if (h0 == warp) shared.load(p, new_pos, lane);
+      rows.load(p, b, head, lane);
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const int hh = h0 + r * kAllWarps;
+        if (hh >= nheads) break;
+        float lo[PER], hi[PER];
+        const bool is_q = hh < p.group, is_k = hh == p.group;
+        rows.finish(p, shared, r, is_q ? shared.wq : shared.wk, (is_q && p.q_norm_w) || (is_k && p.k_norm_w), is_q || is_k, lo, hi);
+        store(hh, lo, hi);
       }
     }
     __syncthreads();
     if (owner) {
       // scores of the new token against the group's queries (log2 domain like the paged part)
-      for (int r = warp; r < p.group; r += kDecWarps) {
+      for (int r = warp; r < p.group; r += kAllWarps) {
         float acc = 0.f;
         for (int i = lane; i < D; i += 32) acc += __bfloat162float(q_s[r * D + i]) * kn_s[i];
         acc = warp_sum(acc);
@@ -546,14 +580,16 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
   float* mo = reinterpret_cast<float*>(smem);             // [warp][16][D]
   float* mm = mo + kDecWarps * 16 * D;                    // [warp][16]
   float* ml = mm + kDecWarps * 16;                        // [warp][16]
+  if (warp < kDecWarps) {
 #pragma unroll
-  for (int i = 0; i < D / 8; ++i) {
-    float* r0 = mo + (warp * 16 + g) * D + i * 8 + 2 * t;
-    float* r1 = mo + (warp * 16 + g + 8) * D + i * 8 + 2 * t;
-    r0[0] = o[i][0]; r0[1] = o[i][1];
-    r1[0] = o[i][2]; r1[1] = o[i][3];
+    for (int i = 0; i < D / 8; ++i) {
+      float* r0 = mo + (warp * 16 + g) * D + i * 8 + 2 * t;
+      float* r1 = mo + (warp * 16 + g + 8) * D + i * 8 + 2 * t;
+      r0[0] = o[i][0]; r0[1] = o[i][1];
+      r1[0] = o[i][2]; r1[1] = o[i][3];
+    }
   }
-  if (t == 0) {
+  if (t == 0 && warp < kDecWarps) {
     mm[warp * 16 + g] = m0; mm[warp * 16 + g + 8] = m1;
     ml[warp * 16 + g] = l0; ml[warp * 16 + g + 8] = l1;
   }
@@ -680,7 +716,8 @@ static int launch_decode(const CUtensorMap& tk, const CUtensorMap& tv, const Dec
     attr_set[dev] = true;
   }
   const dim3 grid = p.units ? dim3(p.units, p.nkv, 1) : dim3(1, p.nkv, p.batch);
-  return launch_pdl(paged_attn_decode_kernel<D, kDecWarps, MODS>, grid, dim3(kDecWarps * 32), size_t(smem), s, tk, tv, p);
+  return launch_pdl(paged_attn_decode_kernel<D, kDecWarps, MODS>, grid, dim3((kDecWarps + dec_helpers<D, kDecWarps>()) * 32), size_t(smem),
+                    s, tk, tv, p);
 }
 
 // Units of the page plan: num_splits per sequence, rounded up to one wave of one CTA per SM, or of two (the scratch, which is sized for nq
@@ -797,6 +834,7 @@ extern "C" int nkb_paged_attn_decode_fused(const float* qkv_partials, int qkv_sp
   p.qkv_partials = qkv_partials;
   p.qkv_split_stride = qkv_split_stride;
   p.qkv_splits = qkv_splits;
+  p.qkv_pairs = head_dim == 64 || ((reinterpret_cast<uintptr_t>(qkv_partials) & 7) == 0 && (qkv_split_stride & 1) == 0);
   p.qkv_bias = reinterpret_cast<const __nv_bfloat16*>(qkv_bias);
   p.positions = positions;
   p.slots = slots;
