@@ -332,14 +332,15 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
   float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
 
   uint8_t* my_smem = smem + min(warp, kDecWarps - 1) * kDecStages * kStageBytes;
+  const uint64_t policy = l2_evict_first();
   auto issue = [&](int blk, int stage) {
     if (lane == 0) {
       uint8_t* dst = my_smem + stage * kStageBytes;
       mbar_expect_tx(&bars[warp][stage], kStageBytes);
 #pragma unroll
       for (int h = 0; h < NH; ++h) {
-        tma_load_4d(dst + h * kHalfBytes, &tmK, &bars[warp][stage], h * 64, 0, kvh, blk);
-        tma_load_4d(dst + kMatBytes + h * kHalfBytes, &tmV, &bars[warp][stage], h * 64, 0, kvh, blk);
+        tma_load_4d_once(dst + h * kHalfBytes, &tmK, &bars[warp][stage], h * 64, 0, kvh, blk, policy);
+        tma_load_4d_once(dst + kMatBytes + h * kHalfBytes, &tmV, &bars[warp][stage], h * 64, 0, kvh, blk, policy);
       }
     }
   };
