@@ -31,5 +31,6 @@ struct NkbHeadRec {
   int taps, channels, q_col, k_col, v_col, gate_act, bf16;
   int batch, tokens, heads, groups, dim, vdim;
   float q_scale, eps, unit_eps;
+  float* conv_out;          // step: room for the convolved channels [batch, channels] (a launch of their own), or null
   int longest;              // scan: most new tokens of a sequence, 0 where the caller does not know
 };

@@ -70,7 +70,8 @@ class HeadRecArg(ctypes.Structure):
                [(n, c_void_p) for n in ("conv_w", "conv_b", "conv_state", "rate", "dt_bias", "skip", "norm_w", "state", "slot_ids",
                                         "q_start", "q_lens", "context_lens", "out")] + \
                [(n, c_int) for n in ("taps", "channels", "q_col", "k_col", "v_col", "gate_act", "bf16", "batch", "tokens", "heads",
-                                     "groups", "dim", "vdim")] + [(n, c_float) for n in ("q_scale", "eps", "unit_eps")] + [("longest", c_int)]
+                                     "groups", "dim", "vdim")] + [(n, c_float) for n in ("q_scale", "eps", "unit_eps")] + \
+               [("conv_out", c_void_p), ("longest", c_int)]
 
 
 class TanhNormArg(ctypes.Structure):

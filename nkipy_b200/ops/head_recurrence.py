@@ -22,6 +22,8 @@ from .linear_attention import linear_state_shape
 from .mixers import ACTIVATIONS, Proj, _ref, gate_heads
 
 UNIT_EPS = 1e-6
+# heads of all sequences from which a decode step convolves its channels in a launch of its own (head_recurrence.cu has both times)
+STEP_CONV_APART = 512
 
 
 @dataclass
@@ -197,8 +199,10 @@ def head_recurrence(r: HeadRecurrence, x: Proj, conv: ShortConv, a: Proj, b: Opt
         arg.x, arg.g, arg.conv_w, arg.conv_b = x.arg(), gate.arg(), conv.w.data_ptr(), _ptr(conv.bias)
         arg.conv_state, arg.taps, arg.channels = conv_state.data_ptr(), conv.taps, x.width
         arg.norm_w, arg.out = None if parts else norm_w.data_ptr(), out.data_ptr()
+        apart = torch.empty((T, x.width), dtype=torch.float32, device=state.device) if T * r.heads >= STEP_CONV_APART else None
+        arg.conv_out = _ptr(apart)
         _lib.check(L.nkb_head_rec_step(ctypes.byref(arg), _stream()), "nkb_head_rec_step")
-        _count_launch()
+        _count_launch(1 if apart is None else 2)
         return gated_group_norm(out, gate, gate_act, norm_w, parts, r.eps, dtype) if parts else out
     y = short_conv(x, conv, conv_state, context_lens, q_start, q_lens, rows, dtype=dtype)
     out = torch.empty((T, inner), dtype=dtype, device=state.device)

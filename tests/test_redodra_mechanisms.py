@@ -475,6 +475,31 @@ def test_state_space_mixer(device, dtype, H, G, N, n, taps, parts, decay, plan):
     assert (state[[1, 3]] == 1e3).all() and (ring[[1, 3]] == 1e3).all()
 
 
+@pytest.mark.gpu
+@in_dtypes
+@pytest.mark.parametrize("H,d,n,taps", [(16, 128, 128, 4), (8, 40, 24, 1), (12, 64, 136, 8), (6, 33, 7, 3)])
+@pytest.mark.parametrize("delta", [True, False])
+def test_steps_of_many_heads(dtype, H, d, n, taps, delta, monkeypatch):
+    """A step whose channels are convolved in a launch of their own gives the bits of one that convolves them itself: outputs, states and
+    kept inputs, at a sequence's first tokens, with inactive rows, and where sixteen bytes do not fit."""
+    from nkipy_b200.ops import head_recurrence as hr
+    device, B, C, D = "cuda", 40, 2 * H * d + H * n, lambda t: t.cuda()
+    rec = HeadRecurrence(H, H, d, n, 0, H * d, 2 * H * d, D(torch.rand(H)), D(rnd(H, seed=2)), delta=delta, q_scale=d ** -0.5,
+                         skip=None if delta else D(rnd(H, seed=3)))
+    conv = ShortConv(D(rnd(taps, C, seed=4)), D(rnd(C, seed=5)))
+    P = lambda w, s: Proj(D(torch.stack([rnd(B, w, seed=s), rnd(B, w, seed=s + 1)])), 0, w)
+    x, a, b, g = P(C, 10), P(H, 12), P(H, 14) if delta else None, P(H * n, 16)
+    ctx = [(1, 2, 3, -1, 9, 40)[i % 6] for i in range(B)]
+    norm, got = D(rnd(n if delta else H * n, seed=6)), []
+    for limit in (1, 1 << 30):
+        monkeypatch.setattr(sys.modules[hr.__module__], "STEP_CONV_APART", limit)
+        state, ring = D(rnd(B, *rec.state_shape, seed=7)), D(rnd(B, taps, C, seed=8))
+        out = hr(rec, x, conv, a, b, g, norm, state, ring, i32(ctx, device), parts=0 if delta else 1, dtype=dtype)
+        got.append((out, state, ring))
+    ops.raise_on_device_error()
+    assert all(torch.equal(u, v) for u, v in zip(*got))
+
+
 @on_devices
 @in_dtypes
 def test_a_write_survives_hundreds_of_tokens(device, dtype):
