@@ -8,6 +8,13 @@ namespace nkb {
 // ---------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------
+static bool bulk_stores() {
+  // measured slower than plain stores for these 16-column chunks (sixteen 512-byte copies per chunk keep the
+  // copy engine busy for 1.7 us): opt-in only
+  static const bool on = getenv("NKIPY_B200_BULK_EPILOGUE") != nullptr;
+  return on;
+}
+
 // ctas_per_sm = 2 caps the ring so that two CTAs (of this or of the next GEMM in
 // the stream, started early by programmatic dependent launch) fit on one SM: the
 // successor then prefetches its weight tiles while this kernel drains.
@@ -15,12 +22,16 @@ template <int BN, int MINB, bool PUSH, bool GROUPED>
 static int ring_stages(const GemmArgs& args, int& smem, bool lean = false) {
   const int a_tiles = args.gated == 1 ? 2 : 1, b_tiles = args.gated == 2 ? 2 : 1;
   const int stage_bytes = a_tiles * kATileBytes + b_tiles * BN * kBlockK * 2;
-  // control block + staging: the push tile (32 tokens x 128 features bf16), or the compact epilogue's two
-  // 16-column buffers of fp32
-  const int extra = 512 + (PUSH ? 32 * kTileRows * 2 : (lean ? 2 * 16 * kTileRows * 4 : 0));
+  // control block + staging: the push tile (32 tokens x 128 features bf16), or two 16-column buffers of fp32 where the compact epilogue
+  // stores by bulk copies
+  const int extra = 512 + (PUSH ? 32 * kTileRows * 2 : (lean && bulk_stores() ? 2 * 16 * kTileRows * 4 : 0));
   const int budget = (MINB == 2 ? 113 * 1024 : 232448) - 1024 - extra - 64;
   int stages = budget / stage_bytes;
   if (stages > kMaxStages) stages = kMaxStages;
+  // A stage more pays for wide operands (us of products with two CTAs per SM, three stages instead of two at 128 tokens: 14336 -> 4096 31.7 ->
+  // 25.2, 4096 -> 128256 229 -> 188; four instead of three at 64: 25.2 -> 22.6 and 174 -> 171), but at 32 the fifth gained nothing and the
+  // steps of one sequence lost by it (four GPT-OSS layers 562 -> 574).
+  if (lean && BN == 32) stages = stages < (MINB == 2 ? 4 : 5) ? stages : (MINB == 2 ? 4 : 5);
   static_assert(sizeof(GemmCtrl) <= 512, "control block grew");
   smem = stages * stage_bytes + 1024 + extra + 64;
   return stages;
@@ -35,10 +46,7 @@ static bool lean_ok(const GemmArgs& a) {
 // transpose_out = 2 tells the compact epilogue that every token row of the output may go out as one bulk
 // copy: base, leading dimension, split stride and row count all on 16-byte boundaries.
 void mark_bulk(GemmArgs& a) {
-  // measured slower than plain stores for these 16-column chunks (sixteen 512-byte copies per chunk keep the
-  // copy engine busy for 1.7 us): opt-in only
-  static const bool on = getenv("NKIPY_B200_BULK_EPILOGUE") != nullptr;
-  if (!a.transpose_out || !on) return;
+  if (!a.transpose_out || !bulk_stores()) return;
   const long long esz = (a.out_fp32 && !a.gated) ? 4 : 2;
   const bool ok = (reinterpret_cast<uintptr_t>(a.out) % 16 == 0) && (a.ldo * esz) % 16 == 0 &&
                   (a.rows * esz) % 16 == 0 && (a.split_stride * 4) % 16 == 0;
