@@ -13,8 +13,8 @@
 // chunks' barriers.  The state-space form has u = dt v and neither A nor S^T k.
 //
 // 32-bit numbers enter products as three bf16 parts (24 bits, taken off by truncation, so exact): with bf16 keys and queries
-// three part products are exact; of two 32-bit numbers those below 2^-32 (state) or 2^-24 (the 16 x 16 matrices, entries of at
-// most about one) are left out.  Tensor cores cut off a sum's last bits where fp32 units round: no chain is longer than two steps
+// three part products are exact; of the nine of two 32-bit numbers all but the last are taken (it is below 2^-28 of a product: a second
+// part is up to 2^-7 of a number, a third 2^-14; without the two before it a product was good to 2^-20).  Tensor cores cut off a sum's last bits where fp32 units round: no chain is longer than two steps
 // of leading parts, the decayed state never is an accumulator, and 1 + A has its diagonal outside the product.
 //
 // Bound by issue: of the 4130 clocks a chunk of 128 x 128 takes with the delta rule, 2690 are products (8 clocks each and SM quarter).
@@ -92,9 +92,10 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], 
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-// Part products of a 16 x 16 tile in three parts and a 16 x 16 matrix in three planes, the smallest first; product i of six.
+// Part products of a 16 x 16 tile in three parts and a 16 x 16 matrix in three planes, the smallest first; product i of eight.
+constexpr int kPartProducts = 8;
 __device__ __forceinline__ void part_product(int i, float (&acc)[2][4], const uint32_t (&a)[3][4], const uint32_t (&m)[3][4]) {
-  const int order = i < 3 ? 2 : (i < 5 ? 1 : 0), j = i < 3 ? i : (i < 5 ? i - 3 : 0);
+  const int order = i < 2 ? 3 : (i < 5 ? 2 : (i < 7 ? 1 : 0)), j = i < 2 ? i + 1 : (i < 5 ? i - 2 : (i < 7 ? i - 5 : 0));
   mma_bf16(acc[0], a[order - j], m[j][0], m[j][1]);
   mma_bf16(acc[1], a[order - j], m[j][2], m[j][3]);
 }
@@ -502,7 +503,7 @@ __global__ void __launch_bounds__(Chunk<DK, MW, T>::THREADS, 1) head_chunk_kerne
         }
       }
     }
-    // (1 + A)^-1 b; part products of one order share an accumulator
+    // (1 + A)^-1 b; part products of one order share an accumulator, the two smallest that of the second largest
     if constexpr (DELTA) {
       uint32_t a[3][4], m[3][4];
       float d[3][2][4];
@@ -512,12 +513,14 @@ __global__ void __launch_bounds__(Chunk<DK, MW, T>::THREADS, 1) head_chunk_kerne
       for (int o = 0; o < 3; ++o)
 #pragma unroll
         for (int h = 0; h < 2; ++h) zero4(d[o][h]);
-      part_product(0, d[2], a, m);
-      part_product(3, d[1], a, m);
-      part_product(5, d[0], a, m);
-      part_product(1, d[2], a, m);
-      part_product(4, d[1], a, m);
+      part_product(0, d[1], a, m);
       part_product(2, d[2], a, m);
+      part_product(7, d[0], a, m);
+      part_product(1, d[1], a, m);
+      part_product(3, d[2], a, m);
+      part_product(5, d[1], a, m);
+      part_product(4, d[2], a, m);
+      part_product(6, d[1], a, m);
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         add4(d[1][h], d[2][h]);
@@ -619,7 +622,7 @@ __global__ void __launch_bounds__(Chunk<DK, MW, T>::THREADS, 1) head_chunk_kerne
             ldsm_x4_t(base + at_k + j * C::KPLANE + (2 * i + e) * 32, z[0], z[1], z[2], z[3]);
           }
       };
-      constexpr int STEPS = DK / 32, PER = (6 + STEPS - 1) / STEPS;
+      constexpr int STEPS = DK / 32, PER = (kPartProducts + STEPS - 1) / STEPS;
       load_keys(0);
 #pragma unroll
       for (int i = 0; i < STEPS; ++i) {
@@ -640,7 +643,7 @@ __global__ void __launch_bounds__(Chunk<DK, MW, T>::THREADS, 1) head_chunk_kerne
             }
 #pragma unroll
         for (int e = 0; e < PER; ++e)
-          if (i * PER + e < 6) part_product(i * PER + e, po, w, m);
+          if (i * PER + e < kPartProducts) part_product(i * PER + e, po, w, m);
 #pragma unroll
         for (int h = 0; h < 4; ++h)
 #pragma unroll

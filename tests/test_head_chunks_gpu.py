@@ -104,3 +104,35 @@ def test_numbers_that_are_not_finite_stay_where_they_are(dtype, delta):
     assert bad.sum() == 2 and bad[0, 9] and bad[1, 40]
     keep = torch.isfinite(s)
     assert err(s[keep], s1[keep]) < 8e-6
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32], ids=["bf16", "f32"])
+@pytest.mark.parametrize("heads,vdim", [(80, 16), (80, 128)])
+@pytest.mark.parametrize("chunks", [True, False])
+def test_products_of_two_32_bit_numbers(dtype, heads, vdim, chunks):
+    """Errors of the two products that take numbers of 24 bits on both sides, (1 + A)^-1 b and P u, do not add up: their mean over the
+    heads.  Two write strengths w just below 129/256, whose second parts are as large as they come, and powers of two otherwise."""
+    d, n = 128, 96
+    p = Problem(dtype, True, heads, 1, d, vdim, [n], [0])
+    p.rec.rate.zero_()
+    p.x.zero_()
+    g = torch.Generator(device=DEV).manual_seed(7)
+    p.b[:2] = (torch.rand(2, heads, generator=g, device=DEV) * 0.0077 + 0.0079).to(dtype)
+    w = torch.sigmoid(p.b[:2].double())
+    p.x[0, d] = 1024.0                                   # k_0 = (1, 0, ...)
+    p.x[1, d:d + 4] = 1024.0                             # k_1 = (1, 1, 1, 1) / 2
+    p.x[0, 2 * d:] = 64.0                                # v_0; the other tokens are zeros
+    u = 64.0 * w[0]
+    state = p.run(chunks)[1][1].double()                 # [heads, vdim, d]: second channel u_1 / 2 = -w_1 u_0 / 4
+    off = (state[:, :, 1] / (-0.25 * w[1] * u)[:, None] - 1).mean()
+    # a few roundings of 2^-25 each that average out, and the exponential's own bias within a ulp; six part products: -1.7e-7
+    assert off.abs() < 2.0 ** -23.5
+    if dtype == torch.float32:
+        p.x[1, d:2 * d] = 0.0
+        p.x[1, 0] = 1024.0                               # q_1 = (1, 0, ...): o_1 = q_scale u_0
+        p.rec.q_scale = 129 / 128 - 2.0 ** -23           # its parts as large as they come
+        p.b[0, :4] = 40.0                                # w = 1 where the row's norm is read from
+        o = p.run(chunks)[0][1].double().view(heads, vdim)
+        off = (o[4:] / (o[:4].mean() * w[0, 4:, None]) - 1).mean()
+        # as above, and the norm's rounding of one number, 2^-24; six part products: -3e-7
+        assert off.abs() < 2.0 ** -23 + 2.0 ** -24
