@@ -21,8 +21,10 @@
 // Code is kept small: with the preparation unrolled the two kinds of warps pushed one another out of the instruction cache
 // (4 x 2048 tokens of 32 heads 585 us, rolled up 329; token by token 1317).
 //
-// A chunk whose results are not all finite numbers is computed token by token in fp32, so that infinities and NaN go where they
-// do in the recurrence.
+// A number that is not three bf16 parts, because it is infinite, NaN or too small (below 2^-110 a third part may lie under bf16's
+// smallest number, 2^-133), leaves bits behind a third part.  A chunk with one in its state or its u is computed token by token in
+// fp32: infinities and NaN go where they do in the recurrence, and what is tiny keeps its bits.  Only of what the chunk's own decays
+// make smaller than 2^-40 of what it was, bits below 2^-133 are lost.
 #include "common.cuh"
 #include "proj_src.cuh"
 #include "mma_frag.cuh"
@@ -66,19 +68,30 @@ __device__ __forceinline__ float high_part(float x) { return __uint_as_float(__f
 __device__ __forceinline__ uint32_t pack_high(float lo, float hi) {
   return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632);
 }
+// what two parts leave of a number; its lower half is not zero where it is no bf16 number
+__device__ __forceinline__ float third_part(float x) {
+  const float r = x - high_part(x);
+  return r - high_part(r);
+}
 // two numbers as three pairs of bf16 that add up to them
 __device__ __forceinline__ void split3(float x, float y, uint32_t& a, uint32_t& b, uint32_t& c) {
-  const float xr = x - high_part(x), yr = y - high_part(y);
   a = pack_high(x, y);
-  b = pack_high(xr, yr);
-  c = pack_high(xr - high_part(xr), yr - high_part(yr));
+  b = pack_high(x - high_part(x), y - high_part(y));
+  c = pack_high(third_part(x), third_part(y));
+}
+// unless the lower half of `lost` is set (at once: left to itself, the compiler keeps all third parts to the end and spills)
+__device__ __forceinline__ void split3(float x, float y, uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& lost) {
+  const float xt = third_part(x), yt = third_part(y);
+  split3(x, y, a, b, c);
+  asm volatile("lop3.b32 %0, %0, %1, %2, 0xfe;" : "+r"(lost) : "r"(__float_as_uint(xt)), "r"(__float_as_uint(yt)));
 }
 // a 16 x 16 tile in accumulator layout as three A operands
-__device__ __forceinline__ void split_tile(const float (&x)[4], const float (&y)[4], uint32_t (&p)[3][4]) {
-  split3(x[0], x[1], p[0][0], p[1][0], p[2][0]);
-  split3(x[2], x[3], p[0][1], p[1][1], p[2][1]);
-  split3(y[0], y[1], p[0][2], p[1][2], p[2][2]);
-  split3(y[2], y[3], p[0][3], p[1][3], p[2][3]);
+template <typename... Lost>
+__device__ __forceinline__ void split_tile(const float (&x)[4], const float (&y)[4], uint32_t (&p)[3][4], Lost&... lost) {
+  split3(x[0], x[1], p[0][0], p[1][0], p[2][0], lost...);
+  split3(x[2], x[3], p[0][1], p[1][1], p[2][1], lost...);
+  split3(y[0], y[1], p[0][2], p[1][2], p[2][2], lost...);
+  split3(y[2], y[3], p[0][3], p[1][3], p[2][3], lost...);
 }
 __device__ __forceinline__ void zero4(float (&x)[4]) { x[0] = x[1] = x[2] = x[3] = 0.f; }
 __device__ __forceinline__ void add4(float (&x)[4], const float (&y)[4]) {
@@ -107,7 +120,7 @@ __device__ __forceinline__ void load_planes(uint32_t (&m)[3][4], uint32_t addr) 
 // of 16 channels at a time, the others' in `lo`.  Rows and parts of the next step are on their way during a step.
 template <int DK, int PL, bool KEYS, int PLANE>
 __device__ __forceinline__ void state_products(const float (&S)[DK / 8][4], uint32_t rows, uint32_t q_ofs, float (&hi)[2][2][4],
-                                               float (&lo)[2][2][4]) {
+                                               float (&lo)[2][2][4], uint32_t& lost) {
   constexpr int STEPS = DK / 16, W0 = KEYS ? 0 : 1;     // [0]: keys, [1]: queries
   constexpr int RUN = 2;                                // steps of a chain of leading parts
   float run[2][2][4];
@@ -129,7 +142,7 @@ __device__ __forceinline__ void state_products(const float (&S)[DK / 8][4], uint
       }
   };
   load(0);
-  split_tile(S[0], S[1], a[0]);
+  split_tile(S[0], S[1], a[0], lost);
 #pragma unroll
   for (int i = 0; i < STEPS; ++i) {
     const uint32_t(&x)[3][4] = a[i & 1];
@@ -142,7 +155,7 @@ __device__ __forceinline__ void state_products(const float (&S)[DK / 8][4], uint
         if (i % RUN == 0) zero4(run[w][h]);
         mma_bf16(run[w][h], x[0], y[0][2 * h], y[0][2 * h + 1]);
       }
-    if (i + 1 < STEPS) split_tile(S[(2 * i + 2) % (DK / 8)], S[(2 * i + 3) % (DK / 8)], a[(i + 1) & 1]);
+    if (i + 1 < STEPS) split_tile(S[(2 * i + 2) % (DK / 8)], S[(2 * i + 3) % (DK / 8)], a[(i + 1) & 1], lost);
 #pragma unroll
     for (int order = PL > 1 ? 3 : 2; order >= 1; --order)
 #pragma unroll
@@ -469,6 +482,7 @@ __global__ void __launch_bounds__(Chunk<DK, MW, T>::THREADS, 1) head_chunk_kerne
     const int left = n - c * kTok;                                 // tokens from here on
     if (!mbar_wait(&full[c % NST], (c / NST) & 1, &abort_flag, cp.status, ERR_WAIT_SMEM_FULL)) return;
     float U[2][4], O[2][4], v[2][4];
+    uint32_t lost = 0;
     if constexpr (F32) {
       const float* vr = reinterpret_cast<const float*>(s + C::oV) + cw + gr;
 #pragma unroll
@@ -487,7 +501,7 @@ __global__ void __launch_bounds__(Chunk<DK, MW, T>::THREADS, 1) head_chunk_kerne
     }
     {
       float hi[2][2][4], lo[2][2][4];
-      state_products<DK, PL, DELTA, C::KPLANE>(S, base + at_n, C::oQ, hi, lo);
+      state_products<DK, PL, DELTA, C::KPLANE>(S, base + at_n, C::oQ, hi, lo, lost);
       // b = w i v - (w i^2 G) S^T k
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
@@ -508,7 +522,7 @@ __global__ void __launch_bounds__(Chunk<DK, MW, T>::THREADS, 1) head_chunk_kerne
       uint32_t a[3][4], m[3][4];
       float d[3][2][4];
       load_planes(m, base + C::oT + at_m);
-      split_tile(U[0], U[1], a);
+      split_tile(U[0], U[1], a, lost);
 #pragma unroll
       for (int o = 0; o < 3; ++o)
 #pragma unroll
@@ -528,12 +542,20 @@ __global__ void __launch_bounds__(Chunk<DK, MW, T>::THREADS, 1) head_chunk_kerne
         add4(U[h], d[0][h]);
       }
     }
-    float odd = 0.f;                                               // NaN once one of u is not finite
+    // u, and decayed to the chunk's end for the state's update
+    uint32_t w[3][4], a[3][4];
+    split_tile(U[0], U[1], w, lost);
 #pragma unroll
-    for (int h = 0; h < 2; ++h)
+    for (int h = 0; h < 2; ++h) {
+      const float2 d = *reinterpret_cast<const float2*>(f + F_D * 16 + h * 8 + q2);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) odd = fmaf(U[h][e], 0.f, odd);
-    if (__any_sync(0xffffffffu, odd != 0.f)) {
+      for (int e = 0; e < 4; ++e) {
+        U[h][e] *= e & 1 ? d.y : d.x;
+        if (!((e & 1 ? d.y : d.x) < 0x1p-40f)) lost |= __float_as_uint(third_part(U[h][e]));
+      }
+    }
+    split_tile(U[0], U[1], a);
+    if (__any_sync(0xffffffffu, (lost & 0xffffu) != 0)) {
       for (int t = 0; t < min(left, kTok); ++t) {
         float sk0 = 0.f, sk1 = 0.f, sq0 = 0.f, sq1 = 0.f;
         const auto two = [&](int at, int i) {
@@ -597,19 +619,11 @@ __global__ void __launch_bounds__(Chunk<DK, MW, T>::THREADS, 1) head_chunk_kerne
     }
     // the state's update, and beside it P u
     {
-      uint32_t a[3][4], w[3][4], m[3][4];
+      uint32_t m[3][4];
       float po[2][4];
       load_planes(m, base + C::oP + at_m);
-      split_tile(U[0], U[1], w);
       zero4(po[0]);
       zero4(po[1]);
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const float2 d = *reinterpret_cast<const float2*>(f + F_D * 16 + h * 8 + q2);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) U[h][e] *= e & 1 ? d.y : d.x;
-      }
-      split_tile(U[0], U[1], a);
       const float gc = f[F_GC * 16];
       // two steps of 16 channels at a time: four tiles whose part products take turns
       uint32_t kb[2][2][PL][4];

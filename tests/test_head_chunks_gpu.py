@@ -27,8 +27,8 @@ class Problem:
         self.state = r(len(lens) + 1, *self.rec.state_shape, std=0.3)
         self.pad = pad
 
-    def run(self, chunks):
-        """(results before norm and gate, state); chunks False: token by token."""
+    def run(self, chunks, parts=1):
+        """(results, each of `parts` parts of a row brought to size 1, and state); chunks False: token by token."""
         rec, T = self.rec, sum(self.lens)
         wide = torch.zeros(T, self.x.shape[1] + self.pad, dtype=self.dtype, device=DEV)
         wide[:, :self.x.shape[1]] = self.x
@@ -39,7 +39,7 @@ class Problem:
         starts = [sum(self.lens[:i]) for i in range(len(self.lens))]
         # parts equal to the row's elements would lose the size: the norm over whole rows keeps what is compared here
         out = head_recurrence(rec, x, self.conv, P(self.a), P(self.b), gate, torch.ones(rec.heads * rec.vdim, device=DEV), state, ring,
-                              i32([n + d for n, d in zip(self.lens, self.done)]), parts=1, gate_act="none", q_start=i32(starts),
+                              i32([n + d for n, d in zip(self.lens, self.done)]), parts=parts, gate_act="none", q_start=i32(starts),
                               q_lens=i32(self.lens), rows=i32([i + 1 for i in range(len(self.lens))]), dtype=self.dtype,
                               max_q_len=0 if chunks else 1)
         torch.cuda.synchronize()
@@ -136,3 +136,34 @@ def test_products_of_two_32_bit_numbers(dtype, heads, vdim, chunks):
         off = (o[4:] / (o[:4].mean() * w[0, 4:, None]) - 1).mean()
         # as above, and the norm's rounding of one number, 2^-24; six part products: -3e-7
         assert off.abs() < 2.0 ** -23 + 2.0 ** -24
+
+
+# the rules that go by chunks (the state-space form of 32-bit models goes token by token), with four and with eight warps that hold states
+forms = pytest.mark.parametrize("dtype,delta,heads", [(torch.bfloat16, True, 2), (torch.bfloat16, True, 40), (torch.bfloat16, False, 2),
+                                                      (torch.bfloat16, False, 40), (torch.float32, True, 2)])
+
+
+@forms
+def test_tiny_states_and_values_keep_their_bits(dtype, delta, heads):
+    """Numbers whose third bf16 parts would lie under bf16's smallest: states of some 2^-120 and values of the same size."""
+    p = Problem(dtype, delta, heads, 1, 128, 128, [100, 40], [5, 0])
+    p.state *= 2.0 ** -118
+    p.x[:, 2 * 128:] *= 2.0 ** -118
+    (_, s), (_, s1), (_, states) = p.run(True), p.run(False), p.exact()
+    assert err(s[1:] * 2.0 ** 100, states * 2.0 ** 100) < 8e-6 and err(s1[1:] * 2.0 ** 100, states * 2.0 ** 100) < 8e-6
+
+
+def alike(a, b):
+    """Infinities and NaN in the same places, and the rest as close as sums in another order are."""
+    keep = torch.isfinite(b)
+    assert keep.any()
+    return torch.equal(torch.isnan(a), torch.isnan(b)) and torch.equal(a[torch.isinf(b)], b[torch.isinf(b)]) and err(a[keep], b[keep]) < 5e-3
+
+
+@forms
+def test_infinite_states_stay_where_they_are(dtype, delta, heads):
+    p = Problem(dtype, delta, heads, 1, 128, 128, [100, 40], [5, 7])
+    p.state[1, 0, 9, 40] = float("inf")
+    p.state[2, 1, 70, 3] = -float("inf")
+    (o, s), (o1, s1) = p.run(True, heads), p.run(False, heads)     # rows of a head that are not affected stay numbers
+    assert alike(s, s1) and alike(o, o1) and not torch.isfinite(s[1, 0, 9, 40]) and torch.isfinite(s[1, 0, 10]).all()
