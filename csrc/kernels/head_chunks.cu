@@ -22,9 +22,9 @@
 // (4 x 2048 tokens of 32 heads 585 us, rolled up 329; token by token 1317).
 //
 // A number that is not three bf16 parts, because it is infinite, NaN or too small (below 2^-110 a third part may lie under bf16's
-// smallest number, 2^-133), leaves bits behind a third part.  A chunk with one in its state or its u is computed token by token in
-// fp32: infinities and NaN go where they do in the recurrence, and what is tiny keeps its bits.  Only of what the chunk's own decays
-// make smaller than 2^-40 of what it was, bits below 2^-133 are lost.
+// smallest number, 2^-133), leaves bits behind a third part.  A chunk with one in its state, u, A, P or 32-bit keys and queries is
+// computed token by token in fp32: infinities and NaN go where they do in the recurrence, and what is tiny keeps its bits.  Only
+// where the chunk's own decays multiply to less than 2^-40, what they make tiny loses bits below 2^-133.
 #include "common.cuh"
 #include "proj_src.cuh"
 #include "mma_frag.cuh"
@@ -47,13 +47,14 @@ struct Chunk {
   static constexpr int KP = DK * 2 + 16, KPLANE = kTok * KP;                    // pitch of a row of keys, a plane
   static constexpr int VP = F32 ? (COLS + 4) * 4 : COLS * 2 + 16;
   static constexpr int oQ = PL * KPLANE, oV = 2 * PL * KPLANE, oT = oV + kTok * VP, oP = oT + 3 * kTok * kMatPitch;
-  static constexpr int oF = oP + 3 * kTok * kMatPitch, STAGE = oF + 9 * 16 * 4;
+  static constexpr int oF = oP + 3 * kTok * kMatPitch, STAGE = oF + 8 * 16 * 4;
   static constexpr int SP = 20;                        // pitch of the fp32 scratch matrices
   static constexpr int SCRATCH = 2 * kTok * SP * 4;
   static constexpr int oScratch = NST * STAGE, oOut = oScratch + kPrep * SCRATCH, SMEM = oOut + MW * kTok * 48;
 };
+constexpr float kFaded = 0x1p-40f;
 // rows of a stage's factors
-enum { F_EV = 0, F_EPG = 1, F_IQG = 2, F_D = 3, F_G = 4, F_EP = 5, F_IQ = 6, F_OU = 7, F_GC = 8 };
+enum { F_EV = 0, F_EPG = 1, F_IQG = 2, F_D = 3, F_G = 4, F_EP = 5, F_IQ = 6, F_GC = 7 };  // F_GC: the chunk's decay, then (a whole number) whether it lost bits
 
 struct ChunkParams {
   NkbHeadRec r;
@@ -217,6 +218,7 @@ __global__ void __launch_bounds__(Chunk<DK, MW, T>::THREADS, 1) head_chunk_kerne
       const int t0 = c * kTok;
       if (!mbar_wait(&empty[c % NST], ((c / NST) & 1) ^ 1u, &abort_flag, cp.status, ERR_WAIT_SMEM_EMPTY)) return;
       float a_raw = 0.f, b_raw = 0.f;
+      uint32_t lost = 0;
       if (lane < kTok && t0 + lane < n) {
         a_raw = proj_load(p.a, row0 + t0 + lane, head);
         if (DELTA) b_raw = proj_load(p.b, row0 + t0 + lane, head);
@@ -264,12 +266,12 @@ __global__ void __launch_bounds__(Chunk<DK, MW, T>::THREADS, 1) head_chunk_kerne
           }
           uint32_t u[3], w[3];
           uint8_t* d = s + tok * C::KP + ch * 2;
-          split3(k4.x, k4.y, u[0], u[1], u[2]);
-          split3(k4.z, k4.w, w[0], w[1], w[2]);
+          split3(k4.x, k4.y, u[0], u[1], u[2], lost);
+          split3(k4.z, k4.w, w[0], w[1], w[2], lost);
 #pragma unroll
           for (int j = 0; j < 3; ++j) *reinterpret_cast<uint2*>(d + j * C::KPLANE) = make_uint2(u[j], w[j]);
-          split3(q4.x, q4.y, u[0], u[1], u[2]);
-          split3(q4.z, q4.w, w[0], w[1], w[2]);
+          split3(q4.x, q4.y, u[0], u[1], u[2], lost);
+          split3(q4.z, q4.w, w[0], w[1], w[2], lost);
 #pragma unroll
           for (int j = 0; j < 3; ++j) *reinterpret_cast<uint2*>(d + C::oQ + j * C::KPLANE) = make_uint2(u[j], w[j]);
         }
@@ -369,7 +371,6 @@ __global__ void __launch_bounds__(Chunk<DK, MW, T>::THREADS, 1) head_chunk_kerne
         f[F_G * 16 + lane] = g;
         f[F_EP * 16 + lane] = ep;
         f[F_IQ * 16 + lane] = iq;
-        f[F_OU * 16 + lane] = iq * mq[lane * C::SP + lane];
       }
       __syncwarp();
       // lane j < 16: column j of A, decay from token j to the end and up to token j; lane 16 + j: column j of P
@@ -426,7 +427,8 @@ __global__ void __launch_bounds__(Chunk<DK, MW, T>::THREADS, 1) head_chunk_kerne
         }
         __syncwarp();
       }
-      // both in parts, a pair of columns at a time
+      // both in parts, a pair of columns at a time; an infinite key or query shows on the diagonal of P
+      uint32_t small = 0;
 #pragma unroll 1
       for (int i = lane; i < kTok * 8; i += 32) {
         const int t = i >> 3, j2 = (i & 7) * 2;
@@ -434,15 +436,19 @@ __global__ void __launch_bounds__(Chunk<DK, MW, T>::THREADS, 1) head_chunk_kerne
         uint32_t w[3];
         if (DELTA) {
           const float2 y = *reinterpret_cast<const float2*>(mk + t * C::SP + j2);
-          split3(y.x, y.y, w[0], w[1], w[2]);
+          split3(y.x, y.y, w[0], w[1], w[2], small);
 #pragma unroll
           for (int k = 0; k < 3; ++k) *reinterpret_cast<uint32_t*>(d + k * kTok * kMatPitch) = w[k];
         }
         const float2 y = *reinterpret_cast<const float2*>(mq + t * C::SP + j2);
-        split3(y.x, y.y, w[0], w[1], w[2]);
+        split3(y.x, y.y, w[0], w[1], w[2], small);
 #pragma unroll
         for (int k = 0; k < 3; ++k) *reinterpret_cast<uint32_t*>(d + (C::oP - C::oT) + k * kTok * kMatPitch) = w[k];
       }
+      // (all exponent bits: not finite, or such a large one beside a small one)
+      if (!(f[F_GC * 16] < kFaded) || (small & 0x7f800000u) == 0x7f800000u) lost |= small;
+      lost = __any_sync(0xffffffffu, (lost & 0xffffu) != 0);
+      if (lane == 0) f[F_GC * 16 + 1] = __uint_as_float(lost ? 1u : 0u);
       __syncwarp();
       if (lane == 0) mbar_arrive(&full[c % NST]);
     }
@@ -482,7 +488,7 @@ __global__ void __launch_bounds__(Chunk<DK, MW, T>::THREADS, 1) head_chunk_kerne
     const int left = n - c * kTok;                                 // tokens from here on
     if (!mbar_wait(&full[c % NST], (c / NST) & 1, &abort_flag, cp.status, ERR_WAIT_SMEM_FULL)) return;
     float U[2][4], O[2][4], v[2][4];
-    uint32_t lost = 0;
+    uint32_t lost = __float_as_uint(f[F_GC * 16 + 1]);
     if constexpr (F32) {
       const float* vr = reinterpret_cast<const float*>(s + C::oV) + cw + gr;
 #pragma unroll
@@ -549,28 +555,27 @@ __global__ void __launch_bounds__(Chunk<DK, MW, T>::THREADS, 1) head_chunk_kerne
     for (int h = 0; h < 2; ++h) {
       const float2 d = *reinterpret_cast<const float2*>(f + F_D * 16 + h * 8 + q2);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        U[h][e] *= e & 1 ? d.y : d.x;
-        if (!((e & 1 ? d.y : d.x) < 0x1p-40f)) lost |= __float_as_uint(third_part(U[h][e]));
-      }
+      for (int e = 0; e < 4; ++e) U[h][e] *= e & 1 ? d.y : d.x;
     }
-    split_tile(U[0], U[1], a);
+    const float gc = f[F_GC * 16];
+    uint32_t small = 0;
+    split_tile(U[0], U[1], a, small);
+    if (!(gc < kFaded)) lost |= small;
     if (__any_sync(0xffffffffu, (lost & 0xffffu) != 0)) {
       for (int t = 0; t < min(left, kTok); ++t) {
-        float sk0 = 0.f, sk1 = 0.f, sq0 = 0.f, sq1 = 0.f;
-        const auto two = [&](int at, int i) {
-          float2 w = make_float2(0.f, 0.f);
-#pragma unroll
-          for (int j = PL - 1; j >= 0; --j) {
-            const float2 y = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(s + at + j * C::KPLANE + t * C::KP + (i * 8 + q2) * 2));
-            w.x += y.x;
-            w.y += y.y;
+        float sk0 = 0.f, sk1 = 0.f, sq0 = 0.f, sq1 = 0.f, qk = 0.f;
+        const auto two = [&](int at, int col, int i) {
+          if constexpr (F32) {                                     // from memory: their parts may have lost bits
+            const T* row = x + (row0 + c * kTok + t) * p.x.ld + col + head / (p.heads / p.groups) * p.dim + i * 8 + q2;
+            return i * 8 < p.dim ? make_float2(row[0], row[1]) : make_float2(0.f, 0.f);
+          } else {
+            return unpack_bf16x2(*reinterpret_cast<const uint32_t*>(s + at + t * C::KP + (i * 8 + q2) * 2));
           }
-          return w;
         };
 #pragma unroll
         for (int i = 0; i < NT; ++i) {
-          const float2 q = two(C::oQ, i), k = two(0, i);
+          const float2 q = two(C::oQ, p.q_col, i), k = two(0, p.k_col, i);
+          qk = fmaf(q.x, k.x, fmaf(q.y, k.y, qk));
           sq0 = fmaf(q.x, S[i][0], fmaf(q.y, S[i][1], sq0));
           sq1 = fmaf(q.x, S[i][2], fmaf(q.y, S[i][3], sq1));
           if (DELTA) {
@@ -584,6 +589,7 @@ __global__ void __launch_bounds__(Chunk<DK, MW, T>::THREADS, 1) head_chunk_kerne
           sk1 += __shfl_xor_sync(0xffffffffu, sk1, w);
           sq0 += __shfl_xor_sync(0xffffffffu, sq0, w);
           sq1 += __shfl_xor_sync(0xffffffffu, sq1, w);
+          qk += __shfl_xor_sync(0xffffffffu, qk, w);
         }
         const T* vr = reinterpret_cast<const T*>(s + C::oV + t * C::VP) + cw + gr;
         const float v0 = cast_in<T>(vr[0]), v1 = cast_in<T>(vr[8]), g = f[F_G * 16 + t], ev = f[F_EV * 16 + t];
@@ -593,7 +599,7 @@ __global__ void __launch_bounds__(Chunk<DK, MW, T>::THREADS, 1) head_chunk_kerne
           u0 = fmaf(-es, sk0, u0);
           u1 = fmaf(-es, sk1, u1);
         }
-        const float oq = f[F_IQ * 16 + t] * g, ou = f[F_OU * 16 + t];
+        const float oq = f[F_IQ * 16 + t] * g, ou = f[F_IQ * 16 + t] * qk;
         float o0 = fmaf(oq, sq0, ou * u0), o1 = fmaf(oq, sq1, ou * u1);
         if (!DELTA) {
           o0 = fmaf(skip, v0, o0);
@@ -606,7 +612,7 @@ __global__ void __launch_bounds__(Chunk<DK, MW, T>::THREADS, 1) head_chunk_kerne
         }
 #pragma unroll
         for (int i = 0; i < NT; ++i) {
-          const float2 k = two(0, i);
+          const float2 k = two(0, p.k_col, i);
           S[i][0] = fmaf(k.x, u0, g * S[i][0]);
           S[i][1] = fmaf(k.y, u0, g * S[i][1]);
           S[i][2] = fmaf(k.x, u1, g * S[i][2]);
@@ -624,7 +630,6 @@ __global__ void __launch_bounds__(Chunk<DK, MW, T>::THREADS, 1) head_chunk_kerne
       load_planes(m, base + C::oP + at_m);
       zero4(po[0]);
       zero4(po[1]);
-      const float gc = f[F_GC * 16];
       // two steps of 16 channels at a time: four tiles whose part products take turns
       uint32_t kb[2][2][PL][4];
       const auto load_keys = [&](int i) {

@@ -167,3 +167,22 @@ def test_infinite_states_stay_where_they_are(dtype, delta, heads):
     p.state[2, 1, 70, 3] = -float("inf")
     (o, s), (o1, s1) = p.run(True, heads), p.run(False, heads)     # rows of a head that are not affected stay numbers
     assert alike(s, s1) and alike(o, o1) and not torch.isfinite(s[1, 0, 9, 40]) and torch.isfinite(s[1, 0, 10]).all()
+
+
+@forms
+def test_infinite_keys_and_queries_reach_what_they_reach(dtype, delta, heads):
+    p = Problem(dtype, delta, heads, heads, 128, 128, [100, 40], [5, 0])
+    p.x[37, heads * 128 + 5] = float("inf")                  # a key of head 0
+    p.x[70, 128 + 7] = float("inf")                          # a query of head 1
+    p.x[120, heads * 128 + 128 + 3] = float("nan")           # a key of head 1
+    p.x[131, heads * 128 + 9] = float("inf")                 # a key of head 0, whose first value is 0
+    p.x[131, 2 * heads * 128] = 0.0
+    (o, s), (o1, s1) = p.run(True, heads), p.run(False, heads)
+    assert alike(s, s1) and alike(o, o1) and not torch.isfinite(s[1, 0, :, 5]).any() and torch.isfinite(s[1, 1]).all()
+
+
+def test_tiny_32_bit_keys_keep_their_bits():
+    p = Problem(torch.float32, True, 2, 1, 128, 128, [100, 40], [0, 0])
+    p.x[:, :2 * 128] *= 2.0 ** -118
+    (_, s), (_, s1), (_, states) = p.run(True), p.run(False), p.exact()
+    assert err(s[1:] * 2.0 ** 100, states * 2.0 ** 100) < 8e-6 and err(s1[1:] * 2.0 ** 100, states * 2.0 ** 100) < 8e-6
