@@ -64,6 +64,11 @@ struct ChunkParams {
 __device__ __forceinline__ void hc_cp16(void* dst, const void* src, bool on) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(on ? 16 : 0) : "memory");
 }
+// a warp goes on, or gives up, as a whole: matrix instructions and shuffles follow
+__device__ __forceinline__ bool hc_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+  const bool ok = mbar_wait(bar, parity, abort_flag, status, code);
+  return __all_sync(0xffffffffu, ok);
+}
 __device__ __forceinline__ float high_part(float x) { return __uint_as_float(__float_as_uint(x) & 0xffff0000u); }
 // the upper halves of two words
 __device__ __forceinline__ uint32_t pack_high(float lo, float hi) {
@@ -216,7 +221,7 @@ __global__ void __launch_bounds__(Chunk<DK, MW, T>::THREADS, 1) head_chunk_kerne
     for (int c = warp - MW; c < chunks; c += kPrep) {
       uint8_t* s = sm + c % NST * C::STAGE;
       const int t0 = c * kTok;
-      if (!mbar_wait(&empty[c % NST], ((c / NST) & 1) ^ 1u, &abort_flag, cp.status, ERR_WAIT_SMEM_EMPTY)) return;
+      if (!hc_wait(&empty[c % NST], ((c / NST) & 1) ^ 1u, &abort_flag, cp.status, ERR_WAIT_SMEM_EMPTY)) return;
       float a_raw = 0.f, b_raw = 0.f;
       uint32_t lost = 0;
       if (lane < kTok && t0 + lane < n) {
@@ -486,7 +491,7 @@ __global__ void __launch_bounds__(Chunk<DK, MW, T>::THREADS, 1) head_chunk_kerne
     const float* f = reinterpret_cast<const float*>(s + C::oF);
     const uint32_t base = smem_u32(s);
     const int left = n - c * kTok;                                 // tokens from here on
-    if (!mbar_wait(&full[c % NST], (c / NST) & 1, &abort_flag, cp.status, ERR_WAIT_SMEM_FULL)) return;
+    if (!hc_wait(&full[c % NST], (c / NST) & 1, &abort_flag, cp.status, ERR_WAIT_SMEM_FULL)) return;
     float U[2][4], O[2][4], v[2][4];
     uint32_t lost = __float_as_uint(f[F_GC * 16 + 1]);
     if constexpr (F32) {
