@@ -75,6 +75,7 @@ int nkb_gemm_bf16(const void* A, const void* B, void* out, int rows, int cols, i
                   int gate_off, const void* bias, int bias_on_rows, const void* residual, int block_n, int max_ctas,
                   int weights_operand, int ctas_per_sm, int act, float act_a, float act_b, void* stream);
 int nkb_gemm_effective_splits(int k, int splits);
+int nkb_gemm_ring_stages(int block_n, int ctas_per_sm, int gated, int push);
 int nkb_gemm_bf16_2cta(const void* A, const void* B, void* out, int m, int n, int k, long long lda, long long ldb,
                        long long ldo, const void* bias, const void* residual, int gated, int gate_off, int act,
                        float act_a, float act_b, int splits, long long split_stride, int static_b, int tile_n, void* stream);

@@ -24,17 +24,29 @@ static int ring_stages(const GemmArgs& args, int& smem, bool lean = false) {
   const int stage_bytes = a_tiles * kATileBytes + b_tiles * BN * kBlockK * 2;
   // control block + staging: the push tile (32 tokens x 128 features bf16), or two 16-column buffers of fp32 where the compact epilogue
   // stores by bulk copies
-  const int extra = 512 + (PUSH ? 32 * kTileRows * 2 : (lean && bulk_stores() ? 2 * 16 * kTileRows * 4 : 0));
+  constexpr int kBulkStaging = 2 * 16 * kTileRows * 4;
+  const int extra = 512 + (PUSH ? 32 * kTileRows * 2 : (lean && bulk_stores() ? kBulkStaging : 0));
   const int budget = (MINB == 2 ? 113 * 1024 : 232448) - 1024 - extra - 64;
   int stages = budget / stage_bytes;
-  if (stages > kMaxStages) stages = kMaxStages;
   // A stage more pays for wide operands (us of products with two CTAs per SM, three stages instead of two at 128 tokens: 14336 -> 4096 31.7 ->
   // 25.2, 4096 -> 128256 229 -> 188; four instead of three at 64: 25.2 -> 22.6 and 174 -> 171), but at 32 the fifth gained nothing and the
-  // steps of one sequence lost by it (four GPT-OSS layers 562 -> 574).
-  if (lean && BN == 32) stages = stages < (MINB == 2 ? 4 : 5) ? stages : (MINB == 2 ? 4 : 5);
+  // steps of one sequence lost by it (four GPT-OSS layers 562 -> 574): rings of 32 tokens that have four stages and more do not grow by the
+  // staging's memory.  (The push tile's is in use, so those rings are what they were.)
+  if (lean && BN == 32 && !PUSH && !bulk_stores()) {
+    const int before = (budget - kBulkStaging) / stage_bytes, most = before > 4 ? before : 4;
+    if (stages > most) stages = most;
+  }
   static_assert(sizeof(GemmCtrl) <= 512, "control block grew");
+  if (stages > kMaxStages) stages = kMaxStages;
   smem = stages * stage_bytes + 1024 + extra + 64;
   return stages;
+}
+
+template <int BN>
+static int ring_of(const GemmArgs& args, bool two, bool push) {
+  int smem = 0;
+  if (push) return ring_stages<BN, 2, true, false>(args, smem, true);
+  return two ? ring_stages<BN, 2, false, false>(args, smem, true) : ring_stages<BN, 1, false, false>(args, smem, true);
 }
 
 // The decode orientation (transposed output, bias per row or none) runs the kernel with the compact epilogue.
@@ -234,6 +246,21 @@ extern "C" int nkb_gemm_bf16(const void* A, const void* B, void* out, int rows, 
     case 128: return launch_gemm<128, 1>(ta, tb, args, max_ctas, s);
     case 256: return launch_gemm<256, 1>(ta, tb, args, max_ctas, s);
     default: return -2;
+  }
+}
+
+// Stages of the ring that products of up to block_n tokens in the decode orientation get (push: with the fused push epilogue, which has
+// two CTAs per SM), 0 where there is no such form.
+extern "C" int nkb_gemm_ring_stages(int block_n, int ctas_per_sm, int gated, int push) {
+  GemmArgs args{};
+  args.gated = gated;
+  const bool two = ctas_per_sm == 2;
+  if (push && (!two || gated)) return 0;
+  switch (block_n) {
+    case 32: return ring_of<32>(args, two, push);
+    case 64: return ring_of<64>(args, two, push);
+    case 128: return ring_of<128>(args, two, push);
+    default: return 0;
   }
 }
 

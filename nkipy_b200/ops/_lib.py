@@ -164,6 +164,7 @@ _SIGNATURES = {
                                  c_int, _P, _P, _P]),
     "nkb_moe_combine": (c_int, [_P, _P, _P, c_int, c_int, c_int, _P, _P]),
     "nkb_gemm_effective_splits": (c_int, [c_int, c_int]),
+    "nkb_gemm_ring_stages": (c_int, [c_int, c_int, c_int, c_int]),
     "nkb_decode_gemm_splits": (c_int, [c_int, c_int, c_int]),
     "nkb_decode_gemm": (c_int, [_P, _P, _P, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int, c_int,
                                 c_int, _P, _P, c_float, c_float, c_int, c_int, _P]),
