@@ -212,7 +212,7 @@ extern "C" int nkb_gemm_bf16(const void* A, const void* B, void* out, int rows, 
   args.act_a = act_a;
   args.act_b = act_b;
   args.gate_off = gate_off;
-  args.transpose_out = transpose_out;
+  args.transpose_out = transpose_out ? 1 : 0;   // 2 is set by mark_bulk only, with the staging memory it needs
   args.out_fp32 = out_fp32;
   args.bias_on_rows = bias_on_rows;
   args.ldo = ldo;

@@ -460,3 +460,20 @@ def test_linear_cta_pair_kernel_gated(M, I, K):
     rel = ((y.float() - ref).norm() / ref.norm()).item()
     assert y.shape == (M, I) and rel < 1e-2, rel
     assert O.device_status() == 0
+
+
+@pytest.mark.parametrize("block_n", [32, 64, 128])
+def test_any_true_transpose_flag_is_the_same(block_n):
+    """The flag of the C entry is yes or no: no value of it selects an epilogue for which no shared memory is set aside."""
+    M, N, K = block_n - 3, 256, 512
+    g = torch.Generator(device=DEV).manual_seed(block_n)
+    x, w = (torch.randn(n, K, device=DEV, generator=g).to(torch.bfloat16) for n in (M, N))
+    outs = []
+    for flag in (1, 2, 3):
+        y = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+        rc = ops._lib.lib().nkb_gemm_bf16(w.data_ptr(), x.data_ptr(), y.data_ptr(), N, M, K, K, K, N, flag, 0, 1, 0, 0, 0, None, 1, None,
+                                          block_n, 0, 0, 2, 0, 0.0, 0.0, ops._stream())
+        assert rc == 0
+        outs.append(y)
+    assert all(torch.equal(y, outs[0]) for y in outs) and rel_err(outs[0], x.float() @ w.float().T) < 5e-3
+    assert ops.device_status() == 0
