@@ -442,9 +442,9 @@ class GenerationEngine:
         host[:B] = ids
         if wanted <= pitch:
             host[2 * pitch:2 * pitch + wanted] = rows
+        self._opened.update(slots)               # from the copy on, whatever becomes of the step
         self._inputs.copy_(inputs, non_blocking=True)
         self.decode_step_device()
-        self._opened.update(slots)
         logits = None
         if wanted:
             at = self._inputs[2 * pitch:2 * pitch + wanted] if wanted <= pitch else self._to_device(np.array(rows, dtype=np.int32))[0]

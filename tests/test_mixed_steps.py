@@ -135,6 +135,23 @@ def test_release_takes_any_iterable(device):
 
 
 @pytest.mark.parametrize("device", DEVICES)
+def test_release_after_a_failed_step(device, monkeypatch):
+    """Rows whose lengths a decode step has brought over are inactive after their release, also where the step itself failed."""
+    e = engine(device)
+    seqs = [e.open_request() for _ in range(3)]
+    e.run_step([StepEntry(s, ids(5, i), [4]) for i, s in enumerate(seqs)])
+
+    def fails():
+        raise RuntimeError("no memory")
+    with monkeypatch.context() as m:
+        m.setattr(e, "decode_step_device", fails)
+        with pytest.raises(RuntimeError, match="no memory"):
+            e.run_step([StepEntry(s, [9], [0]) for s in seqs[:2]])
+    e.release(seqs)
+    assert e.context_lens.tolist() == [-1] * 6
+
+
+@pytest.mark.parametrize("device", DEVICES)
 @pytest.mark.parametrize("lens", [[1], [129], [1, 1, 1], [31, 33, 1, 64, 5], [1] * 70 + [300]])
 def test_positions_of_packed_tokens(device, lens):
     """Positions and slots as counted out one by one, for new sequences and continued ones."""
