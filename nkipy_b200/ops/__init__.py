@@ -733,7 +733,16 @@ def decode_advance(context_lens: torch.Tensor, block_table: torch.Tensor, positi
 def packed_positions(q_start: torch.Tensor, q_lens: torch.Tensor, context_lens: torch.Tensor, block_table: torch.Tensor, tokens: int,
                      block_size: int = 32) -> tuple:
     """(positions, cache slots), int32 [tokens], of the tokens of a packed step: sequence b's q_lens[b] new tokens, in rows q_start[b]
-    on, are the last of its context_lens[b]; its blocks are row b of the table.  The sequences follow one another without gaps."""
+    on, are the last of its context_lens[b]; its blocks are row b of the table.  The sequences follow one another without gaps.  All
+    int32 and contiguous, on one device."""
+    B, dev = q_start.numel(), q_start.device
+    for t, shape in ((q_start, (B,)), (q_lens, (B,)), (context_lens, (B,)), (block_table, (B, block_table.shape[-1]))):
+        if t.dtype != torch.int32 or t.device != dev or not t.is_contiguous():
+            raise TypeError("packed_positions wants contiguous int32 tensors on one device")
+        if t.shape != shape:
+            raise ValueError("packed_positions wants one start, length, context length and table row per sequence")
+    if tokens < 0 or block_size < 1 or (tokens and not block_table.numel()):
+        raise ValueError("packed_positions: sizes do not fit")
     positions = torch.empty((tokens,), dtype=torch.int32, device=q_start.device)
     slots = torch.empty_like(positions)
     if not _native(positions):
@@ -744,7 +753,7 @@ def packed_positions(q_start: torch.Tensor, q_lens: torch.Tensor, context_lens: 
         slots.copy_(block_table.long()[seq, pos // block_size] * block_size + pos % block_size)
         return positions, slots
     rc = _lib.lib().nkb_packed_positions(q_start.data_ptr(), q_lens.data_ptr(), context_lens.data_ptr(), block_table.data_ptr(),
-                                         positions.data_ptr(), slots.data_ptr(), q_start.shape[0], tokens, block_table.stride(0),
+                                         positions.data_ptr(), slots.data_ptr(), B, tokens, block_table.shape[1],
                                          block_size, _stream())
     _lib.check(rc, "nkb_packed_positions")
     _count_launch()

@@ -165,6 +165,20 @@ def test_positions_of_packed_tokens(device, lens):
     assert slots.tolist() == [int(table[b, p // BLOCK_SIZE]) * BLOCK_SIZE + p % BLOCK_SIZE for b, p in want]
 
 
+@pytest.mark.parametrize("device", DEVICES)
+def test_positions_refuse_what_does_not_fit(device):
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=device)
+    good = dict(q_start=i32([0, 2]), q_lens=i32([2, 3]), context_lens=i32([2, 40]), block_table=i32([[1, 2], [3, 4]]), tokens=5)
+    assert ops.packed_positions(**good)[0].tolist() == [0, 1, 37, 38, 39]
+    for bad in (dict(q_lens=i32([2])), dict(context_lens=i32([2, 40, 1])), dict(block_table=i32([[1, 2]])), dict(tokens=-1), dict(block_size=0),
+                dict(block_table=i32([[], []]))):
+        with pytest.raises(ValueError):
+            ops.packed_positions(**{**good, **bad})
+    for bad in (dict(q_lens=good["q_lens"].long()), dict(q_start=i32([0, 9, 2, 9])[::2]), dict(block_table=i32([[1, 2, 9], [3, 4, 9]])[:, :2])):
+        with pytest.raises(TypeError):
+            ops.packed_positions(**{**good, **bad})
+
+
 def test_token_ids_of_all_kinds():
     """Lists, tuples, arrays and tensors, of whole numbers and of what stands for them, alone and beside one another."""
     e = engine("cpu")
