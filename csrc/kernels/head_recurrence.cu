@@ -9,7 +9,7 @@
 //                  S^T q = g (S_old^T q) + (k . q) u,
 //              so a token needs one exchange of sums between lanes: a transposing butterfly over the 2 NC sums.  Unit norms,
 //              scales and step sizes are factors of these sums, folded into five numbers per token.  A tile of tokens is copied
-//              as it is while the previous one is multiplied.  Long sequences go by chunks where their sizes allow (head_chunks.cu).
+//              as it is while the previous one is multiplied.
 //   step       one new token per sequence (decode).  A CTA owns a head of a sequence, streams its state through registers once
 //              and computes everything around it itself: the convolution of its channels, unit norms, decay, step size, and
 //              (per-head norms) the norm and gate of the result.
@@ -21,7 +21,6 @@
 #include "proj_src.cuh"
 #include "activations.cuh"
 #include "head_recurrence.h"
-#include "head_chunks.h"
 #include "api.h"
 
 namespace nkb {
@@ -974,7 +973,6 @@ extern "C" int nkb_head_rec_scan(const NkbHeadRec* a, void* stream) {
   if (a->batch <= 0 || a->tokens <= 0) return 0;
   if (!head_rec_ok(*a) || a->x.splits != 1 || !a->q_start || !a->q_lens) return -2;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  if (head_chunks_ok(*a) && head_chunks_pay(*a)) return head_chunks(*a, s);
   const bool async = a->bf16 && a->x.bf16 && ((a->dim | a->vdim | a->q_col | a->k_col | a->v_col) & 7) == 0 && al16(a->x.ptr) &&
                      a->x.ld % 8 == 0;
   if (a->dim <= 32) return launch_rec<4>(*a, async, s);

@@ -32,5 +32,4 @@ struct NkbHeadRec {
   int batch, tokens, heads, groups, dim, vdim;
   float q_scale, eps, unit_eps;
   float* conv_out;          // step: room for the convolved channels [batch, channels] (a launch of their own), or null
-  int longest;              // scan: most new tokens of a sequence, 0 where the caller does not know
 };

@@ -314,7 +314,7 @@ class DeltaMixer:
         x, gate, strength, decay = columns(y, self.widths)
         return ops.head_recurrence(self.rule, x, self.conv, decay, strength, gate, self.norm, cache.state[entry],
                                    cache.state[entry + 1], b.context_lens, q_start=b.q_start, q_lens=b.q_lens, rows=b.rows,
-                                   dtype=model.dtype, max_q_len=b.max_q_len)
+                                   dtype=model.dtype)
 
 
 class StateSpaceMixer:
@@ -336,7 +336,7 @@ class StateSpaceMixer:
         gate, x, dt = columns(y, self.widths)
         return ops.head_recurrence(self.rule, x, self.conv, dt, None, gate, self.norm, cache.state[entry], cache.state[entry + 1],
                                    b.context_lens, parts=self.parts, q_start=b.q_start, q_lens=b.q_lens, rows=b.rows,
-                                   dtype=model.dtype, max_q_len=b.max_q_len)
+                                   dtype=model.dtype)
 
 
 class BlendMixer:

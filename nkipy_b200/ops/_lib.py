@@ -71,7 +71,7 @@ class HeadRecArg(ctypes.Structure):
                                         "q_start", "q_lens", "context_lens", "out")] + \
                [(n, c_int) for n in ("taps", "channels", "q_col", "k_col", "v_col", "gate_act", "bf16", "batch", "tokens", "heads",
                                      "groups", "dim", "vdim")] + [(n, c_float) for n in ("q_scale", "eps", "unit_eps")] + \
-               [("conv_out", c_void_p), ("longest", c_int)]
+               [("conv_out", c_void_p)]
 
 
 class TanhNormArg(ctypes.Structure):

@@ -158,8 +158,8 @@ def head_recurrence(r: HeadRecurrence, x: Proj, conv: ShortConv, a: Proj, b: Opt
 
     state [slots, heads, vdim, dim_p] and conv_state [slots, taps, channels], fp32, are read and written in place at slot
     rows[b] (rows None: b).  context_lens counts the new tokens; a sequence whose tokens are all new starts from zero, one with
-    a negative length is skipped.  q_lens None: one new token per sequence (a decode step).  max_q_len: most new tokens of a sequence,
-    where the caller knows it (it decides how the tokens are worked off)."""
+    a negative length is skipped.  q_lens None: one new token per sequence (a decode step).  max_q_len, the most new tokens of a
+    sequence, may be given; results do not depend on it."""
     T, inner = x.t.shape[-2], r.heads * r.vdim
     if r.delta != (b is not None):
         raise ValueError("the delta rule has write strengths, the state-space form has none")
@@ -207,7 +207,6 @@ def head_recurrence(r: HeadRecurrence, x: Proj, conv: ShortConv, a: Proj, b: Opt
     y = short_conv(x, conv, conv_state, context_lens, q_start, q_lens, rows, dtype=dtype)
     out = torch.empty((T, inner), dtype=dtype, device=state.device)
     arg.x, arg.q_start, arg.q_lens, arg.out = Proj(y, 0, y.shape[1]).arg(), q_start.data_ptr(), q_lens.data_ptr(), out.data_ptr()
-    arg.longest = max_q_len
     _lib.check(L.nkb_head_rec_scan(ctypes.byref(arg), _stream()), "nkb_head_rec_scan")
     _count_launch()
     if parts:
