@@ -571,11 +571,6 @@ static int launch_rec(const NkbHeadRec& p, bool async, cudaStream_t s) {
 }
 
 // ------------------------------------------------------------------------------------------------ step
-// TH threads hold 128 columns of the state at a time, in blocks of TH / 8.  Bound by streaming the state twice; what keeps it from
-// that is the time in which a CTA's loads are back and the convolution, norms and gates of its head are not.  512 threads with
-// half the columns each do that part in one pass and hold two heads per SM in 64 registers a thread: 64 sequences of 32 heads of
-// 128 x 128, 84 -> 79 us with the delta rule and 78 -> 65 us without (256 threads held one head per SM).  With 256 threads no number
-// of CTAs per SM is asked for (0): asked for one, the compiler takes twice the registers, 64 x 64 34 -> 60 us.
 // The convolution of a step's tokens in a launch of its own: V channels of a sequence per thread.
 template <int V>
 __global__ void __launch_bounds__(128) conv_step_kernel(const __grid_constant__ NkbHeadRec p) {
@@ -631,10 +626,20 @@ __global__ void __launch_bounds__(128) conv_step_kernel(const __grid_constant__ 
   }
 }
 
+// TH threads hold 128 columns of the state at a time, in blocks of TH / 8.  Bound by streaming the state twice; what keeps it from
+// that is the time in which a CTA's loads are back and the convolution, norms and gates of its head are not.  512 threads with
+// half the columns each do that part in one pass and hold two heads per SM in 64 registers a thread: 64 sequences of 32 heads of
+// 128 x 128, 84 -> 79 us with the delta rule and 78 -> 65 us without (256 threads held one head per SM).  With 256 threads no number
+// of CTAs per SM is asked for (0): asked for one, the compiler takes twice the registers, 64 x 64 34 -> 60 us.
+//
 // APART: the channels have been convolved by the launch just before (within the step, what a CTA waits for is the convolution of its
-// channels, with nothing left to load).  Everything else that the step reads was written before that launch began, so it is on its way
-// before the wait for it: the state above all.  Both launches, 64 sequences of 32 heads of 128 x 128: 70.5 -> 64.9 us with the delta rule,
+// channels, with nothing left to load).  Everything else that the step reads, the state above all, is on its way before the wait for
+// that launch.  What makes it final by then: the step's CTAs start only once every CTA of conv_step_kernel has let them, which each does
+// behind its own wait for all kernels before it, such as the projection that writes the gates.  So conv_step_kernel must not call
+// griddep_launch before griddep_wait.  Both launches, 64 sequences of 32 heads of 128 x 128: 70.5 -> 64.9 us with the delta rule,
 // 56.0 -> 47.6 without; 16 sequences 21.0 -> 19.5 and 17.3 -> 16.4, 8 sequences 11.7 -> 11.3 and 9.7 -> 9.7, 4 sequences 8.2 -> 9.1.
+// Smaller heads change sides at the same number of them (delta rule, 256, 512 and 1024 heads of all sequences): 64 x 64 6.7 -> 6.9, 12.1 -> 10.8,
+// 21.6 -> 15.7; 32 x 32 4.9 -> 5.4, 6.4 -> 6.6, 12.0 -> 11.2.
 template <int TH, int CH, bool DELTA, bool APART, typename OutT>
 __global__ void __launch_bounds__(TH, TH == 512 ? 2 : 0) head_rec_step_kernel(const __grid_constant__ NkbHeadRec p) {
   constexpr int D8 = 8 * CH, kCols = TH / 8, kBlocks = 128 / kCols;
