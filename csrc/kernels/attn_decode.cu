@@ -339,8 +339,8 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
       mbar_expect_tx(&bars[warp][stage], kStageBytes);
 #pragma unroll
       for (int h = 0; h < NH; ++h) {
-        tma_load_4d_once(dst + h * kHalfBytes, &tmK, &bars[warp][stage], h * 64, 0, kvh, blk, policy);
-        tma_load_4d_once(dst + kMatBytes + h * kHalfBytes, &tmV, &bars[warp][stage], h * 64, 0, kvh, blk, policy);
+        tma_load_4d_as(dst + h * kHalfBytes, &tmK, &bars[warp][stage], h * 64, 0, kvh, blk, policy);
+        tma_load_4d_as(dst + kMatBytes + h * kHalfBytes, &tmV, &bars[warp][stage], h * 64, 0, kvh, blk, policy);
       }
     }
   };

@@ -221,22 +221,36 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m
       ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(x), "r"(y)
       : "memory");
 }
-// The same load of bytes that are read once per step (weights and cached keys of a decode step, several times the size of L2): first to
-// be evicted, they do not push out what the next kernels read (partial sums, activations, tables, and their own instructions, which the
-// next layer runs again).  Decode steps of four Llama layers 569 -> 562 us (1 sequence), 890 -> 879 (64), of four GPT-OSS layers 586 -> 562.
+// The same load with an L2 policy.  Bytes that are read once per step (weights and cached keys of a decode step, several times the size
+// of L2) are first to be evicted, so that they do not push out what the next kernels read (partial sums, activations, tables, and their own
+// instructions, which the next layer runs again).  Decode steps of four Llama layers 569 -> 562 us (1 sequence), 890 -> 879 (64), of four
+// GPT-OSS layers 586 -> 562.  Pages that many sequences read are no slower by it: attention of 64 sequences over a shared prefix of 1024 and 64
+// tokens of their own 34.2 -> 33.5 us, 4096 and 64 120.7 -> 119.0, 16 sequences 29.8 -> 29.8.
+//
+// A model that fits in L2 reads its weights there step after step, and loses by the policy: 60 MB of weights (two layers of 1024), one sequence
+// 81.1 -> 84.8 us, 16 92.2 -> 94.1.  A launch does not know its model, so the line is a matrix (of all experts) of an eighth of L2: below it
+// the weights keep the usual policy (that model: 81.9 and 91.1).  Models between both, us without, with the policy for all, with the line:
+// 76 MB (head of 33 MB), one sequence 84.0, 87.9, 85.2; one layer of 2048 (111 MB) 66.5, 63.6, 62.1; 125 MB, matrices below 12 MB but for the
+// head, 162, 158, 160.
+constexpr long long kOnceBytes = 16 << 20;
 __device__ __forceinline__ uint64_t l2_evict_first() {
   uint64_t p;
   asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
   return p;
 }
-__device__ __forceinline__ void tma_load_2d_once(void* smem_dst, const CUtensorMap* m, uint64_t* bar, int x, int y, uint64_t policy) {
+__device__ __forceinline__ uint64_t l2_evict_normal() {
+  uint64_t p;
+  asm("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(p));
+  return p;
+}
+__device__ __forceinline__ void tma_load_2d_as(void* smem_dst, const CUtensorMap* m, uint64_t* bar, int x, int y, uint64_t policy) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4}], [%2], %5;" ::"r"(
           smem_u32(smem_dst)),
       "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(x), "r"(y), "l"(policy)
       : "memory");
 }
-__device__ __forceinline__ void tma_load_3d_once(void* smem_dst, const CUtensorMap* m, uint64_t* bar, int x, int y, int z,
+__device__ __forceinline__ void tma_load_3d_as(void* smem_dst, const CUtensorMap* m, uint64_t* bar, int x, int y, int z,
                                                  uint64_t policy) {
   asm volatile(
       "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %5}], [%2], "
@@ -244,7 +258,7 @@ __device__ __forceinline__ void tma_load_3d_once(void* smem_dst, const CUtensorM
       "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z), "l"(policy)
       : "memory");
 }
-__device__ __forceinline__ void tma_load_4d_once(void* smem_dst, const CUtensorMap* m, uint64_t* bar, int x, int y, int z, int w,
+__device__ __forceinline__ void tma_load_4d_as(void* smem_dst, const CUtensorMap* m, uint64_t* bar, int x, int y, int z, int w,
                                                  uint64_t policy) {
   asm volatile(
       "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %5, %6}], [%2], "

@@ -204,27 +204,22 @@ __device__ __forceinline__ bool gemm_bf16_body(const CUtensorMap& tmA, const CUt
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     // weights on the row side that a single column of tiles reads (experts: mostly) are read once per launch
-    const bool once = GROUPED ? args.cols <= grp.num_groups * BN : Sync::lean && args.weights_operand == 0 && args.num_col_tiles == 1;
-    const uint64_t policy = l2_evict_first();
+    const bool once = (GROUPED ? args.cols <= grp.num_groups * BN : Sync::lean && args.weights_operand == 0 && args.num_col_tiles == 1) &&
+                      2LL * a_tiles * args.rows * args.k * (GROUPED ? grp.num_groups : 1) >= kOnceBytes;
+    const uint64_t policy = once ? l2_evict_first() : l2_evict_normal();
     auto issue = [&](int stage, int kb, int row0, int col0, int group, bool expect, bool do_a, bool do_b) {
       uint8_t* a_ptr = tiles + stage * stage_bytes;
       uint8_t* b_ptr = a_ptr + a_tiles * kATileBytes;
       if (expect) mbar_expect_tx(&ctrl->full[stage], stage_bytes);
       if (do_a) {
         if constexpr (GROUPED) {
-          if (once) {
-            tma_load_3d_once(a_ptr, &tmA, &ctrl->full[stage], kb * kBlockK, row0, group, policy);
-            if (args.gated == 1)
-              tma_load_3d_once(a_ptr + kATileBytes, &tmA, &ctrl->full[stage], kb * kBlockK, args.gate_off + row0, group, policy);
-          } else {
-            tma_load_3d(a_ptr, &tmA, &ctrl->full[stage], kb * kBlockK, row0, group);
-            if (args.gated == 1)
-              tma_load_3d(a_ptr + kATileBytes, &tmA, &ctrl->full[stage], kb * kBlockK, args.gate_off + row0, group);
-          }
-        } else if (once) {
-          tma_load_2d_once(a_ptr, &tmA, &ctrl->full[stage], kb * kBlockK, row0, policy);
+          tma_load_3d_as(a_ptr, &tmA, &ctrl->full[stage], kb * kBlockK, row0, group, policy);
           if (args.gated == 1)
-            tma_load_2d_once(a_ptr + kATileBytes, &tmA, &ctrl->full[stage], kb * kBlockK, args.gate_off + row0, policy);
+            tma_load_3d_as(a_ptr + kATileBytes, &tmA, &ctrl->full[stage], kb * kBlockK, args.gate_off + row0, group, policy);
+        } else if constexpr (Sync::lean) {
+          tma_load_2d_as(a_ptr, &tmA, &ctrl->full[stage], kb * kBlockK, row0, policy);
+          if (args.gated == 1)
+            tma_load_2d_as(a_ptr + kATileBytes, &tmA, &ctrl->full[stage], kb * kBlockK, args.gate_off + row0, policy);
         } else {
           tma_load_2d(a_ptr, &tmA, &ctrl->full[stage], kb * kBlockK, row0);
           if (args.gated == 1)
