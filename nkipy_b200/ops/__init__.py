@@ -734,8 +734,8 @@ def packed_positions(q_start: torch.Tensor, q_lens: torch.Tensor, context_lens: 
                      block_size: int = 32) -> tuple:
     """(positions, cache slots), int32 [tokens], of the tokens of a packed step: sequence b's q_lens[b] new tokens, in rows q_start[b]
     on, are the last of its context_lens[b]; its blocks are row b of the table.  The sequences follow one another without gaps.  All
-    int32 and contiguous, on one device."""
-    B, dev = q_start.numel(), q_start.device
+    int32 and contiguous (the table may be part of a larger one), on one device."""
+    B, dev, block_table = q_start.numel(), q_start.device, block_table.contiguous()
     for t, shape in ((q_start, (B,)), (q_lens, (B,)), (context_lens, (B,)), (block_table, (B, block_table.shape[-1]))):
         if t.dtype != torch.int32 or t.device != dev or not t.is_contiguous():
             raise TypeError("packed_positions wants contiguous int32 tensors on one device")

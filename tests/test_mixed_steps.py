@@ -174,7 +174,10 @@ def test_positions_refuse_what_does_not_fit(device):
                 dict(block_table=i32([[], []]))):
         with pytest.raises(ValueError):
             ops.packed_positions(**{**good, **bad})
-    for bad in (dict(q_lens=good["q_lens"].long()), dict(q_start=i32([0, 9, 2, 9])[::2]), dict(block_table=i32([[1, 2, 9], [3, 4, 9]])[:, :2])):
+    slots = ops.packed_positions(**good)[1].tolist()
+    for part in (i32([[1, 2, 9], [3, 4, 9]])[:, :2], i32([[9, 1, 2], [9, 3, 4]])[:, 1:], i32([[1, 3], [2, 4]]).T):
+        assert ops.packed_positions(**{**good, "block_table": part})[1].tolist() == slots
+    for bad in (dict(q_lens=good["q_lens"].long()), dict(q_start=i32([0, 9, 2, 9])[::2])):
         with pytest.raises(TypeError):
             ops.packed_positions(**{**good, **bad})
 
